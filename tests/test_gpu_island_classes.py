@@ -1,0 +1,88 @@
+"""The island solve at the edges of its classes (tiny packs, one warp, one
+block of two sizes, the clustered grid solve) against a plain numpy solve of
+the same contacts, and against the same islands solved next to others."""
+import numpy as np
+import pytest
+
+import velox_b200 as vb
+from solve_model import advance
+from velox_b200.binding import SPEC
+
+pytestmark = pytest.mark.gpu
+
+H = 1.0 / 240.0
+# Single precision against float64 over 16 sweeps: each row rounds about 60
+# operations (60 x 2^-24 = 4e-6 of the velocities), and a sweep passes them on
+# without growth; 1e-4 of the largest velocity is the repository's bar for a
+# whole step.
+TOL = 1e-4
+
+
+def chain(n, world=0, start=0.0):
+    """n touching spheres in a row on a plane: one island of n bodies and about 2 n contacts."""
+    s = np.zeros(n + 1, SPEC)
+    s["orientation"] = (0, 0, 0, 1)
+    s["world"] = world
+    s["shape"][0] = 1
+    s["planeNormal"][0] = (0, 1, 0)
+    r = np.random.default_rng(n)
+    s["mass"][1:] = r.uniform(0.5, 2.0, n)
+    s["radius"][1:] = 0.5
+    s["friction"][1:] = 0.5
+    s["restitution"][1:] = 0.2
+    s["position"][1:, 0] = start + np.arange(n) * 0.995
+    s["position"][1:, 1] = 0.499
+    s["velocity"][1:] = r.normal(0.0, 0.5, (n, 3))
+    s["velocity"][1:, 1] -= 1.5
+    s["angularVelocity"][1:] = r.normal(0.0, 1.0, (n, 3))
+    return vb.bodies_from_specs(s, np.zeros((0, 3), np.float32))
+
+
+def solved(ctx, bodies, soup):
+    bodies = bodies.copy()
+    contacts = ctx.backend_find_contacts(bodies, soup, 4 * H)
+    contacts["normalImpulse"] = 0.01
+    contacts["tangentImpulse1"] = -0.002
+    colors, _ = ctx.color(bodies, contacts)
+    want = advance(bodies, contacts, colors, H, 8)
+    ctx.backend_advance_substeps(bodies, contacts, (0.0, 0.0, 0.0), H, 1)
+    ctx.backend_fetch_impulses(contacts)
+    return bodies, contacts, want
+
+
+# bodies: 8 and 9 straddle the packed islands (16 contacts), 64 / 65 and
+# 128 / 129 the one-warp class (64 bodies, 256 rows), 512 / 513 and 3072 / 3073
+# the two block classes; 40 leaves a lone row in some colours.
+@pytest.mark.parametrize("n", [1, 2, 8, 9, 40, 64, 65, 129, 512, 513, 3072, 3073])
+def test_island_class_edges(ctx, n):
+    bodies, hull, faces = chain(n)
+    got, contacts, (v, w, jn) = solved(ctx, bodies, vb.make_soup(hull, faces))
+    assert len(contacts) >= 2 * n - 1
+    scale = max(1.0, np.abs(v).max())
+    assert np.abs(got["velocity"] - v).max() < TOL * scale
+    assert np.abs(got["angularVelocity"] - w).max() < TOL * max(1.0, np.abs(w).max())
+    impulses = np.sort(contacts["normalImpulse"])
+    assert np.abs(impulses - np.sort(jn)).max() < TOL * max(1.0, np.abs(jn).max())
+
+
+def test_islands_of_every_class_side_by_side(ctx):
+    """Chains of several sizes in one world, far apart: each solves as it does alone, bit for bit."""
+    sizes = [3, 8, 9, 64, 65, 200, 513]
+    parts, at, total = [], 0.0, 0
+    for n in sizes:
+        parts.append(chain(n, start=at)[0][1:])
+        at += n * 0.995 + 30.0
+    ground = chain(1)[0][:1]
+    bodies = np.concatenate([ground] + parts).astype(vb.BODY)
+    soup = vb.make_soup(np.zeros((0, 3)), np.zeros(0))
+    both = vb.binding.records(bodies, vb.BODY).copy()
+    contacts = ctx.backend_find_contacts(both, soup, 4 * H)
+    ctx.backend_advance_substeps(both, contacts, (0.0, -9.81, 0.0), H, 4)
+    at = 1
+    for n, part in zip(sizes, parts):
+        alone = vb.binding.records(np.concatenate([ground, part]), vb.BODY).copy()
+        contacts = ctx.backend_find_contacts(alone, soup, 4 * H)
+        ctx.backend_advance_substeps(alone, contacts, (0.0, -9.81, 0.0), H, 4)
+        for name in ("position", "orientation", "velocity", "angularVelocity"):
+            assert np.array_equal(both[name][at:at + n], alone[name][1:]), (n, name)
+        at += n

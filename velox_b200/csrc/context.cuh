@@ -220,6 +220,7 @@ struct Context {
     DevBuf caFlagBuf, caBodyMarkBuf, caCandBuf, caSpecBuf;
     DevBuf localIdxBuf;                 // island-local body index (block solve)
     DevBuf prepBuf, frameBuf;           // per-row pose terms / per-body inertia frames (solve)
+    DevBuf planeBuf;                    // per-row terms of the islands that one block solves (RowPlanes)
     DevBuf fpKeyBuf, fpValBuf, fpSlotBuf, fpColorBuf, fpRunStartBuf, fpIslandBuf;  // parallel colouring
     DevBuf coopBuf;                     // CoopState of cooperative launches
     DevBuf giantBuf;                    // giant island list (solve)

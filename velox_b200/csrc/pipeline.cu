@@ -13,8 +13,9 @@
 //                island-local colour order equals its global colour order
 //   solve        one launch runs every island's whole substep loop
 //                (integration, warm start, 2*velocityIterations coloured
-//                sweeps, transform integration); tiny islands run one thread
-//                each, larger ones a block with a barrier between colours
+//                sweeps, transform integration); tiny islands share warps,
+//                larger ones run one block each (solve_rows.cuh), the largest
+//                the whole grid
 //   rewind       conservative advancement for deep end-of-step overlaps
 //   correction   split-impulse position correction, coloured per island
 #include <algorithm>
@@ -22,6 +23,7 @@
 #include <cstring>
 
 #include "context.cuh"
+#include "solve_rows.cuh"
 
 namespace vxb {
 
@@ -165,44 +167,6 @@ VXD uint32_t aggregatedSlot(uint32_t* counter) {
     if (lane == leader) base = atomicAdd(counter, (uint32_t)__popc(active));
     base = __shfl_sync(active, base, leader);
     return base + __popc(active & laneMaskLt());
-}
-
-VXD Mass loadMass(const BodyArrays& B, uint32_t i) {
-    const float4 in = B.inertia[i];
-    Mass m;
-    m.invI = V3{in.x, in.y, in.z};
-    m.invMass = in.w;
-    m.iq = q4(B.iq[i]);
-    m.flags = B.filt[i].x;
-    return m;
-}
-
-VXD SolverBody loadSolverBody(const BodyArrays& B, uint32_t i) {
-    SolverBody s;
-    s.p = f3(B.pos[i]);
-    s.q = q4(B.rot[i]);
-    s.v = f3(B.vel[i]);
-    s.w = f3(B.ang[i]);
-    s.m = loadMass(B, i);
-    s.sphere = shapeOf(s.m.flags) == kSphere;
-    return s;
-}
-
-VXD void loadRow(const vx_contact& c, RowContact& r) {
-    r.normal = V3{c.normal.x, c.normal.y, c.normal.z};
-    r.point = V3{c.point.x, c.point.y, c.point.z};
-    r.la = V3{c.localAnchorA.x, c.localAnchorA.y, c.localAnchorA.z};
-    r.lb = V3{c.localAnchorB.x, c.localAnchorB.y, c.localAnchorB.z};
-    r.bias0 = c.bias0; r.vn0 = c.vn0; r.restitution = c.restitution;
-    r.friction1 = c.friction1; r.friction2 = c.friction2;
-    r.rolling = c.rollingFriction; r.spinning = c.spinningFriction;
-    r.nImp = c.normalImpulse; r.t1Imp = c.tangentImpulse1; r.t2Imp = c.tangentImpulse2;
-    r.r1Imp = c.rollingImpulse1; r.r2Imp = c.rollingImpulse2; r.sImp = c.spinningImpulse;
-}
-VXD void storeRow(vx_contact& c, const RowContact& r) {
-    c.point = vx_vec3{r.point.x, r.point.y, r.point.z};
-    c.normalImpulse = r.nImp; c.tangentImpulse1 = r.t1Imp; c.tangentImpulse2 = r.t2Imp;
-    c.rollingImpulse1 = r.r1Imp; c.rollingImpulse2 = r.r2Imp; c.spinningImpulse = r.sImp;
 }
 
 // integrateKernel semantics (src/backend_cuda.cu:80-89) for body i.
@@ -803,8 +767,6 @@ VXD uint32_t ufFind(uint32_t* parent, uint32_t x) {
     return x;
 }
 
-VXD bool solvedContact(uint32_t fa, uint32_t fb) { return !isSensor(fa) && !isSensor(fb); }
-
 // Lock-free linking: a failed CAS means another thread linked that root, so
 // the retry loop always makes global progress; the bound only turns a
 // malfunction into a reported error instead of a hang.
@@ -1079,15 +1041,13 @@ __global__ void bodyStartKernel(const uint64_t* keys, uint32_t n, uint32_t* body
 // Islands the block kernels cannot hold (solveClusterKernel's share), counted
 // for the host's single read of the plan.
 constexpr uint32_t kTinyLimit = 16;   // islands of at most this many contacts: packed tiny solve
-constexpr int kBlockBodies = 512;     // islands beyond these sizes: the whole grid (giant islands)
-constexpr int kBlockRows = 3072;
 __global__ void giantCountKernel(const uint32_t* islandStart, const uint32_t* bodyStart, uint32_t islands,
                                  uint32_t realIslands, Counters* C) {
     uint32_t count = 0;
     for (uint32_t isl = blockIdx.x * blockDim.x + threadIdx.x; isl < islands; isl += gridDim.x * blockDim.x) {
         const uint32_t rows = islandStart[isl + 1] - islandStart[isl];
         const uint32_t nb = isl < realIslands ? bodyStart[isl + 1] - bodyStart[isl] : 0u;
-        if (rows > kTinyLimit && (nb > (uint32_t)kBlockBodies || rows > (uint32_t)kBlockRows)) ++count;
+        if (islandClassOf(nb, rows, kTinyLimit) == kGiantIsland) ++count;
     }
     for (int off = 16; off > 0; off >>= 1) count += __shfl_xor_sync(0xffffffffu, count, off);
     if ((threadIdx.x & 31) == 0 && count) atomicAdd(&C->giantCount, count);
@@ -1104,34 +1064,6 @@ __global__ void freeRangeKernel(const uint32_t* bodyStart, uint32_t entries, Cou
 // ---------------------------------------------------------------------------
 // island solve (src/backend_cuda.cu:569-761 semantics)
 // ---------------------------------------------------------------------------
-
-struct SolveArgs {
-    BodyArrays B;
-    vx_contact* contacts;        // key-sorted storage
-    const uint32_t* order;       // solve order -> contact index
-    const uint32_t* islandStart; // islands + 1 (solve-order ranges)
-    const uint32_t* segStart;    // segments + 1
-    const uint32_t* islandSeg;   // islands + 1 (first segment)
-    const uint32_t* bodyOrder;   // bodies sorted by island
-    const uint32_t* bodyStart;   // islands + 2
-    uint32_t islands;
-    uint32_t realIslands;  // islands >= realIslands (the null island) own no bodies
-    V3 gravity;
-    float h;
-    int substeps;
-    int sweeps;
-    int warmStart;     // warm start on the first substep
-    int integrate;     // integrate velocities (s > 0) and transforms each substep
-    int coneBlock;
-    uint32_t tinyLimit;
-    int positionIterations;  // position-correction mode when > 0
-    RowPrep* prep;           // per solve-order row, rebuilt every substep (block / global paths)
-    float4* frames;          // per body inertia frame, rebuilt every substep (global path)
-    int stackStabilization;
-    float stackStiffness, stackDamping;
-    uint32_t* fault;         // set when the island plan is inconsistent (Counters::planFault)
-    const uint2* rowBodies;  // per solve-order row: (a, b) of its contact (giant islands)
-};
 
 VXD void positionRow(const SolveArgs& A, uint32_t ci) {
     const vx_contact& cc = A.contacts[ci];
@@ -1165,28 +1097,13 @@ VXD void positionRow(const SolveArgs& A, uint32_t ci) {
 
 
 
-// Block-cooperative island processing: contacts of one colour in parallel,
-// a block barrier between colours. The island's dynamic bodies live in shared
-// memory for the whole substep loop (islands of up to kBlockBodies bodies and
-// kBlockRows contacts); larger islands run the same schedule on global memory.
-constexpr int kBlockThreads = 256;
-// Islands of up to kSmallBodies bodies and kSmallRows contacts run on one warp
-// each, many per SM (a colour of a small island has a few rows; a 256-thread
-// block would leave most of its threads idle and hold a whole SM's share of
-// shared memory).
-constexpr int kSmallThreads = 32;
-constexpr int kSmallBodies = 64;
-constexpr int kSmallRows = 256;
-constexpr size_t blockSmem(int bodies, int rows) {
-    return (size_t)bodies * (7 * sizeof(float4) + sizeof(uint32_t)) + (size_t)rows * sizeof(int2);
-}
-constexpr size_t kBlockSmem = blockSmem(kBlockBodies, kBlockRows);
-constexpr size_t kSmallSmem = blockSmem(kSmallBodies, kSmallRows);
+// Bodies of a pack of tiny islands in shared memory.
+constexpr int kGiantBlockThreads = 256;  // one block per giant island (no cooperative grid)
+constexpr size_t blockSmem(int bodies) { return (size_t)bodies * (7 * sizeof(float4) + sizeof(uint32_t)); }
 
 struct SharedBodies {
     float4 *p, *q, *v, *w, *inertia, *iq, *frame;
     uint32_t* flags;
-    int2* rowIdx;  // per island row: local index of a / b, -1 = read-only global body
 };
 
 template <int Bodies>
@@ -1200,7 +1117,6 @@ VXD SharedBodies carve(float4* base) {
     S.iq = S.inertia + Bodies;
     S.frame = S.iq + Bodies;
     S.flags = reinterpret_cast<uint32_t*>(S.frame + Bodies);
-    S.rowIdx = reinterpret_cast<int2*>(S.flags + Bodies);
     return S;
 }
 
@@ -1225,44 +1141,6 @@ VXD SolverBody globalBody(const BodyArrays& B, uint32_t id) {
     SolverBody b = loadSolverBody(B, id);
     cacheFrame(b);
     return b;
-}
-
-// op: 0 warm start, 1 velocity sweep, 2 position row, 3 prepare (pose terms)
-VXD void sharedRow(const SolveArgs& A, const SharedBodies& S, uint32_t k, uint32_t s0, int op) {
-    vx_contact& cc = A.contacts[A.order[s0 + k]];
-    const int2 li = S.rowIdx[k];
-    SolverBody a = li.x >= 0 ? sharedBody(S, li.x) : globalBody(A.B, cc.a);
-    SolverBody b = li.y >= 0 ? sharedBody(S, li.y) : globalBody(A.B, cc.b);
-    if (!solvedContact(a.m.flags, b.m.flags)) return;
-    if (op == 2) {
-        const float ima = solverInvMass(a.m), imb = solverInvMass(b.m);
-        const float invMassSum = ima + imb;
-        if (invMassSum <= 0.0f) return;
-        const V3 n{cc.normal.x, cc.normal.y, cc.normal.z};
-        const V3 wa = anchorWorld(a.sphere, a.p, a.q, V3{cc.localAnchorA.x, cc.localAnchorA.y, cc.localAnchorA.z});
-        const V3 wb = anchorWorld(b.sphere, b.p, b.q, V3{cc.localAnchorB.x, cc.localAnchorB.y, cc.localAnchorB.z});
-        const float gap = cc.bias0 + dot(n, wa - wb);
-        if (gap >= -1e-3f) return;
-        float resolve = 0.6f;
-        if (A.stackStabilization && lengthSq(a.v - b.v) < 1e-4f)
-            resolve += 0.2f * (A.stackStiffness / 1000.0f) / (1.0f + A.stackDamping * A.h);
-        const float push = -resolve * (gap + 1e-3f) / invMassSum;
-        if (isDynamic(a.m.flags) && !isAsleep(a.m.flags) && li.x >= 0) S.p[li.x] = pack(a.p + n * (push * ima), 0.0f);
-        if (isDynamic(b.m.flags) && !isAsleep(b.m.flags) && li.y >= 0) S.p[li.y] = pack(b.p - n * (push * imb), 0.0f);
-        return;
-    }
-    RowContact r;
-    loadRow(cc, r);
-    RowPrep& P = A.prep[s0 + k];
-    if (op == 3) {  // prepare
-        prepRow(a, b, r, A.h, A.coneBlock != 0, P);
-        return;
-    }
-    if (op == 0) warmPrepRow(a, b, r, P);
-    else sweepRow(a, b, r, P, A.coneBlock != 0);
-    if (li.x >= 0 && isDynamic(a.m.flags)) { S.v[li.x] = pack(a.v, 0.0f); S.w[li.x] = pack(a.w, 0.0f); }
-    if (li.y >= 0 && isDynamic(b.m.flags)) { S.v[li.y] = pack(b.v, 0.0f); S.w[li.y] = pack(b.w, 0.0f); }
-    storeRow(cc, r);
 }
 
 VXD void sharedIntegrateVelocity(const SolveArgs& A, const SharedBodies& S, int li, uint32_t id) {
@@ -1354,89 +1232,6 @@ __device__ void solveIslandGlobal(const SolveArgs& A, uint32_t isl) {
     }
 }
 
-// Small = the island fits the one-warp variant.
-VXD bool smallIsland(uint32_t nb, uint32_t rows) { return nb <= (uint32_t)kSmallBodies && rows <= (uint32_t)kSmallRows; }
-
-template <int Threads, int Bodies, int Rows, bool Small>
-__global__ void __launch_bounds__(Threads) solveBlockKernel(SolveArgs A, uint32_t* localIdx) {
-    extern __shared__ float4 smemRaw[];
-    const SharedBodies S = carve<Bodies>(smemRaw);
-    for (uint32_t isl = blockIdx.x; isl < A.islands; isl += gridDim.x) {
-        const uint32_t s0 = A.islandStart[isl], s1 = A.islandStart[isl + 1];
-        if (s1 - s0 <= A.tinyLimit) continue;
-        const uint32_t b0 = isl < A.realIslands ? A.bodyStart[isl] : 0u;
-        const uint32_t b1 = isl < A.realIslands ? A.bodyStart[isl + 1] : 0u;
-        const uint32_t nb = b1 - b0, rows = s1 - s0;
-        if (nb > (uint32_t)Bodies || rows > (uint32_t)Rows) continue;  // a giant island
-        if (!Small && smallIsland(nb, rows)) continue;                 // the one-warp variant's
-        for (uint32_t k = threadIdx.x; k < nb; k += blockDim.x) {
-            const uint32_t id = A.bodyOrder[b0 + k];
-            S.p[k] = A.B.pos[id]; S.q[k] = A.B.rot[id]; S.v[k] = A.B.vel[id]; S.w[k] = A.B.ang[id];
-            S.inertia[k] = A.B.inertia[id]; S.iq[k] = A.B.iq[id]; S.flags[k] = A.B.filt[id].x;
-            localIdx[id] = k;
-        }
-        __syncthreads();
-        for (uint32_t k = threadIdx.x; k < rows; k += blockDim.x) {
-            const vx_contact& cc = A.contacts[A.order[s0 + k]];
-            const bool da = isDynamic(A.B.filt[cc.a].x), db = isDynamic(A.B.filt[cc.b].x);
-            int la = da ? (int)localIdx[cc.a] : -1, lb = db ? (int)localIdx[cc.b] : -1;
-            // a dynamic body outside this island's list means an inconsistent plan: report it, never index smem
-            if (la >= 0 && ((uint32_t)la >= nb || A.bodyOrder[b0 + la] != cc.a)) { atomicOr(A.fault, 1u); la = -1; }
-            if (lb >= 0 && ((uint32_t)lb >= nb || A.bodyOrder[b0 + lb] != cc.b)) { atomicOr(A.fault, 1u); lb = -1; }
-            S.rowIdx[k] = make_int2(la, lb);
-        }
-        __syncthreads();
-        const uint32_t g0 = A.islandSeg[isl], g1 = A.islandSeg[isl + 1];
-        if (A.positionIterations > 0) {
-            for (int it = 0; it < A.positionIterations; ++it)
-                for (uint32_t g = g0; g < g1; ++g) {
-                    for (uint32_t k = A.segStart[g] - s0 + threadIdx.x; k < A.segStart[g + 1] - s0; k += blockDim.x)
-                        sharedRow(A, S, k, s0, 2);
-                    __syncthreads();
-                }
-        } else {
-            for (int s = 0; s < A.substeps; ++s) {
-                if (A.integrate && s > 0)
-                    for (uint32_t k = threadIdx.x; k < nb; k += blockDim.x)
-                        sharedIntegrateVelocity(A, S, (int)k, A.bodyOrder[b0 + k]);
-                for (uint32_t k = threadIdx.x; k < nb; k += blockDim.x) {
-                    Mass m;
-                    const float4 in = S.inertia[k];
-                    m.invI = V3{in.x, in.y, in.z};
-                    m.invMass = in.w;
-                    m.iq = q4(S.iq[k]);
-                    m.flags = S.flags[k];
-                    S.frame[k] = pack(inertiaFrameAt(m, q4(S.q[k])));
-                }
-                __syncthreads();
-                for (uint32_t k = threadIdx.x; k < rows; k += blockDim.x) sharedRow(A, S, k, s0, 3);
-                __syncthreads();
-                if (A.warmStart && s == 0)
-                    for (uint32_t g = g0; g < g1; ++g) {
-                        for (uint32_t k = A.segStart[g] - s0 + threadIdx.x; k < A.segStart[g + 1] - s0; k += blockDim.x)
-                            sharedRow(A, S, k, s0, 0);
-                        __syncthreads();
-                    }
-                for (int it = 0; it < A.sweeps; ++it)
-                    for (uint32_t g = g0; g < g1; ++g) {
-                        for (uint32_t k = A.segStart[g] - s0 + threadIdx.x; k < A.segStart[g + 1] - s0; k += blockDim.x)
-                            sharedRow(A, S, k, s0, 1);
-                        __syncthreads();
-                    }
-                if (A.integrate) {
-                    for (uint32_t k = threadIdx.x; k < nb; k += blockDim.x) sharedIntegrateTransform(A, S, (int)k);
-                    __syncthreads();
-                }
-            }
-        }
-        for (uint32_t k = threadIdx.x; k < nb; k += blockDim.x) {
-            const uint32_t id = A.bodyOrder[b0 + k];
-            A.B.pos[id] = S.p[k]; A.B.rot[id] = S.q[k]; A.B.vel[id] = S.v[k]; A.B.ang[id] = S.w[k];
-        }
-        __syncthreads();
-    }
-}
-
 // ---- tiny islands packed into warps -----------------------------------------
 //
 // Islands of at most tinyLimit (16) contacts are packed, in island order, into
@@ -1511,7 +1306,7 @@ __global__ void tinyPackKernel(SolveArgs A, const uint32_t* list, const uint32_t
 }
 
 // Per-warp shared memory of the pack kernel: the bodies and their ids.
-constexpr size_t kPackBodySmem = blockSmem(kPackBodies, 0);
+constexpr size_t kPackBodySmem = blockSmem(kPackBodies);
 constexpr size_t kPackWarpSmem = (kPackBodySmem + kPackBodies * sizeof(uint32_t) + 15) / 16 * 16;
 
 VXD void solveTinyPack(const SolveArgs& A, const uint32_t* list, const uint32_t* packFirst, uint32_t packs,
@@ -2136,7 +1931,7 @@ __global__ void __launch_bounds__(kClusterThreads) solveClusterKernel(SolveArgs 
 VXD bool isGiant(const SolveArgs& A, uint32_t isl) {
     const uint32_t rows = A.islandStart[isl + 1] - A.islandStart[isl];
     const uint32_t nb = isl < A.realIslands ? A.bodyStart[isl + 1] - A.bodyStart[isl] : 0u;
-    return rows > A.tinyLimit && (nb > (uint32_t)kBlockBodies || rows > (uint32_t)kBlockRows);
+    return islandClassOf(nb, rows, A.tinyLimit) == kGiantIsland;
 }
 
 __global__ void giantEntryKernel(SolveArgs A, const uint32_t* islandOf, uint32_t m, uint32_t n, uint64_t* keys,
@@ -2181,7 +1976,7 @@ __global__ void giantMemberKernel(SolveArgs A, const uint64_t* bodyKeys, uint32_
 }
 
 // Fallback when the device cannot run a cooperative grid: one block per giant island.
-__global__ void __launch_bounds__(kBlockThreads) solveGiantBlockKernel(SolveArgs A, const uint32_t* giants) {
+__global__ void __launch_bounds__(kGiantBlockThreads) solveGiantBlockKernel(SolveArgs A, const uint32_t* giants) {
     solveIslandGlobal(A, giants[blockIdx.x]);
 }
 
@@ -3301,6 +3096,8 @@ static SolveArgs solveArgs(Context& c, vx_contact* cs, const IslandPlan& plan) {
     A.tinyLimit = kTinyLimit;
     A.fault = &c.dCounters->planFault;
     A.prep = P<RowPrep>(c.prepBuf);
+    A.planes = P<float4>(c.planeBuf);
+    A.rows = plan.contacts;
     A.frames = P<float4>(c.frameBuf);
     return A;
 }
@@ -3309,6 +3106,18 @@ static int prepareSegments(Context& c, const IslandPlan& plan) {
     if (plan.islands == 0) return VXB_OK;
     LAUNCH(c, islandSegKernel, blocksFor(plan.islands + 1, 256), 256, P<uint32_t>(c.islandStartBuf),
            P<uint32_t>(c.scanBuf), plan.islands, plan.segments, P<uint32_t>(c.islandSegBuf));
+    return VXB_OK;
+}
+
+// The islands of one class, a block each, as many blocks as fit at once.
+template <int Class>
+static int launchIslands(Context& c, const SolveArgs& A) {
+    using Shape = ClassShape<Class>;
+    auto* kernel = A.coneBlock ? solveIslandKernel<Class, true> : solveIslandKernel<Class, false>;
+    VXB_CUDA(c, cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Shape::kSmem));
+    const uint32_t grid = std::min<uint32_t>(A.islands, (uint32_t)(c.smCount * Shape::kBlocksPerSm));
+    kernel<<<grid, Shape::kThreads, Shape::kSmem, c.stream>>>(A, P<uint32_t>(c.localIdxBuf));
+    ++c.launches;
     return VXB_OK;
 }
 
@@ -3353,22 +3162,9 @@ static int launchSolve(Context& c, const SolveArgs& A) {
             A, (const uint32_t*)tList, (const uint32_t*)tFirst, (const Counters*)c.dCounters, P<uint32_t>(c.localIdxBuf));
         ++c.launches;
     }
-    auto* large = solveBlockKernel<kBlockThreads, kBlockBodies, kBlockRows, false>;
-    auto* small = solveBlockKernel<kSmallThreads, kSmallBodies, kSmallRows, true>;
-    static int smallPerSm = 0;
-    if (!smallPerSm) {
-        cudaFuncSetAttribute(large, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kBlockSmem);
-        cudaFuncSetAttribute(small, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmallSmem);
-        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&smallPerSm, small, kSmallThreads, kSmallSmem) != cudaSuccess ||
-            smallPerSm <= 0)
-            smallPerSm = 8;
-    }
-    small<<<std::min<uint32_t>(A.islands, (uint32_t)(c.smCount * smallPerSm)), kSmallThreads, kSmallSmem, c.stream>>>(
-        A, P<uint32_t>(c.localIdxBuf));
-    ++c.launches;
-    large<<<std::min<uint32_t>(A.islands, (uint32_t)c.smCount * 2), kBlockThreads, kBlockSmem, c.stream>>>(
-        A, P<uint32_t>(c.localIdxBuf));
-    ++c.launches;
+    VXB_TRY(launchIslands<kSmallIsland>(c, A));
+    VXB_TRY(launchIslands<kMediumIsland>(c, A));
+    VXB_TRY(launchIslands<kLargeIsland>(c, A));
     // giant islands: list them, then one cooperative launch over all of them
     VXB_TRY(ensure(c, c.giantBuf, ((size_t)A.islands + 1) * 4 + 64));
     VXB_TRY(ensure(c, c.coopBuf, sizeof(CoopState)));
@@ -3483,13 +3279,14 @@ static int launchSolve(Context& c, const SolveArgs& A) {
         }
     }
     // no cooperative grid (or no solvable giant rows): one block per giant island
-    LAUNCH(c, solveGiantBlockKernel, giants, kBlockThreads, A, (const uint32_t*)list);
+    LAUNCH(c, solveGiantBlockKernel, giants, kGiantBlockThreads, A, (const uint32_t*)list);
     return VXB_OK;
 }
 
 // Substep loop over islands + contact-free bodies (advanceSubsteps).
 static int solveBuffers(Context& c, uint32_t m) {
     VXB_TRY(ensure(c, c.prepBuf, (size_t)m * sizeof(RowPrep) + 256));
+    VXB_TRY(ensure(c, c.planeBuf, (size_t)m * kPlaneWords * sizeof(float4) + 256));
     VXB_TRY(ensure(c, c.frameBuf, (size_t)c.n * 16 + 256));
     return VXB_OK;
 }

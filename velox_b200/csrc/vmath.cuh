@@ -36,16 +36,19 @@ VXD V3& operator-=(V3& a, const V3& b) { a.x -= b.x; a.y -= b.y; a.z -= b.z; ret
 VXD V3& operator*=(V3& a, float s) { a.x *= s; a.y *= s; a.z *= s; return a; }
 
 VXD float dot(const V3& a, const V3& b) { return a.x * b.x + a.y * b.y + a.z * b.z; }
-VXD float signedZero(float value, int order) {
-    return value != 0.0f ? value : (order > 0 ? 0.0f : -0.0f);
+// The components alone, zeros signed as the subtraction leaves them. The sign
+// rule of cross costs more than the product (five compares and three selects,
+// on predicates, against nine operations), so code that can show that a zero's
+// sign reaches no result uses this one.
+VXD V3 crossRaw(const V3& a, const V3& b) {
+    return V3{a.y * b.z - a.z * b.y, a.z * b.x - a.x * b.z, a.x * b.y - a.y * b.x};
 }
+VXD float signedZero(float value, float zero) { return value != 0.0f ? value : zero; }
 VXD V3 cross(const V3& a, const V3& b) {
-    const int order = a.x != b.x ? (a.x > b.x ? 1 : -1)
-                    : a.y != b.y ? (a.y > b.y ? 1 : -1)
-                    : a.z != b.z ? (a.z > b.z ? 1 : -1) : 1;
-    return V3{signedZero(a.y * b.z - a.z * b.y, order),
-              signedZero(a.z * b.x - a.x * b.z, order),
-              signedZero(a.x * b.y - a.y * b.x, order)};
+    const bool positive = (a.x > b.x) | ((a.x == b.x) & ((a.y > b.y) | ((a.y == b.y) & (a.z >= b.z))));
+    const float zero = positive ? 0.0f : -0.0f;
+    const V3 r = crossRaw(a, b);
+    return V3{signedZero(r.x, zero), signedZero(r.y, zero), signedZero(r.z, zero)};
 }
 VXD float lengthSq(const V3& v) { return dot(v, v); }
 VXD float length(const V3& v) { return sqrtf(lengthSq(v)); }
@@ -90,10 +93,18 @@ VXD Q4 qnormalize(const Q4& q) {
     return Q4{x * inv, y * inv, z * inv, w * inv};
 }
 
+// The inner product's zeros reach the outer one only as factors and by value
+// (a zero result there takes its sign from the operands' order), so their own
+// signs do not change the result.
 VXD V3 rotate(const Q4& q, const V3& v) {
     const V3 u{q.x, q.y, q.z};
-    const V3 t = cross(u, cross(u, v) + v * q.w);
+    const V3 t = cross(u, crossRaw(u, v) + v * q.w);
     return v + t * 2.0f;
+}
+// rotate whose zero components may carry the other sign.
+VXD V3 rotateRaw(const Q4& q, const V3& v) {
+    const V3 u{q.x, q.y, q.z};
+    return v + crossRaw(u, crossRaw(u, v) + v * q.w) * 2.0f;
 }
 VXD V3 rotateInv(const Q4& q, const V3& v) { return rotate(Q4{-q.x, -q.y, -q.z, q.w}, v); }
 
