@@ -141,6 +141,7 @@ struct Context {
     uint32_t caWidenings = 0;  // rewind replays with a widened body set (last step)
     uint32_t planContacts = 0; // contacts of the current island plan
     uint32_t planGiants = 0;   // giant islands of the current plan
+    uint32_t planLargest = 0;  // contacts of its largest island
     bool giantLinked = false;  // dataflow links of the plan's giant islands are built
     bool clusterBuilt = false; // spatial clusters of the plan's giant islands are built
     bool tinyPacked = false;   // the plan's tiny islands are packed into warps
