@@ -73,6 +73,7 @@ struct Counters {
     uint32_t planePairs;     // body-plane candidate pairs emitted
     uint32_t contactsTmp;    // contacts appended by the narrow phase
     uint32_t records;        // pairs with at least one contact
+    uint32_t hardPairs;      // pairs listed for the narrow phase's warp queries
     uint32_t contacts;       // contacts after placement (== contactsTmp when no overflow)
     uint32_t islands;        // contact islands
     uint32_t segments;       // (island, colour) segments
@@ -102,7 +103,7 @@ struct Counters {
     uint32_t clusterRows;    // their rows
     uint32_t clusterColours; // most colours of a giant island
     uint32_t giantCount;     // islands the block kernels cannot hold
-    uint32_t pad[1];
+    uint32_t caHard;         // pairs listed for the probe's warp queries
 };
 
 // Pipeline stages timed with CUDA events when timing is enabled.
@@ -232,6 +233,7 @@ struct Context {
     DevBuf clusterInfoBuf, clusterKeyBuf, clusterValBuf, clusterOfBuf, clusterCountBuf, clusterStartBuf,
         clusterRowsBuf;                 // spatial clusters of a giant island
     DevBuf clusterLinkBuf;              // cross-cluster predecessor links + remote-successor flags
+    DevBuf hardBuf;                     // narrow phase: pairs for the warp queries
     DevBuf caInfoBuf;                   // rewind pass: one record per candidate
     DevBuf tuneSaveBuf;                 // launch-shape trials: device copy of the counters
 

@@ -794,21 +794,10 @@ VXD GjkResult gjkDistance(const Convex& A, const Convex& B) {
 //
 // gjkSeeded for Normal-quality pairs (quality 0: 32 iterations, no re-seeding)
 // with the same arithmetic in the same order, the simplex in named registers
-// instead of an indexed array, and the support mappings inlined: a single
-// thread runs it at register latency rather than local-memory latency, which
-// is what the rewind pass's chains of dependent queries wait on. When the
-// general routine would report an overlap (and go on to EPA) this one hands
-// the simplex to gjkOverlapTail, the branch gjkSeeded itself would take.
-
-VXD SupportVert supportVertexInline(const Convex& A, const Convex& B, const V3& dir) {
-    SupportVert s;
-    const V3 oa = supportOffsetBody(A, dir);
-    const V3 ob = supportOffsetBody(B, -dir);
-    s.a = A.position + oa;
-    s.b = B.position + ob;
-    s.p = (A.position - B.position) + (oa - ob);
-    return s;
-}
+// instead of an indexed array: it runs at register latency rather than
+// local-memory latency. Where the general routine would report an overlap (and
+// go on to EPA) this one hands the simplex to the caller, who continues with
+// the branch gjkSeeded itself would take.
 
 // One face of solveTetrahedron: solve the triangle (x, y, z) and keep it when
 // its closest point is nearer than the best so far (strictly).
@@ -832,45 +821,52 @@ VXD void tetFaceCandidate(const SupportVert& x, const SupportVert& y, const Supp
     }
 }
 
-// solveTetrahedron (gjk.h:382-445) on named vertices; true = origin inside.
+// solveTetrahedron (gjk.h:382-445) on named vertices; true = origin inside. One
+// copy of a face's code for the four faces: unrolled, GJK's loop did not fit
+// the instruction cache (narrow phase of 64 box pyramids 2.2 -> 1.7 ms, of a
+// heap of 40,000 bodies 1.6 -> 1.3 ms, with the support mapping out of line). The
+// crosses only enter products and lengths, where a zero's sign does not matter.
 VXD bool solveTetrahedronV(SupportVert& v0, SupportVert& v1, SupportVert& v2, const SupportVert& v3, float& b0,
                            float& b1, float& b2, int& count, float scale) {
-    const float volume = dot(v1.p - v0.p, cross(v2.p - v0.p, v3.p - v0.p));
+    const float volume = dot(v1.p - v0.p, crossRaw(v2.p - v0.p, v3.p - v0.p));
     const float floorVol = 1e-10f * scale * scale * scale;
+    const bool flat = fabsf(volume) < floorVol;  // every face is a candidate
     SupportVert t0 = v0, t1 = v0, t2 = v0;
     float c0 = 0.0f, c1 = 0.0f, c2 = 0.0f;
     int bc = 0;
     float bestDist = 1e30f;
-    if (fabsf(volume) < floorVol) {
-        tetFaceCandidate(v0, v1, v2, t0, t1, t2, c0, c1, c2, bc, bestDist);
-        tetFaceCandidate(v0, v1, v3, t0, t1, t2, c0, c1, c2, bc, bestDist);
-        tetFaceCandidate(v0, v2, v3, t0, t1, t2, c0, c1, c2, bc, bestDist);
-        tetFaceCandidate(v1, v2, v3, t0, t1, t2, c0, c1, c2, bc, bestDist);
-        v0 = t0; v1 = t1; v2 = t2; b0 = c0; b1 = c1; b2 = c2; count = bc;
-        return false;
-    }
     bool inside = true;
     const float boundary = 3e-6f * scale;
-#pragma unroll
+#pragma unroll 1
     for (int f = 0; f < 4; ++f) {
-        const SupportVert& x = f == 3 ? v1 : v0;
-        const SupportVert& y = f == 0 || f == 1 ? v1 : v2;
-        const SupportVert& z = f == 0 ? v2 : v3;
-        const SupportVert& o = f == 0 ? v3 : f == 1 ? v2 : f == 2 ? v1 : v0;
-        const V3 a = x.p, b = y.p, c = z.p;
-        const V3 n = cross(b - a, c - a);
-        const float nLen = length(n);
-        if (nLen < 1e-20f) continue;
-        const float originDist = dot(n, -a) / nLen;
-        const float oppositeDist = dot(n, o.p - a) / nLen;
-        if (originDist * oppositeDist < 0.0f || fabsf(originDist) <= boundary) {
-            inside = false;
-            tetFaceCandidate(x, y, z, t0, t1, t2, c0, c1, c2, bc, bestDist);
+        const SupportVert x = f == 3 ? v1 : v0, y = f < 2 ? v1 : v2, z = f == 0 ? v2 : v3;
+        if (!flat) {
+            const V3 a = x.p, o = f == 0 ? v3.p : f == 1 ? v2.p : f == 2 ? v1.p : v0.p;
+            const V3 n = crossRaw(y.p - a, z.p - a);
+            const float nLen = length(n);
+            if (nLen < 1e-20f) continue;
+            const float originDist = dot(n, -a) / nLen;
+            const float oppositeDist = dot(n, o - a) / nLen;
+            if (!((originDist * oppositeDist < 0.0f) | (fabsf(originDist) <= boundary))) continue;
         }
+        inside = false;
+        tetFaceCandidate(x, y, z, t0, t1, t2, c0, c1, c2, bc, bestDist);
     }
     if (!inside) { v0 = t0; v1 = t1; v2 = t2; b0 = c0; b1 = c1; b2 = c2; count = bc; }
     return inside;
 }
+
+// The support mapping and tetrahedron step of one thread; a warp passes its own
+// (gjk_warp.cuh).
+struct ThreadSupport {
+    VXD SupportVert operator()(const Convex& A, const Convex& B, const V3& dir) const {
+        return supportVertex(A, B, dir);
+    }
+    VXD bool tetrahedron(SupportVert& v0, SupportVert& v1, SupportVert& v2, const SupportVert& v3, float& b0, float& b1,
+                         float& b2, int& count, float scale) const {
+        return solveTetrahedronV(v0, v1, v2, v3, b0, b1, b2, count, scale);
+    }
+};
 
 enum : int { kGjkSeparated = 0, kGjkOverlapExpand = 1, kGjkOverlapInside = 2, kGjkGeneral = 3 };
 
@@ -884,12 +880,13 @@ VXD void toSimplex(const SupportVert& v0, const SupportVert& v1, const SupportVe
 // kGjkSeparated: r holds the result. kGjkOverlap*: gjkSeeded would take its
 // overlap branch with simplex s (kGjkOverlapExpand: after expanding it).
 // kGjkGeneral: not a Normal-quality pair.
-VXD int gjkDistanceFast(const Convex& A, const Convex& B, GjkResult& r, Simplex& s) {
+template <class Support = ThreadSupport>
+VXD int gjkDistanceFast(const Convex& A, const Convex& B, GjkResult& r, Simplex& s, Support support = Support{}) {
     if (pairQuality(A, B) != 0) return kGjkGeneral;
     const float scale = pairScale(A, B);
     V3 dir = A.position - B.position;
     if (lengthSq(dir) < 1e-12f) dir = V3{1.0f, 0.0f, 0.0f};
-    SupportVert v0 = supportVertexInline(A, B, dir), v1 = v0, v2 = v0, v3 = v0;
+    SupportVert v0 = support(A, B, dir), v1 = v0, v2 = v0, v3 = v0;
     float b0 = 1.0f, b1 = 0.0f, b2 = 0.0f;
     int count = 1;
     for (int it = 0; it < 32; ++it) {
@@ -903,7 +900,7 @@ VXD int gjkDistanceFast(const Convex& A, const Convex& B, GjkResult& r, Simplex&
             return kGjkOverlapExpand;
         }
         const V3 d = -closest;
-        const SupportVert w = supportVertexInline(A, B, d);
+        const SupportVert w = support(A, B, d);
         const float progress = dot(w.p, d) - dot(closest, d);
         const float progressFloor = 1e-6f * sqrtf(distSq) + 1e-9f;
         if (progress < progressFloor) break;
@@ -921,7 +918,7 @@ VXD int gjkDistanceFast(const Convex& A, const Convex& B, GjkResult& r, Simplex&
             solveTriangleV(v0, v1, v2, b0, b1, b2, count);
         } else {
             v3 = w; count = 4;
-            if (solveTetrahedronV(v0, v1, v2, v3, b0, b1, b2, count, scale)) {
+            if (support.tetrahedron(v0, v1, v2, v3, b0, b1, b2, count, scale)) {
                 toSimplex(v0, v1, v2, v3, b0, b1, b2, 4, s);
                 return kGjkOverlapInside;
             }
@@ -1278,16 +1275,20 @@ VXD uint64_t manifoldFeatureKey(uint32_t a, uint32_t b) {
     return ((uint64_t(a) + 1) << 32) | (uint64_t(b) + 1);
 }
 
+// Largest gap that two bodies can close within dt, and so keep a contact at.
+VXD float contactReach(const BodyView& a, const BodyView& b, float dt) {
+    const float slop = 1e-3f;
+    return (sweeps(a.flags) ? maxPointSpeed(a) : 0.0f) * dt + (sweeps(b.flags) ? maxPointSpeed(b) : 0.0f) * dt +
+           a.specDist + b.specDist + slop;
+}
+
 // Appends a speculative contact when the pair can touch within dt
 // (narrowphase.h:425-463).
 static __device__ __noinline__ void emitContact(const BodyView& a, const BodyView& b, uint32_t ia, uint32_t ib,
                                          const V3& normal, const V3& point, float gap, float dt,
                                          vx_contact* out, int cap, int& n, uint64_t featureKey) {
     if (n >= cap) return;
-    const float slop = 1e-3f;
-    const float reach = (sweeps(a.flags) ? maxPointSpeed(a) : 0.0f) * dt +
-                        (sweeps(b.flags) ? maxPointSpeed(b) : 0.0f) * dt + a.specDist + b.specDist + slop;
-    if (gap > reach) return;
+    if (gap > contactReach(a, b, dt)) return;
     const float vn = dot(pointVelocity(a.p, a.v, a.w, point) - pointVelocity(b.p, b.v, b.w, point), normal);
     const V3 la = anchorLocal(shapeOf(a.flags) == kSphere, a.p, a.q, point);
     const V3 lb = anchorLocal(shapeOf(b.flags) == kSphere, b.p, b.q, point);
@@ -1395,13 +1396,12 @@ VXD bool isConvexVolume(uint32_t s) {
            s == kRoundedBox || s == kEllipsoid;
 }
 
-// Convex pair (narrowphase.h:555-607): GJK/EPA, then face clipping for
+// Convex pair (narrowphase.h:555-607): GJK/EPA (r), then face clipping for
 // Box/Hull pairs closer than 5 cm (boxes snap to the best separating face
 // axis first), else one GJK witness contact.
-static __device__ __noinline__ void convexConvex(const BodyView& a, const BodyView& b, uint32_t ia, uint32_t ib,
-                                          const Soup& soup, float dt, vx_contact* out, int cap, int& n) {
-    const Convex ca = makeConvex(a, soup), cb = makeConvex(b, soup);
-    const GjkResult r = gjkDistanceQuick(ca, cb);  // gjkDistance's result
+static __device__ __noinline__ void convexContacts(const BodyView& a, const BodyView& b, uint32_t ia, uint32_t ib,
+                                            const Convex& ca, const Convex& cb, const GjkResult& r, float dt,
+                                            vx_contact* out, int cap, int& n) {
     const uint32_t sa = shapeOf(a.flags), sb = shapeOf(b.flags);
     if (r.distance < 0.05f && (sa == kBox || sa == kHull) && (sb == kBox || sb == kHull)) {
         V3 manifoldNormal = r.normal;
@@ -1431,6 +1431,12 @@ static __device__ __noinline__ void convexConvex(const BodyView& a, const BodyVi
         }
     }
     emitContact(a, b, ia, ib, r.normal, (r.pointA + r.pointB) * 0.5f, r.distance, dt, out, cap, n, 0);
+}
+VXD void convexConvex(const BodyView& a, const BodyView& b, uint32_t ia, uint32_t ib, const Soup& soup, float dt,
+                      vx_contact* out, int cap, int& n) {
+    const Convex ca = makeConvex(a, soup), cb = makeConvex(b, soup);
+    const GjkResult r = gjkDistanceQuick(ca, cb);  // gjkDistance's result
+    convexContacts(a, b, ia, ib, ca, cb, r, dt, out, cap, n);
 }
 
 // ---- static triangle meshes and compounds (narrowphase.h:609-714) ---------
@@ -1531,6 +1537,25 @@ VXD bool isComplexShape(uint32_t s) { return s == kMesh || s == kCompound; }
 // through collideSimplePair, contacts owned by the parents: anchors in the
 // parents' frames, vn0 from the parents' point velocities, feature keys
 // tagged with the child numbers.
+static __device__ __noinline__ void ownContacts(const BodyView& a, const BodyView& b, uint32_t ia, uint32_t ib, int x,
+                                                int y, vx_contact* out, int added) {
+    const uint64_t tag = (uint64_t)(x + 1) * 0x9e3779b185ebca87ull ^ (uint64_t)(y + 1) * 0xc2b2ae3d27d4eb4full;
+    for (int k = 0; k < added; ++k) {
+        vx_contact& c = out[k];
+        const BodyView& ownerA = c.a == ia ? a : b;
+        const BodyView& ownerB = c.b == ib ? b : a;
+        const V3 point = v3(c.point), normal = v3(c.normal);
+        const V3 la = rotateInv(ownerA.q, point - ownerA.p);
+        const V3 lb = rotateInv(ownerB.q, point - ownerB.p);
+        c.localAnchorA = vx_vec3{la.x, la.y, la.z};
+        c.localAnchorB = vx_vec3{lb.x, lb.y, lb.z};
+        c.vn0 = dot(pointVelocity(ownerA.p, ownerA.v, ownerA.w, point) -
+                        pointVelocity(ownerB.p, ownerB.v, ownerB.w, point),
+                    normal);
+        c.featureKey ^= tag;
+    }
+}
+
 static __device__ __noinline__ int collideCompound(const BodyView& a, const BodyView& b, uint32_t ia, uint32_t ib,
                                                    const Soup& soup, float dt, vx_contact* out, int cap) {
     const bool ca = shapeOf(a.flags) == kCompound, cb = shapeOf(b.flags) == kCompound;
@@ -1542,21 +1567,7 @@ static __device__ __noinline__ int collideCompound(const BodyView& a, const Body
         for (int y = 0; y < countB && total < cap; ++y) {
             const BodyView gb = cb ? compoundChildView(b, soup.children[b.hullFirst + y]) : b;
             const int added = collideSimplePair(ga, gb, ia, ib, soup, dt, out + total, cap - total);
-            const uint64_t tag = (uint64_t)(x + 1) * 0x9e3779b185ebca87ull ^ (uint64_t)(y + 1) * 0xc2b2ae3d27d4eb4full;
-            for (int k = 0; k < added; ++k) {
-                vx_contact& c = out[total + k];
-                const BodyView& ownerA = c.a == ia ? a : b;
-                const BodyView& ownerB = c.b == ib ? b : a;
-                const V3 point = v3(c.point), normal = v3(c.normal);
-                const V3 la = rotateInv(ownerA.q, point - ownerA.p);
-                const V3 lb = rotateInv(ownerB.q, point - ownerB.p);
-                c.localAnchorA = vx_vec3{la.x, la.y, la.z};
-                c.localAnchorB = vx_vec3{lb.x, lb.y, lb.z};
-                c.vn0 = dot(pointVelocity(ownerA.p, ownerA.v, ownerA.w, point) -
-                                pointVelocity(ownerB.p, ownerB.v, ownerB.w, point),
-                            normal);
-                c.featureKey ^= tag;
-            }
+            ownContacts(a, b, ia, ib, x, y, out + total, added);
             total += added;
         }
     }

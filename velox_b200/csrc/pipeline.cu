@@ -23,6 +23,7 @@
 #include <cstring>
 
 #include "context.cuh"
+#include "pair_warp.cuh"
 #include "solve_rows.cuh"
 
 namespace vxb {
@@ -486,10 +487,50 @@ VXD bool pointLess(const vx_contact& x, const vx_contact& y) {
 // within one (a, b) key), append them and a record keyed for the global sort.
 // mode 0: key = (a << bodyBits) | b; mode 1: key = pair index, emission order kept.
 // Which pair classes one instantiation handles: plane pairs compile to a
-// light kernel (high occupancy), convex pairs to the GJK/EPA kernel.
-// Mesh and compound pairs (among the general pairs) take a third
-// instantiation, launched only when such bodies are loaded.
-enum PairClass : int { kAnyPairs = 0, kPlanePairs = 1, kConvexPairs = 2, kComplexPairs = 3 };
+// light kernel (high occupancy), convex pairs to the GJK kernel. Convex pairs
+// whose cores overlap (or that are not Normal quality) and mesh and compound
+// pairs are listed in `hard` for collideHardKernel: a thread's EPA runs up to
+// 1 ms, and one such lane held its warp and the stage's tail for that long.
+// Listed pairs: the contacts of those pairs from the query results that
+// collideHardKernel left (face clipping fills a warp's lanes again).
+enum PairClass : int { kAnyPairs = 0, kPlanePairs = 1, kConvexPairs = 2, kListedPairs = 3 };
+
+// Result of one listed pair's query.
+struct HardResult {
+    float distance;
+    V3 normal, pointA, pointB;
+};
+
+// Contacts of one pair in the order of the reference's host sort within one
+// (a, b) key (mode 0; mode 1 keeps the emission order).
+VXD void orderContacts(vx_contact* buf, int count, int mode) {
+    if (mode != 0) return;
+    for (int x = 1; x < count; ++x) {
+        vx_contact key = buf[x];
+        int y = x - 1;
+        while (y >= 0 && pointLess(key, buf[y])) { buf[y + 1] = buf[y]; --y; }
+        buf[y + 1] = key;
+    }
+}
+
+// A pair's contacts and record at reserved positions.
+VXD void storeContacts(const vx_contact* buf, int count, uint32_t off, uint32_t rec, uint32_t p, int mode, int bodyBits,
+                       vx_contact* tmp, uint32_t contactCap, uint64_t* recKeys, uint32_t* recVals, uint2* recInfo,
+                       uint32_t recCap, Counters* C) {
+    if (off + (uint32_t)count > contactCap || rec >= recCap) {
+        atomicOr(&C->overflow, 2u);
+        return;
+    }
+    for (int x = 0; x < count; ++x) {
+        tmp[off + x] = buf[x];
+        // the record's 8 tail bytes are padding: zero them so contact
+        // images (snapshots, read-back) are deterministic bytes
+        *reinterpret_cast<uint2*>(reinterpret_cast<char*>(tmp + off + x) + 120) = make_uint2(0u, 0u);
+    }
+    recKeys[rec] = mode == 0 ? (((uint64_t)buf[0].a << bodyBits) | buf[0].b) : (uint64_t)p;
+    recVals[rec] = rec;
+    recInfo[rec] = make_uint2(off, (uint32_t)count);
+}
 
 // `order` (optional): the pairs in the order to process them (convex pairs
 // grouped by shape combination so that a warp runs one code path).
@@ -498,37 +539,52 @@ __global__ void __launch_bounds__(128) collideKernel(BodyArrays B, Soup soup, co
                                                      const uint32_t* order, uint32_t npairs, float dt, int mode,
                                                      int bodyBits, vx_contact* tmp, uint32_t contactCap,
                                                      uint64_t* recKeys, uint32_t* recVals, uint2* recInfo,
-                                                     uint32_t recCap, Counters* C) {
+                                                     uint32_t recCap, uint32_t* hard, const HardResult* results,
+                                                     Counters* C) {
     const uint32_t stride = gridDim.x * blockDim.x;
+    if (Class == kListedPairs) npairs = C->hardPairs;
     const uint32_t rounded = (npairs + 31u) & ~31u;
     for (uint32_t base = blockIdx.x * blockDim.x; base < rounded; base += stride) {
         const uint32_t slot = base + threadIdx.x;
         const uint32_t p = slot < npairs && order ? order[slot] : slot;
         vx_contact buf[kMaxContactsPerPair];
         int count = 0;
+        bool later = false;
         if (slot < npairs) {
             const uint64_t pr = pairs[p];
             const uint32_t i = (uint32_t)(pr >> 32), j = (uint32_t)pr;
             const BodyView a = loadView(B, i);
             const BodyView b = loadView(B, j);
-            const bool complex = isComplexShape(shapeOf(a.flags)) || isComplexShape(shapeOf(b.flags));
             if (Class == kAnyPairs) {
                 count = collidePair(a, b, i, j, soup, dt, buf, kMaxContactsPerPair);
             } else if (Class == kPlanePairs) {
                 if (shapeOf(b.flags) == kPlane) planeConvex(a, b, i, j, soup, dt, buf, kMaxContactsPerPair, count);
                 else planeConvex(b, a, j, i, soup, dt, buf, kMaxContactsPerPair, count);
-            } else if (Class == kConvexPairs) {
-                if (!complex) convexConvex(a, b, i, j, soup, dt, buf, kMaxContactsPerPair, count);
-            } else if (complex) {
-                count = collidePair(a, b, i, j, soup, dt, buf, kMaxContactsPerPair);
+            } else if (isComplexShape(shapeOf(a.flags)) || isComplexShape(shapeOf(b.flags))) {
+                later = Class == kConvexPairs;  // (as a listed pair: done by its warp)
+            } else if (Class == kListedPairs) {
+                const HardResult h = results[slot];
+                GjkResult r;
+                r.distance = h.distance;
+                r.normal = h.normal; r.pointA = h.pointA; r.pointB = h.pointB;
+                r.overlapping = true;
+                convexContacts(a, b, i, j, makeConvex(a, soup), makeConvex(b, soup), r, dt, buf, kMaxContactsPerPair,
+                               count);
+            } else {
+                const Convex ca = makeConvex(a, soup), cb = makeConvex(b, soup);
+                GjkResult r;
+                Simplex s;
+                later = gjkDistanceFast(ca, cb, r, s) != kGjkSeparated;
+                if (!later) convexContacts(a, b, i, j, ca, cb, r, dt, buf, kMaxContactsPerPair, count);
             }
-            if (mode == 0)
-                for (int x = 1; x < count; ++x) {
-                    vx_contact key = buf[x];
-                    int y = x - 1;
-                    while (y >= 0 && pointLess(key, buf[y])) { buf[y + 1] = buf[y]; --y; }
-                    buf[y + 1] = key;
-                }
+            orderContacts(buf, count, mode);
+        }
+        if (Class == kConvexPairs) {
+            const unsigned m = __ballot_sync(0xffffffffu, later);
+            uint32_t at = 0;
+            if (m && (threadIdx.x & 31) == 0) at = atomicAdd(&C->hardPairs, (uint32_t)__popc(m));
+            at = __shfl_sync(0xffffffffu, at, 0);
+            if (later) hard[at + __popc(m & laneMaskLt())] = p;
         }
         // Warp-wide exclusive scan of the counts, one atomic per warp.
         const int lane = threadIdx.x & 31;
@@ -549,20 +605,47 @@ __global__ void __launch_bounds__(128) collideKernel(BodyArrays B, Soup soup, co
         if (count > 0) {
             const uint32_t off = cbase + incl - (uint32_t)count;
             const uint32_t rec = rbase + __popc(hasMask & laneMaskLt());
-            if (off + (uint32_t)count > contactCap || rec >= recCap) {
-                atomicOr(&C->overflow, 2u);
-            } else {
-                for (int x = 0; x < count; ++x) {
-                    tmp[off + x] = buf[x];
-                    // the record's 8 tail bytes are padding: zero them so contact
-                    // images (snapshots, read-back) are deterministic bytes
-                    *reinterpret_cast<uint2*>(reinterpret_cast<char*>(tmp + off + x) + 120) = make_uint2(0u, 0u);
-                }
-                recKeys[rec] = mode == 0 ? (((uint64_t)buf[0].a << bodyBits) | buf[0].b) : (uint64_t)p;
-                recVals[rec] = rec;
-                recInfo[rec] = make_uint2(off, (uint32_t)count);
-            }
+            storeContacts(buf, count, off, rec, p, mode, bodyBits, tmp, contactCap, recKeys, recVals, recInfo, recCap,
+                          C);
         }
+    }
+}
+
+// The listed pairs' queries, a warp each; the contacts of convex pairs follow
+// in collideKernel<kListedPairs>, mesh and compound pairs are finished here
+// (pair_warp.cuh). The list's length stays on the device; the grid is what
+// fits the GPU at once. Narrow phase of one step: 3.7 -> 0.5 ms with 2,500
+// bodies on a mesh, 1.9 -> 0.5 ms in the falling scene of 100,000 bodies (a few
+// deep pairs).
+constexpr int kQueryThreads = 128;  // warps that share a block's shared memory for their queries
+constexpr size_t kQuerySmem = kQueryThreads / 32 * sizeof(WarpQuery);
+
+__global__ void __launch_bounds__(kQueryThreads) collideHardKernel(BodyArrays B, Soup soup, const uint64_t* pairs,
+                                                                   const uint32_t* hard, float dt, int mode,
+                                                                   int bodyBits, vx_contact* tmp, uint32_t contactCap,
+                                                                   uint64_t* recKeys, uint32_t* recVals,
+                                                                   uint2* recInfo, uint32_t recCap,
+                                                                   HardResult* results, Counters* C) {
+    const uint32_t count = C->hardPairs, warps = (gridDim.x * blockDim.x) >> 5;
+    for (uint32_t k = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; k < count; k += warps) {
+        const uint32_t p = hard[k];
+        const uint64_t pr = pairs[p];
+        const uint32_t i = (uint32_t)(pr >> 32), j = (uint32_t)pr;
+        const BodyView a = loadView(B, i), b = loadView(B, j);
+        if (!isComplexShape(shapeOf(a.flags)) && !isComplexShape(shapeOf(b.flags))) {
+            const GjkResult r = gjkDistanceWarp(makeConvex(a, soup), makeConvex(b, soup));
+            if (warpLane() == 0u) results[k] = HardResult{r.distance, r.normal, r.pointA, r.pointB};
+            __syncwarp();
+            continue;
+        }
+        vx_contact buf[kMaxContactsPerPair];
+        const int n = collidePairWarp(a, b, i, j, soup, dt, buf, kMaxContactsPerPair);
+        if (n > 0 && warpLane() == 0u) {
+            orderContacts(buf, n, mode);
+            const uint32_t off = atomicAdd(&C->contactsTmp, (uint32_t)n), rec = atomicAdd(&C->records, 1u);
+            storeContacts(buf, n, off, rec, p, mode, bodyBits, tmp, contactCap, recKeys, recVals, recInfo, recCap, C);
+        }
+        __syncwarp();
     }
 }
 
@@ -2174,73 +2257,10 @@ __global__ void freeBodiesKernel(BodyArrays B, const uint32_t* bodyOrder, uint32
 // conservative-advancement rewind (src/world.cpp:4233-4357, gapAt :2916-2958)
 // ---------------------------------------------------------------------------
 
-struct GapProbe { float gap; V3 normal; };
-
 VXD BodyView withPose(BodyView b, const V3& p, const Q4& q) {
     b.p = p;
     b.q = q;
     return b;
-}
-
-// Distance query of the rewind: gjkDistance's results, the common case in registers.
-VXD GjkResult distanceQuery(const Convex& ca, const Convex& cb) { return gjkDistanceQuick(ca, cb); }
-
-// meshSimpleGapProbe (narrowphase.h:719-749): the smallest gap (strictly
-// smaller replaces) between `a` and the triangles of mesh `b` whose BVH
-// leaves overlap a cube of half width `search` around a's position.
-__device__ __noinline__ void meshGap(const BodyView& a, const BodyView& b, const Soup& soup, float search,
-                                     GapProbe& best) {
-    const vx_mesh& m = soup.meshes[b.hullFirst];
-    const V3 lo = a.p - V3{search, search, search}, hi = a.p + V3{search, search, search};
-    const Convex ca = makeConvex(a, soup);
-    meshVisit(soup, m, lo, hi, [&](uint32_t tri) {
-        const GjkResult g = distanceQuery(ca, meshTriangle(soup, m, tri));
-        if (g.distance < best.gap) best = GapProbe{g.distance, g.normal};
-        return true;
-    });
-}
-
-// gapAt (world.cpp:2916-2958) for two non-compound bodies, b not a mesh.
-VXD GapProbe gapConvex(const BodyView& a, const BodyView& b, const Soup& soup) {
-    if (shapeOf(b.flags) == kPlane) {
-        const Convex c = makeConvex(a, soup);
-        const V3 deep = c.position + supportOffsetBody(c, -b.planeN);
-        return GapProbe{dot(b.planeN, deep) - b.planeOff - c.radius, b.planeN};
-    }
-    const GjkResult r = distanceQuery(makeConvex(a, soup), makeConvex(b, soup));
-    return GapProbe{r.distance, r.normal};
-}
-
-// gapAt's compound and mesh cases: the minimum over every child pair (A's
-// children outer, B's inner) and every searched triangle, the first minimum
-// kept, starting from (1e30, +y) as the reference's recursion does.
-__device__ __noinline__ GapProbe gapComplex(const BodyView& a, const BodyView& b, const Soup& soup, float search) {
-    GapProbe best{1e30f, V3{0.0f, 1.0f, 0.0f}};
-    const bool ca = shapeOf(a.flags) == kCompound, cb = shapeOf(b.flags) == kCompound;
-    const uint32_t countA = ca ? a.hullCount : 1u, countB = cb ? b.hullCount : 1u;
-    for (uint32_t x = 0; x < countA; ++x) {
-        const BodyView ga = ca ? compoundChildView(a, soup.children[a.hullFirst + x]) : a;
-        for (uint32_t y = 0; y < countB; ++y) {
-            const BodyView gb = cb ? compoundChildView(b, soup.children[b.hullFirst + y]) : b;
-            if (shapeOf(gb.flags) == kMesh) {
-                meshGap(ga, gb, soup, search, best);
-            } else {
-                const GapProbe g = gapConvex(ga, gb, soup);
-                if (g.gap < best.gap) best = g;
-            }
-        }
-    }
-    return best;
-}
-
-// Signed gap and normal (from b towards a) of the rewind's distance oracle;
-// `dt` sizes the mesh search cube as the rewind loop does (world.cpp:4272-4273).
-__device__ __noinline__ GapProbe gapAt(const BodyView& a, const BodyView& b, const Soup& soup, float dt) {
-    if (isComplexShape(shapeOf(a.flags)) || isComplexShape(shapeOf(b.flags))) {
-        const float search = maxPointSpeed(a) * dt + a.radius + length(a.half) + a.hh + 0.1f;
-        return gapComplex(a, b, soup, search);
-    }
-    return gapConvex(a, b, soup);
 }
 
 // Bounding spheres more than 1 mm apart give a positive end gap, so the
@@ -2273,27 +2293,65 @@ VXD void orientPair(const BodyArrays& B, uint64_t key, uint32_t& i, uint32_t& j)
     if (!isDynamic(B.filt[i].x) && isDynamic(B.filt[j].x)) { const uint32_t t = i; i = j; j = t; }
 }
 
-// `order` (optional): the pairs grouped by shape combination, so that a warp's
-// lanes mostly take the same distance-query path; every outcome is written at
-// the pair's own index.
+// The probe: end-state gap of every pair, one thread each; pairs whose query
+// overlaps (or that involve a mesh or compound) are listed in `hard` for
+// caProbeHardKernel. `order` (optional): the pairs grouped by shape
+// combination, so that a warp's lanes mostly take the same distance-query
+// path; every outcome is written at the pair's own index.
+VXD void caFlag(const BodyArrays& B, uint32_t r, uint32_t i, uint32_t j, uint32_t flagsB, const GapProbe& end,
+                uint32_t* flags, uint32_t* bodyMark, float4* endGap) {
+    uint32_t flag = 0;
+    if (end.gap < -8e-3f) {
+        flag = 1;
+        endGap[r] = make_float4(end.gap, end.normal.x, end.normal.y, end.normal.z);
+        bodyMark[i] = 1;  // only dynamic bodies move in a rewind
+        if (isDynamic(flagsB)) bodyMark[j] = 1;
+    }
+    flags[r] = flag;
+}
+
 __global__ void caProbeKernel(BodyArrays B, Soup soup, const uint64_t* pairKeys, const uint32_t* order,
-                              uint32_t npairs, float dt, uint32_t* flags, uint32_t* bodyMark, float4* endGap) {
+                              uint32_t npairs, uint32_t* flags, uint32_t* bodyMark, float4* endGap, uint32_t* hard,
+                              Counters* C) {
     for (uint32_t slot = blockIdx.x * blockDim.x + threadIdx.x; slot < npairs; slot += gridDim.x * blockDim.x) {
         const uint32_t r = order ? order[slot] : slot;
         uint32_t i, j;
         orientPair(B, pairKeys[r], i, j);
         const BodyView a = loadView(B, i), b = loadView(B, j);
-        uint32_t flag = 0;
+        GapProbe end{0.0f, V3{0.0f, 0.0f, 0.0f}};
+        bool later = false;
         if (!spheresApart(a, b) && caEligible(a, b, B, i)) {
-            const GapProbe end = gapAt(a, b, soup, dt);
-            if (end.gap < -8e-3f) {
-                flag = 1;
-                endGap[r] = make_float4(end.gap, end.normal.x, end.normal.y, end.normal.z);
-                bodyMark[i] = 1;  // only dynamic bodies move in a rewind
-                if (isDynamic(b.flags)) bodyMark[j] = 1;
+            if (isComplexShape(shapeOf(a.flags)) || isComplexShape(shapeOf(b.flags))) {
+                later = true;
+            } else if (shapeOf(b.flags) == kPlane) {
+                const Convex c = makeConvex(a, soup);
+                const V3 deep = c.position + supportOffsetBody(c, -b.planeN);
+                end = GapProbe{dot(b.planeN, deep) - b.planeOff - c.radius, b.planeN};
+            } else {
+                GjkResult g;
+                Simplex s;
+                later = gjkDistanceFast(makeConvex(a, soup), makeConvex(b, soup), g, s) != kGjkSeparated;
+                if (!later) end = GapProbe{g.distance, g.normal};
             }
         }
-        flags[r] = flag;
+        if (later) hard[aggregatedSlot(&C->caHard)] = r;
+        else caFlag(B, r, i, j, b.flags, end, flags, bodyMark, endGap);
+    }
+}
+
+__global__ void __launch_bounds__(kQueryThreads) caProbeHardKernel(BodyArrays B, Soup soup, const uint64_t* pairKeys,
+                                                                   const uint32_t* hard, float dt, uint32_t* flags,
+                                                                   uint32_t* bodyMark, float4* endGap,
+                                                                   const Counters* C) {
+    const uint32_t count = C->caHard, warps = (gridDim.x * blockDim.x) >> 5;
+    for (uint32_t k = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; k < count; k += warps) {
+        const uint32_t r = hard[k];
+        uint32_t i, j;
+        orientPair(B, pairKeys[r], i, j);
+        const BodyView a = loadView(B, i), b = loadView(B, j);
+        const GapProbe end = gapAtWarp(a, b, soup, dt);
+        if (warpLane() == 0u) caFlag(B, r, i, j, b.flags, end, flags, bodyMark, endGap);
+        __syncwarp();
     }
 }
 
@@ -2313,8 +2371,8 @@ VXD Q4 orientationAt(const Mass& m, const Q4& start, const V3& L, float elapsed)
     return q;
 }
 
-// Full rewind logic for one oriented pair on the current state. Returns true
-// when the pair was rewound.
+// Full rewind logic for one oriented pair on the current state, by one warp.
+// Returns true when the pair was rewound.
 // `cached`: the probe's end-state gap for this pair when neither body has
 // moved since the probe (else null: computed here). `spec` (optional): write
 // the rewound states there (a: pos, rot, vel, ang; then b) instead of into B.
@@ -2329,7 +2387,7 @@ __device__ __noinline__ bool caRewind(BodyArrays& B, const Soup& soup, uint32_t 
         const float4 g = *cached;
         end = GapProbe{g.x, V3{g.y, g.z, g.w}};
     } else {
-        end = gapAt(a, b, soup, dt);
+        end = gapAtWarp(a, b, soup, dt);
     }
     if (end.gap >= -8e-3f) return false;
     const bool bStatic = isStaticBody(b.flags), bDyn = isDynamic(b.flags);
@@ -2350,12 +2408,12 @@ __device__ __noinline__ bool caRewind(BodyArrays& B, const Soup& soup, uint32_t 
         ++queries;
         const Q4 qa = orientationAt(ma, qa0, La, dt * t);
         const Q4 qb = bStatic ? qb0 : orientationAt(mb, qb0, Lb, dt * t);
-        const GapProbe g = gapAt(withPose(a, pa0 + da * t, qa), withPose(b, pb0 + db * t, qb), soup, dt);
+        const GapProbe g = gapAtWarp(withPose(a, pa0 + da * t, qa), withPose(b, pb0 + db * t, qb), soup, dt);
         n = g.normal;
         if (g.gap < 1e-3f) break;
         t = vmin(1.0f, t + g.gap / bound);
     }
-    atomicAdd(gapQueries, queries);
+    if (warpLane() == 0u) atomicAdd(gapQueries, queries);
     if (t >= 1.0f) return false;
     a.p = pa0 + da * t;
     a.q = qa0;
@@ -2382,6 +2440,7 @@ __device__ __noinline__ bool caRewind(BodyArrays& B, const Soup& soup, uint32_t 
     const float remaining = dt * (1.0f - t);
     advanceTransform(ma, a.p, a.q, a.v, a.w, remaining);
     if (bDyn) advanceTransform(mb, b.p, b.q, b.v, b.w, remaining);
+    if (warpLane() != 0u) return true;
     if (spec) {
         spec[0] = pack(a.p, 0.0f); spec[1] = pack(a.q); spec[2] = pack(a.v, 0.0f); spec[3] = pack(a.w, 0.0f);
         spec[4] = pack(b.p, 0.0f); spec[5] = pack(b.q); spec[6] = pack(b.v, 0.0f); spec[7] = pack(b.w, 0.0f);
@@ -2402,27 +2461,27 @@ VXD uint64_t globalTimerNs() {
 
 // Every flagged pair evaluated in parallel on the probe's state (read-only):
 // in the ordered pass, a flagged pair whose bodies no earlier rewind has moved
-// sees exactly this state, so its outcome can be taken from here.
-// `spread` (1..32): threads per pair, so that a few pairs occupy many SMs
-// and share warps with few others (each is a long serial loop). The working
-// lanes are the first 32 / spread of each warp: local memory interleaves the
-// lanes' words, so contiguous lanes share L1 sectors of their stack frames
-// (lanes 0-7 use one sector of every line).
-__global__ void caSpeculateKernel(BodyArrays B, Soup soup, const uint64_t* pairKeys, const uint32_t* flaggedList,
-                                  uint32_t flagged, uint32_t spread, const float4* endGap, float dt,
-                                  const float4* prevPos, const float4* prevRot, float4* specState,
-                                  uint32_t* specResult, Counters* C) {
-    const uint32_t perWarp = 32u / spread, lane = threadIdx.x & 31u;
-    if (lane >= perWarp) return;
-    const uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, warps = (gridDim.x * blockDim.x) >> 5;
-    for (uint32_t k = warp * perWarp + lane; k < flagged; k += warps * perWarp) {
+// sees exactly this state, so its outcome can be taken from here. A warp per
+// pair: up to 25 dependent distance queries.
+__global__ void __launch_bounds__(kQueryThreads) caSpeculateKernel(BodyArrays B, Soup soup, const uint64_t* pairKeys,
+                                                                   const uint32_t* flaggedList, uint32_t flagged,
+                                                                   const float4* endGap, float dt,
+                                                                   const float4* prevPos, const float4* prevRot,
+                                                                   float4* specState, uint32_t* specResult,
+                                                                   Counters* C) {
+    const uint32_t warps = (gridDim.x * blockDim.x) >> 5;
+    for (uint32_t k = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; k < flagged; k += warps) {
         const uint32_t r = flaggedList[k];
         uint32_t i, j;
         orientPair(B, pairKeys[r], i, j);
         const uint64_t t0 = globalTimerNs();
-        specResult[k] = caRewind(B, soup, i, j, dt, prevPos, prevRot, &C->caGapQueries, endGap + r,
-                                 specState + 8 * (size_t)k) ? 1u : 0u;
-        atomicMax(&C->caSpecMicros, (uint32_t)((globalTimerNs() - t0) / 1000u));
+        const bool moved = caRewind(B, soup, i, j, dt, prevPos, prevRot, &C->caGapQueries, endGap + r,
+                                    specState + 8 * (size_t)k);
+        if (warpLane() == 0u) {
+            specResult[k] = moved ? 1u : 0u;
+            atomicMax(&C->caSpecMicros, (uint32_t)((globalTimerNs() - t0) / 1000u));
+        }
+        __syncwarp();
     }
 }
 
@@ -2432,27 +2491,27 @@ __global__ void caSpeculateKernel(BodyArrays B, Soup soup, const uint64_t* pairK
 // exactly as the reference's single ordered loop would evaluate it: it sees
 // the same body states and rewound marks, as long as no rewind moves a body
 // outside the marked set (that case is flagged; the caller widens the set and
-// replays the pass from a snapshot). Workers (lane 0 of a warp) take ready
-// candidates from a queue, so independent chains never wait for one another.
-// Cooperative launch (all workers resident); every wait is bounded.
+// replays the pass from a snapshot). Workers (warps) take ready candidates
+// from a queue, so independent chains never wait for one another; a worker
+// goes on with a successor that it made ready, so a chain passes through the
+// queue only where it forks. Cooperative launch (all workers resident); every
+// wait is bounded.
+//
+// What bounds it: the longest chain of evaluations, each up to 25 dependent
+// distance queries, and about 2.7 us a link where nothing is evaluated. Workers
+// were one lane per SM, whose queries kept 10 KB stack frames in local memory
+// (more lanes per SM evicted one another's); a warp keeps its polytope in
+// shared memory and shares the scans. Rewind stage of one step: 7.2 -> 1.4 ms
+// with 2,500 bodies on a mesh, 9.2 -> 6.6 ms in a heap of 40,000, 8.8 -> 6.5 ms
+// among 1,000 tumbling boxes. One, two or four blocks of workers per SM: the
+// same times (the chain binds).
 constexpr int kCaWidenLimit = 8;  // replays with a widened marked set before the serial loop
 constexpr uint32_t kProbeGroupMin = 8192;  // pairs from which the probe groups them by shape combination
 constexpr int kCaWidenHops = 8;   // hops of widening per replay
 constexpr int kCaInitialHops = 8; // hops of widening before the first pass
-// Workers of the rewind pass: one block of kCaFlowThreads threads per SM, one
-// worker lane per warp. A worker's distance queries keep a stack frame of
-// about 10 KB (simplex, EPA polytope) in local memory, where one active lane
-// takes a 32-byte L1 sector per 4-byte word: several workers on an SM evict
-// one another's frames. On a settled 100k-body pile a distance query took
-// 18 us with 1 worker per SM, 31 us with 2, 64 us with 4 and 127 us with 8,
-// at about the same queries per SM per second. The pass is bound by its
-// longest dependency chain, so one fast worker per SM wins (chain 5.0 ms,
-// against 8.1 ms with 2 and 12.1 ms with 8; the pass's 24k evaluations still
-// fit beside it).
-constexpr int kCaFlowThreads = 32;
-constexpr int kCaFlowBlocksPerSm = 1;
+constexpr int kCaFlowBlocksPerSm = 2;
 
-__global__ void __launch_bounds__(256) caFlowKernel(BodyArrays B, Soup soup, const uint32_t* flagRank,
+__global__ void __launch_bounds__(kQueryThreads) caFlowKernel(BodyArrays B, Soup soup, const uint32_t* flagRank,
                                                     const float4* specState, const uint32_t* specResult,
                                                     const uint4* info, uint32_t ncand, const uint32_t* succ,
                                                     uint32_t* pending, uint32_t* queue, uint32_t* depth,
@@ -2462,6 +2521,7 @@ __global__ void __launch_bounds__(256) caFlowKernel(BodyArrays B, Soup soup, con
     const uint32_t tid = blockIdx.x * blockDim.x + threadIdx.x, stride = gridDim.x * blockDim.x;
     uint32_t* tail = &st->queued[0];
     uint32_t* head = &st->queued[1];
+    uint32_t* finished = &st->queued[2];  // candidates done, added when a worker's chain ends
     for (uint32_t k = tid; k < ncand; k += stride)  // roots
         if (pending[k] == 0u) {
             const uint32_t t = atomicAdd(tail, 1u);
@@ -2471,24 +2531,30 @@ __global__ void __launch_bounds__(256) caFlowKernel(BodyArrays B, Soup soup, con
     // Every root is queued before any worker starts: a count that a finished
     // candidate has taken to zero must not read as a root.
     if (!gridSync(&st->bar, &st->timeout, st->spinLimit)) return;
-    if ((threadIdx.x & 31u) != 0u) return;
-    uint32_t rewinds = 0, maxDepth = 0, maxCrit = 0;
+    const bool lead = warpLane() == 0u;
+    uint32_t rewinds = 0, maxDepth = 0, maxCrit = 0, mine = 0, k = kNoPred;
     for (;;) {
-        const uint32_t h = atomicAdd(head, 1u);
-        if (h >= ncand) break;
-        // Claimed before it was filled. Idle workers back off (up to ~1 us) and
-        // read the shared timeout word only every 16th poll: a thousand warps
-        // polling one L2 line at full rate slow the working lanes' own loads.
-        uint32_t k, spins = 0, nap = 32;
-        while ((k = __ldcg(queue + h)) == kNoPred) {
-            if (++spins > st->spinLimit || ((spins & 15u) == 0u && __ldcg(&st->timeout))) {
-                atomicOr(&st->timeout, 1u);
-                return;
+        if (k == kNoPred) {  // the chain ended: claim a queue slot and wait for it to be filled
+            if (lead) {
+                if (mine) atomicAdd(finished, mine);
+                const uint32_t h = atomicAdd(head, 1u);
+                // Idle workers back off (up to ~1 us) and read the shared words
+                // only every 8th poll: polling them at full rate slows the
+                // working warps' own loads.
+                uint32_t spins = 0, nap = 32;
+                while (h < ncand && (k = __ldcg(queue + h)) == kNoPred) {
+                    if (++spins > st->spinLimit) atomicOr(&st->timeout, 1u);
+                    if ((spins & 7u) == 0u && (__ldcg(finished) >= ncand || __ldcg(&st->timeout))) break;
+                    __nanosleep(nap);
+                    if (nap < 1024u) nap <<= 1;
+                }
             }
-            __nanosleep(nap);
-            if (nap < 1024u) nap <<= 1;
+            mine = 0;
+            k = __shfl_sync(kFullWarp, k, 0);
+            if (k == kNoPred) break;
         }
-        __threadfence();  // acquire the predecessors' writes
+        if (lead) __threadfence();  // acquire the predecessors' writes
+        __syncwarp();
         const uint64_t t0 = globalTimerNs();
         // record, successors and chain statistics in one round of loads (the
         // predecessors raised depth and crit before they released this one)
@@ -2498,63 +2564,64 @@ __global__ void __launch_bounds__(256) caFlowKernel(BodyArrays B, Soup soup, con
         const uint32_t crit0 = __ldcg(crit + k);
         const uint32_t i = rec.y, j = rec.z;
         const bool jDyn = (rec.w & 2u) != 0u;
-        const bool touched = __ldcg(rewound + i) || __ldcg(rewound + j);
+        const uint32_t seen = __ldcg(rewound + i) | __ldcg(rewound + j);
+        const bool touched = __shfl_sync(kFullWarp, seen, 0) != 0u;
         if ((rec.w & 1u) || touched) {
             bool rewoundPair;
             if (!touched) {  // flagged, bodies as the probe saw them: the speculative outcome holds
                 const uint32_t sk = flagRank[rec.x];
                 rewoundPair = specResult[sk] != 0u;
-                if (rewoundPair) {
-                    const float4* st4 = specState + 8 * (size_t)sk;
-                    __stcg(B.pos + i, st4[0]); __stcg(B.rot + i, st4[1]); __stcg(B.vel + i, st4[2]); __stcg(B.ang + i, st4[3]);
-                    if (jDyn) {
-                        __stcg(B.pos + j, st4[4]); __stcg(B.rot + j, st4[5]); __stcg(B.vel + j, st4[6]);
-                        __stcg(B.ang + j, st4[7]);
-                    }
+                if (rewoundPair && warpLane() < (jDyn ? 8u : 4u)) {
+                    const uint32_t lane = warpLane(), id = lane < 4u ? i : j;
+                    float4* to = (lane & 3u) == 0u ? B.pos : (lane & 3u) == 1u ? B.rot : (lane & 3u) == 2u ? B.vel : B.ang;
+                    __stcg(to + id, specState[8 * (size_t)sk + lane]);
                 }
             } else {
                 rewoundPair = caRewind(B, soup, i, j, dt, prevPos, prevRot, &C->caGapQueries, nullptr);
             }
             if (rewoundPair) {
                 ++rewinds;
-                __stcg(rewound + i, 1u);
-                if (jDyn) __stcg(rewound + j, 1u);
-                if (!bodyMark[i] || (jDyn && !bodyMark[j])) atomicOr(&C->caOverflow, 1u);
+                if (lead) {
+                    __stcg(rewound + i, 1u);
+                    if (jDyn) __stcg(rewound + j, 1u);
+                    if (!bodyMark[i] || (jDyn && !bodyMark[j])) atomicOr(&C->caOverflow, 1u);
+                }
             }
         }
         const uint64_t elapsed = globalTimerNs() - t0;
         const uint32_t ck = crit0 + (uint32_t)(elapsed < 0x7fffffffull ? elapsed : 0x7fffffffull);
         maxDepth = max(maxDepth, d);
         maxCrit = max(maxCrit, ck);
-        __threadfence();  // release this evaluation's writes before the successors can run
-        // both successors' counts drop in one round; a count that reaches
-        // zero queues its candidate (the same one twice only if it follows
-        // this one on both bodies, and then only the second drop reaches zero)
-        uint32_t left0 = 0u, left1 = 0u;
-        if (next.x != kNoPred) {
-            atomicMax(depth + next.x, d);
-            atomicMax(crit + next.x, ck);
-            left0 = atomicSub(pending + next.x, 1u);
-        }
-        if (next.y != kNoPred) {
-            atomicMax(depth + next.y, d);
-            atomicMax(crit + next.y, ck);
-            left1 = atomicSub(pending + next.y, 1u);
-        }
-        const uint32_t ready = (left0 == 1u ? 1u : 0u) + (left1 == 1u ? 1u : 0u);
-        if (ready) {
-            uint32_t t = atomicAdd(tail, ready);
-            if (left0 == 1u) {
-                if (t < ncand) __stcg(queue + t, next.x);
-                else atomicOr(&st->spill, 4u);
-                ++t;
+        ++mine;
+        k = kNoPred;
+        __syncwarp();
+        if (lead) {
+            __threadfence();  // release this evaluation's writes before the successors can run
+            // both successors' counts drop in one round; a count that reaches
+            // zero makes its candidate ready (the same one twice only if it
+            // follows this one on both bodies, and then only the second drop
+            // reaches zero)
+            uint32_t left0 = 0u, left1 = 0u;
+            if (next.x != kNoPred) {
+                atomicMax(depth + next.x, d);
+                atomicMax(crit + next.x, ck);
+                left0 = atomicSub(pending + next.x, 1u);
             }
-            if (left1 == 1u) {
+            if (next.y != kNoPred) {
+                atomicMax(depth + next.y, d);
+                atomicMax(crit + next.y, ck);
+                left1 = atomicSub(pending + next.y, 1u);
+            }
+            k = left0 == 1u ? next.x : left1 == 1u ? next.y : kNoPred;
+            if (left0 == 1u && left1 == 1u) {
+                const uint32_t t = atomicAdd(tail, 1u);
                 if (t < ncand) __stcg(queue + t, next.y);
                 else atomicOr(&st->spill, 4u);
             }
         }
+        k = __shfl_sync(kFullWarp, k, 0);
     }
+    if (!lead) return;
     if (rewinds) atomicAdd(&C->rewinds, rewinds);
     atomicMax(&st->rounds, maxDepth);
     atomicMax(&C->caCritMicros, maxCrit / 1000u);
@@ -2606,26 +2673,29 @@ __global__ void caWidenKernel(const BodyArrays B, const uint64_t* pairKeys, uint
     }
 }
 
-// The reference's loop verbatim in pair order (one thread): the fallback when
+// The reference's loop verbatim in pair order (one warp): the fallback when
 // a rewind cascades beyond the candidate neighbourhood.
-__global__ void caFullSerialKernel(BodyArrays B, Soup soup, const uint64_t* pairKeys, uint32_t npairs,
+__global__ void __launch_bounds__(32) caFullSerialKernel(BodyArrays B, Soup soup, const uint64_t* pairKeys, uint32_t npairs,
                                    const uint32_t* flags, uint32_t* rewound, float dt, const float4* prevPos,
                                    const float4* prevRot, Counters* C) {
-    if (blockIdx.x != 0 || threadIdx.x != 0) return;
     uint32_t rewinds = 0;
     for (uint32_t r = 0; r < npairs; ++r) {
         const uint64_t key = pairKeys[r];
         const uint32_t ri = (uint32_t)(key >> 32), rj = (uint32_t)key;
-        if (!(flags[r] || rewound[ri] || rewound[rj])) continue;
+        if (!(flags[r] || __ldcg(rewound + ri) || __ldcg(rewound + rj))) continue;
         uint32_t i, j;
         orientPair(B, key, i, j);
         if (caRewind(B, soup, i, j, dt, prevPos, prevRot, &C->caGapQueries, nullptr)) {
             ++rewinds;
-            rewound[i] = 1;
-            if (isDynamic(B.filt[j].x)) rewound[j] = 1;
+            if (threadIdx.x == 0) {
+                __stcg(rewound + i, 1u);
+                if (isDynamic(B.filt[j].x)) __stcg(rewound + j, 1u);
+                __threadfence();
+            }
         }
+        __syncwarp();
     }
-    C->rewinds = rewinds;
+    if (threadIdx.x == 0) C->rewinds = rewinds;
 }
 
 __global__ void copyStateKernel(const BodyArrays B, uint32_t n, float4* snap, int restore) {
@@ -2996,6 +3066,19 @@ static int broadPhase(Context& c, float dt, uint32_t* pairCount) {
 
 // ---- narrow phase ---------------------------------------------------------
 
+// Launch of a warp-per-item kernel over at most `items` items: no more blocks
+// than run at once.
+template <class Kernel, class... Args>
+static int launchQueries(Context& c, uint32_t items, Kernel kernel, Args... args) {
+    int perSm = 0;
+    VXB_CUDA(c, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSm, kernel, kQueryThreads, kQuerySmem));
+    const uint32_t grid = std::min<uint32_t>(blocksFor(items, kQueryThreads / 32),
+                                             (uint32_t)(std::max(perSm, 1) * c.smCount));
+    kernel<<<grid, kQueryThreads, kQuerySmem, c.stream>>>(args...);
+    ++c.launches;
+    return VXB_OK;
+}
+
 // Runs the narrow phase on `npairs` device pairs and leaves the contacts
 // sorted in contactBuf[c.cur] (mode 0) or grouped in pair order (mode 1).
 // World path: `pairs` holds convexSplit convex-convex pairs and `planePairs`
@@ -3011,7 +3094,7 @@ static int narrowPhase(Context& c, const uint64_t* pairs, uint32_t npairs, float
         VXB_TRY(ensure(c, c.recKeyBuf, (size_t)c.recCap * 8));
         VXB_TRY(ensure(c, c.recValBuf, (size_t)c.recCap * 4));
         VXB_TRY(ensure(c, c.recInfoBuf, (size_t)c.recCap * 8));
-        VXB_CUDA(c, cudaMemsetAsync(&c.dCounters->contactsTmp, 0, 8, c.stream));  // contactsTmp + records
+        VXB_CUDA(c, cudaMemsetAsync(&c.dCounters->contactsTmp, 0, 12, c.stream));  // contactsTmp, records, hardPairs
         VXB_CUDA(c, cudaMemsetAsync(&c.dCounters->overflow, 0, 4, c.stream));
         stageBegin(c, kStageNarrowphase);
         vx_contact* tmp = P<vx_contact>(c.contactTmpBuf);
@@ -3031,29 +3114,34 @@ static int narrowPhase(Context& c, const uint64_t* pairs, uint32_t npairs, float
                     VXB_TRY(sortPairs(c, P<uint64_t>(c.classKeyBuf), P<uint32_t>(c.classValBuf), convexSplit, 8));
                 }
                 const uint32_t* order = P<uint32_t>(c.classValBuf);
+                VXB_TRY(ensure(c, c.hardBuf, (size_t)convexSplit * (4 + sizeof(HardResult)) + 64));
+                HardResult* results = P<HardResult>(c.hardBuf);
+                uint32_t* hard = reinterpret_cast<uint32_t*>(results + convexSplit);
                 VXB_TRY(tunedLaunch(c, kTuneCollideConvex, convexSplit, [&](LaunchShape sh) {
                     LAUNCH(c, collideKernel<kConvexPairs>, sh.grid(convexSplit, c.smCount), sh.threads, c.B, soupOf(c),
                            pairs, order, convexSplit, dt, mode, bodyBits, tmp, c.contactCap, recKeys, recVals, recInfo,
-                           c.recCap, c.dCounters);
+                           c.recCap, hard, (const HardResult*)nullptr, c.dCounters);
                 }, CounterRestore{c}));
-                if (c.complexShapes)
-                    VXB_TRY(tunedLaunch(c, kTuneCollideComplex, convexSplit, [&](LaunchShape sh) {
-                        LAUNCH(c, collideKernel<kComplexPairs>, sh.grid(convexSplit, c.smCount), sh.threads, c.B,
-                               soupOf(c), pairs, order, convexSplit, dt, mode, bodyBits, tmp, c.contactCap, recKeys,
-                               recVals, recInfo, c.recCap, c.dCounters);
-                    }, CounterRestore{c}));
+                const int rc = launchQueries(c, convexSplit, collideHardKernel, c.B, soupOf(c), pairs,
+                                             (const uint32_t*)hard, dt, mode, bodyBits, tmp, c.contactCap, recKeys,
+                                             recVals, recInfo, c.recCap, results, c.dCounters);
+                if (rc != VXB_OK) return rc;
+                LAUNCH(c, collideKernel<kListedPairs>, blocksFor(convexSplit, 64, (uint32_t)c.smCount * 16), 64, c.B,
+                       soupOf(c), pairs, (const uint32_t*)hard, convexSplit, dt, mode, bodyBits, tmp, c.contactCap,
+                       recKeys, recVals, recInfo, c.recCap, (uint32_t*)nullptr, (const HardResult*)results,
+                       c.dCounters);
             }
             if (np)
                 VXB_TRY(tunedLaunch(c, kTuneCollidePlane, np, [&](LaunchShape sh) {
                     LAUNCH(c, collideKernel<kPlanePairs>, sh.grid(np, c.smCount), sh.threads, c.B, soupOf(c), planePairs,
                            (const uint32_t*)nullptr, np, dt, mode, bodyBits, tmp, c.contactCap, recKeys, recVals,
-                           recInfo, c.recCap, c.dCounters);
+                           recInfo, c.recCap, (uint32_t*)nullptr, (const HardResult*)nullptr, c.dCounters);
                 }, CounterRestore{c}));
         } else if (npairs) {
             VXB_TRY(tunedLaunch(c, kTuneCollideAny, npairs, [&](LaunchShape sh) {
                 LAUNCH(c, collideKernel<kAnyPairs>, sh.grid(npairs, c.smCount), sh.threads, c.B, soupOf(c), pairs,
                        (const uint32_t*)nullptr, npairs, dt, mode, bodyBits, tmp, c.contactCap, recKeys, recVals,
-                       recInfo, c.recCap, c.dCounters);
+                       recInfo, c.recCap, (uint32_t*)nullptr, (const HardResult*)nullptr, c.dCounters);
             }, CounterRestore{c}));
         }
         stageEnd(c, kStageNarrowphase);
@@ -3105,11 +3193,6 @@ static int launchCooperativeSmem(Context& c, int maxPerSm, size_t smem, Kernel k
                                     c.stream);
     ++c.launches;
     return cudaStatus(c, e, "cudaLaunchCooperativeKernel");
-}
-
-template <class Kernel, class... Args>
-static int launchCooperativeCapped(Context& c, int maxPerSm, Kernel kernel, int threads, Args... args) {
-    return launchCooperativeSmem(c, maxPerSm, 0, kernel, threads, args...);
 }
 
 template <class Kernel, class... Args>
@@ -3561,11 +3644,19 @@ static int conservativeAdvancement(Context& c, uint32_t npairs, float dt) {
         VXB_TRY(sortPairs(c, P<uint64_t>(c.classKeyBuf), P<uint32_t>(c.classValBuf), npairs, 8));
         probeOrder = P<uint32_t>(c.classValBuf);
     }
-    // the probe writes each pair's outcome at its own index and only sets marks: trials need no restore
+    // the probe writes each pair's outcome at its own index and only sets marks: trials restore its list's length
+    uint32_t* hard = queue;
+    auto emptyList = [&]() -> int {
+        VXB_CUDA(c, cudaMemsetAsync(&c.dCounters->caHard, 0, 4, c.stream));
+        return VXB_OK;
+    };
+    VXB_TRY(emptyList());
     VXB_TRY(tunedLaunch(c, kTuneProbe, npairs, [&](LaunchShape sh) {
-        LAUNCH(c, caProbeKernel, sh.grid(npairs, c.smCount), sh.threads, c.B, soupOf(c), pk, probeOrder, npairs, dt,
-               flags, bodyMark, endGap);
-    }, [] { return (int)VXB_OK; }));
+        LAUNCH(c, caProbeKernel, sh.grid(npairs, c.smCount), sh.threads, c.B, soupOf(c), pk, probeOrder, npairs,
+               flags, bodyMark, endGap, hard, c.dCounters);
+    }, emptyList));
+    VXB_TRY(launchQueries(c, npairs, caProbeHardKernel, c.B, soupOf(c), pk, (const uint32_t*)hard, dt, flags, bodyMark,
+                          endGap, (const Counters*)c.dCounters));
     // speculative outcomes of the flagged pairs on the probe's state
     VXB_TRY(exclusiveScan(c, flags, flagRank, npairs, &c.dCounters->caFlagged));
     VXB_TRY(readCounters(c));
@@ -3576,15 +3667,8 @@ static int conservativeAdvancement(Context& c, uint32_t npairs, float dt) {
     uint32_t* specResult = reinterpret_cast<uint32_t*>(specState + 8 * (size_t)flagged);
     uint32_t* flaggedList = specResult + flagged;
     LAUNCH(c, compactKernel, blocksFor(npairs, 256), 256, flags, flagRank, npairs, flaggedList);
-    // Spread the flagged pairs evenly over all SMs, one single-warp block per
-    // group of `lanes` pairs: a distance query's latency grows with the number
-    // of stack frames live on its SM (local memory shares the SM's L1), so a
-    // few flagged pairs run one per SM rather than packed into a few warps.
-    uint32_t lanes = 1;
-    while (lanes < 32 && (size_t)lanes * c.smCount < flagged) lanes <<= 1;
-    const uint32_t spread = 32u / lanes;
-    LAUNCH(c, caSpeculateKernel, (flagged + lanes - 1) / lanes, 32, c.B, soupOf(c), pk, (const uint32_t*)flaggedList,
-           flagged, spread, (const float4*)endGap, dt, prevPos, prevRot, specState, specResult, c.dCounters);
+    VXB_TRY(launchQueries(c, flagged, caSpeculateKernel, c.B, soupOf(c), pk, (const uint32_t*)flaggedList, flagged,
+                          (const float4*)endGap, dt, prevPos, prevRot, specState, specResult, c.dCounters));
     // mark ahead of the cascade before the first pass too (fewer replays)
     {
         const uint32_t* frontier = bodyMark;
@@ -3628,7 +3712,7 @@ static int conservativeAdvancement(Context& c, uint32_t npairs, float dt) {
         }
         VXB_CUDA(c, cudaMemsetAsync(queue, 0xff, (size_t)ncand * 4, c.stream));
         VXB_TRY(resetCoop(c, st));
-        const int rc = launchCooperativeCapped(c, kCaFlowBlocksPerSm, caFlowKernel, kCaFlowThreads, c.B, soupOf(c),
+        const int rc = launchCooperativeSmem(c, kCaFlowBlocksPerSm, kQuerySmem, caFlowKernel, kQueryThreads, c.B, soupOf(c),
                                                (const uint32_t*)flagRank, (const float4*)specState,
                                                (const uint32_t*)specResult, (const uint4*)info, ncand,
                                                (const uint32_t*)succ, pending, queue, depth, crit,
@@ -3662,8 +3746,9 @@ static int conservativeAdvancement(Context& c, uint32_t npairs, float dt) {
     if (serial) {
         if (snapped) LAUNCH(c, copyStateKernel, blocksFor(n, 256), 256, c.B, n, P<float4>(c.snapBuf), 1);
         VXB_CUDA(c, cudaMemsetAsync(rewound, 0, (size_t)n * 4, c.stream));
-        LAUNCH(c, caFullSerialKernel, 1, 32, c.B, soupOf(c), pk, npairs, flags, rewound, dt, prevPos, prevRot,
-               c.dCounters);
+        caFullSerialKernel<<<1, 32, sizeof(WarpQuery), c.stream>>>(c.B, soupOf(c), pk, npairs, flags, rewound, dt,
+                                                                   prevPos, prevRot, c.dCounters);
+        ++c.launches;
     }
     return VXB_OK;
 }
@@ -3862,28 +3947,56 @@ int stageColor(Context& c, const vx_contact* contacts, uint32_t m, int32_t* colo
     return VXB_OK;
 }
 
-__global__ void distanceKernel(BodyArrays B, Soup soup, const uint64_t* pairs, uint32_t npairs, int path,
-                               float* out) {
+VXD void storeDistance(const GjkResult& r, float* o) {
+    o[0] = r.distance;
+    o[1] = r.normal.x; o[2] = r.normal.y; o[3] = r.normal.z;
+    o[4] = r.pointA.x; o[5] = r.pointA.y; o[6] = r.pointA.z;
+    o[7] = r.pointB.x; o[8] = r.pointB.y; o[9] = r.pointB.z;
+    o[10] = r.overlapping ? 1.0f : 0.0f;
+}
+
+__global__ void distanceKernel(BodyArrays B, Soup soup, const uint64_t* pairs, uint32_t npairs, int path, float* out,
+                               uint32_t* hard, Counters* C) {
     for (uint32_t p = blockIdx.x * blockDim.x + threadIdx.x; p < npairs; p += gridDim.x * blockDim.x) {
         const Convex ca = makeConvex(loadView(B, (uint32_t)(pairs[p] >> 32)), soup);
         const Convex cb = makeConvex(loadView(B, (uint32_t)pairs[p]), soup);
-        const GjkResult r = path == 0 ? distanceQuery(ca, cb) : gjkDistance(ca, cb);
-        float* o = out + 11 * (size_t)p;
-        o[0] = r.distance;
-        o[1] = r.normal.x; o[2] = r.normal.y; o[3] = r.normal.z;
-        o[4] = r.pointA.x; o[5] = r.pointA.y; o[6] = r.pointA.z;
-        o[7] = r.pointB.x; o[8] = r.pointB.y; o[9] = r.pointB.z;
-        o[10] = r.overlapping ? 1.0f : 0.0f;
+        GjkResult r;
+        Simplex s;
+        if (path != 0) r = gjkDistance(ca, cb);
+        else if (gjkDistanceFast(ca, cb, r, s) != kGjkSeparated) { hard[aggregatedSlot(&C->hardPairs)] = p; continue; }
+        storeDistance(r, out + 11 * (size_t)p);
+    }
+}
+
+__global__ void __launch_bounds__(kQueryThreads) distanceHardKernel(BodyArrays B, Soup soup, const uint64_t* pairs,
+                                                                    const uint32_t* hard, float* out,
+                                                                    const Counters* C) {
+    const uint32_t count = C->hardPairs, warps = (gridDim.x * blockDim.x) >> 5;
+    for (uint32_t k = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; k < count; k += warps) {
+        const uint32_t p = hard[k];
+        const Convex ca = makeConvex(loadView(B, (uint32_t)(pairs[p] >> 32)), soup);
+        const Convex cb = makeConvex(loadView(B, (uint32_t)pairs[p]), soup);
+        const GjkResult r = gjkDistanceWarp(ca, cb);
+        if (warpLane() == 0u) storeDistance(r, out + 11 * (size_t)p);
+        __syncwarp();
     }
 }
 
 int stageDistance(Context& c, const uint64_t* pairs, uint32_t npairs, int path, float* out) {
     if (npairs == 0) return VXB_OK;
+    VXB_TRY(ensure(c, c.countersBuf, sizeof(Counters)));
+    c.dCounters = P<Counters>(c.countersBuf);
     VXB_TRY(ensure(c, c.pairBuf, (size_t)npairs * 8 + 16));
     VXB_TRY(ensure(c, c.contactTmpBuf, (size_t)npairs * 44 + 16));
+    VXB_TRY(ensure(c, c.hardBuf, (size_t)npairs * 4 + 64));
     VXB_CUDA(c, cudaMemcpyAsync(c.pairBuf.ptr, pairs, (size_t)npairs * 8, cudaMemcpyHostToDevice, c.stream));
+    VXB_CUDA(c, cudaMemsetAsync(&c.dCounters->hardPairs, 0, 4, c.stream));
     LAUNCH(c, distanceKernel, blocksFor(npairs, 64), 64, c.B, soupOf(c), P<uint64_t>(c.pairBuf), npairs, path,
-           P<float>(c.contactTmpBuf));
+           P<float>(c.contactTmpBuf), P<uint32_t>(c.hardBuf), c.dCounters);
+    if (path == 0)
+        VXB_TRY(launchQueries(c, npairs, distanceHardKernel, c.B, soupOf(c), (const uint64_t*)P<uint64_t>(c.pairBuf),
+                              (const uint32_t*)P<uint32_t>(c.hardBuf), P<float>(c.contactTmpBuf),
+                              (const Counters*)c.dCounters));
     VXB_CUDA(c, cudaMemcpyAsync(out, c.contactTmpBuf.ptr, (size_t)npairs * 44, cudaMemcpyDeviceToHost, c.stream));
     VXB_CUDA(c, cudaStreamSynchronize(c.stream));
     return VXB_OK;
