@@ -596,10 +596,10 @@ struct WorldRun {
         a.v = f3(rec[0]); a.w = f3(rec[1]); b.v = f3(rec[2]); b.w = f3(rec[3]);
         const float ln = rec[0].w, l1 = rec[1].w, l2 = rec[2].w;
         const V3 n{cc.normal.x, cc.normal.y, cc.normal.z};
-        // replay of sweepRow's arithmetic (identical branch decisions)
+        // replay of sweepRow's arithmetic (identical branch decisions; the signs of zeros do not matter here)
         const float ima = solverInvMass(a.m), imb = solverInvMass(b.m);
         const bool dynA = isDynamic(a.m.flags), dynB = isDynamic(b.m.flags);
-        const float vn = dot((a.v + cross(a.w, P.ra)) - (b.v + cross(b.w, P.rb)), n);
+        const float vn = dot((a.v + crossRaw(a.w, P.ra)) - (b.v + crossRaw(b.w, P.rb)), n);
         float target = P.targetBase;
         bool resMax = false;
         if (cc.vn0 < -1.0f && (P.liveGap <= 0.0f || vn > 0.0f)) {
@@ -615,8 +615,8 @@ struct WorldRun {
         const float dn = lnp - ln;
         const V3 ni = n * dn;
         SolverBody a1 = a, b1 = b;
-        if (dynA) { a1.v += ni * ima; a1.w += invIF(a1, cross(P.ra, ni)); }
-        if (dynB) { b1.v -= ni * imb; b1.w -= invIF(b1, cross(P.rb, ni)); }
+        if (dynA) { a1.v += ni * ima; a1.w += rowInvIF<false>(a1, crossRaw(P.ra, ni)); }
+        if (dynB) { b1.v -= ni * imb; b1.w -= rowInvIF<false>(b1, crossRaw(P.rb, ni)); }
         const float iA = isoInvI(a.m), iB = isoInvI(b.m);
         const Mass& mA = a.m;
         const Mass& mB = b.m;
@@ -628,7 +628,7 @@ struct WorldRun {
         PrepBar& Pb = V.pbar[j];
         float gImA = 0.0f, gIiA = 0.0f, gImB = 0.0f, gIiB = 0.0f;
         if (P.k1 > 0.0f && P.k2 > 0.0f) {
-            const V3 rv = (a1.v + cross(a1.w, P.ra)) - (b1.v + cross(b1.w, P.rb));
+            const V3 rv = (a1.v + crossRaw(a1.w, P.ra)) - (b1.v + crossRaw(b1.w, P.rb));
             const float rv1 = dot(rv, P.t1), rv2 = dot(rv, P.t2);
             const float next1 = l1 - rv1 / P.k1;
             const float next2 = l2 - rv2 / P.k2;

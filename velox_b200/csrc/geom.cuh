@@ -11,6 +11,8 @@
 // address global or shared memory, and the scratch of EPA and clipping lives
 // in per-thread local arrays sized to the reference's limits.
 #pragma once
+#include <climits>
+
 #include "vmath.cuh"
 #include "velox_b200_types.h"
 
@@ -1603,6 +1605,17 @@ VXD V3 invIF(const SolverBody& b, const V3& v) {
     return rotate(b.frame, V3{l.x * b.m.invI.x, l.y * b.m.invI.y, l.z * b.m.invI.z});
 }
 
+// invIF and cross whose zero components may carry the other sign (Exact = false).
+template <bool Exact>
+VXD V3 rowCross(const V3& a, const V3& b) { return Exact ? cross(a, b) : crossRaw(a, b); }
+template <bool Exact>
+VXD V3 rowInvIF(const SolverBody& b, const V3& v) {
+    if (Exact) return invIF(b, v);
+    if (!isDynamic(b.m.flags) || isRotationLocked(b.m.flags)) return V3{0.0f, 0.0f, 0.0f};
+    const V3 l = rotateRaw(Q4{-b.frame.x, -b.frame.y, -b.frame.z, b.frame.w}, v);
+    return rotateRaw(b.frame, V3{l.x * b.m.invI.x, l.y * b.m.invI.y, l.z * b.m.invI.z});
+}
+
 // The contact fields the solver reads and writes.
 struct RowContact {
     V3 normal, point, la, lb;
@@ -1828,13 +1841,37 @@ VXD void warmPrepRow(SolverBody& a, SolverBody& b, RowContact& c, const RowPrep&
     }
 }
 
+// The friction impulses lie well inside the ellipse: its exact value (two
+// divisions) would not exceed 1, so nothing is rescaled. Holds per axis for
+// |n| <= 0.7 max (0.49 + 0.49 plus rounding stays below 1; max is far from
+// where its square loses precision) or an axis without friction.
+VXD bool insideAxis(float n, float mx) { return (mx <= 0.0f) | ((mx > 1e-10f) & (fabsf(n) <= 0.7f * mx)); }
+
+// -0.0f is the smallest signed integer.
+VXD int negativeZeroKey(float a, float b, float c, float d, float e) {
+    return min(min(__float_as_int(a), min(__float_as_int(b), __float_as_int(c))),
+               min(__float_as_int(d), __float_as_int(e)));
+}
+
 // One sweep of solveContact (narrowphase.h:130-366) with prepared pose terms.
-VXD void sweepRow(SolverBody& a, SolverBody& b, RowContact& c, const RowPrep& P, bool coneBlock) {
+//
+// Exact = false runs it without cross's rule for the sign of zeros, for rows
+// that it provably does not reach. Zeros enter sums and products only, so no
+// non-zero value depends on their signs. A zero's sign survives
+//   in w +- dw only where w is -0, and a w that is not -0 does not become -0;
+//   in n - dot(rv, t) / k (the tangent impulses) only where n is -0;
+//   nowhere in the normal impulse: vmax returns +0.
+// Those cases and rows with rolling or spinning terms take Exact = true. The
+// rule is a quarter of a row's instructions: solve stage of one step with
+// 187,000 small islands 6.4 -> 5.6 ms, of a heap of 40,000 bodies 9.9 -> 9.2 ms;
+// backward pass of 128 rollouts of 24 steps 210 -> 186 ms.
+template <bool Exact>
+VXD void sweepRowAs(SolverBody& a, SolverBody& b, RowContact& c, const RowPrep& P, bool coneBlock) {
     c.point = P.point;
     if (P.kNormal <= 0.0f) return;
     const float ima = solverInvMass(a.m), imb = solverInvMass(b.m);
     const bool dynA = isDynamic(a.m.flags), dynB = isDynamic(b.m.flags);
-    const float vn = dot((a.v + cross(a.w, P.ra)) - (b.v + cross(b.w, P.rb)), c.normal);
+    const float vn = dot((a.v + rowCross<Exact>(a.w, P.ra)) - (b.v + rowCross<Exact>(b.w, P.rb)), c.normal);
     float target = P.targetBase;
     if (c.vn0 < -1.0f && (P.liveGap <= 0.0f || vn > 0.0f)) target = vmax(target, -c.restitution * c.vn0);
     if (!coneBlock) {
@@ -1843,10 +1880,10 @@ VXD void sweepRow(SolverBody& a, SolverBody& b, RowContact& c, const RowPrep& P,
         jn = nextNormal - c.nImp;
         c.nImp = nextNormal;
         const V3 ni = c.normal * jn;
-        if (dynA) { a.v += ni * ima; a.w += invIF(a, cross(P.ra, ni)); }
-        if (dynB) { b.v -= ni * imb; b.w -= invIF(b, cross(P.rb, ni)); }
+        if (dynA) { a.v += ni * ima; a.w += rowInvIF<Exact>(a, rowCross<Exact>(P.ra, ni)); }
+        if (dynB) { b.v -= ni * imb; b.w -= rowInvIF<Exact>(b, rowCross<Exact>(P.rb, ni)); }
         if (P.k1 > 0.0f && P.k2 > 0.0f) {
-            const V3 rv = (a.v + cross(a.w, P.ra)) - (b.v + cross(b.w, P.rb));
+            const V3 rv = (a.v + rowCross<Exact>(a.w, P.ra)) - (b.v + rowCross<Exact>(b.w, P.rb));
             const float old1 = c.t1Imp, old2 = c.t2Imp;
             float next1 = old1 - dot(rv, P.t1) / P.k1;
             float next2 = old2 - dot(rv, P.t2) / P.k2;
@@ -1854,18 +1891,20 @@ VXD void sweepRow(SolverBody& a, SolverBody& b, RowContact& c, const RowPrep& P,
             const float max2 = c.friction2 * c.nImp;
             if (max1 <= 0.0f) next1 = 0.0f;
             if (max2 <= 0.0f) next2 = 0.0f;
-            const float ellipse = (max1 > 0.0f ? next1 * next1 / (max1 * max1) : 0.0f) +
-                                  (max2 > 0.0f ? next2 * next2 / (max2 * max2) : 0.0f);
-            if (ellipse > 1.0f) {
-                const float sc = 1.0f / sqrtf(ellipse);
-                next1 *= sc;
-                next2 *= sc;
+            if (!(insideAxis(next1, max1) & insideAxis(next2, max2))) {
+                const float ellipse = (max1 > 0.0f ? next1 * next1 / (max1 * max1) : 0.0f) +
+                                      (max2 > 0.0f ? next2 * next2 / (max2 * max2) : 0.0f);
+                if (ellipse > 1.0f) {
+                    const float sc = 1.0f / sqrtf(ellipse);
+                    next1 *= sc;
+                    next2 *= sc;
+                }
             }
             c.t1Imp = next1;
             c.t2Imp = next2;
             const V3 fi = P.t1 * (next1 - old1) + P.t2 * (next2 - old2);
-            if (dynA) { a.v += fi * ima; a.w += invIF(a, cross(P.ra, fi)); }
-            if (dynB) { b.v -= fi * imb; b.w -= invIF(b, cross(P.rb, fi)); }
+            if (dynA) { a.v += fi * ima; a.w += rowInvIF<Exact>(a, rowCross<Exact>(P.ra, fi)); }
+            if (dynB) { b.v -= fi * imb; b.w -= rowInvIF<Exact>(b, rowCross<Exact>(P.rb, fi)); }
         }
     } else {
         const float oldNormal = c.nImp;
@@ -1876,7 +1915,7 @@ VXD void sweepRow(SolverBody& a, SolverBody& b, RowContact& c, const RowPrep& P,
             const float det = kNormal * (k1 * k2 - k12 * k12) - kN1 * (kN1 * k2 - kN2 * k12) +
                               kN2 * (kN1 * k12 - kN2 * k1);
             if (fabsf(det) > 1e-12f) {
-                const V3 rv = (a.v + cross(a.w, P.ra)) - (b.v + cross(b.w, P.rb));
+                const V3 rv = (a.v + rowCross<Exact>(a.w, P.ra)) - (b.v + rowCross<Exact>(b.w, P.rb));
                 const float bN = target - dot(rv, c.normal);
                 const float b1 = -dot(rv, P.t1);
                 const float b2 = -dot(rv, P.t2);
@@ -1906,9 +1945,10 @@ VXD void sweepRow(SolverBody& a, SolverBody& b, RowContact& c, const RowPrep& P,
         c.t1Imp = next1;
         c.t2Imp = next2;
         const V3 imp = c.normal * (nextNormal - oldNormal) + P.t1 * (next1 - old1) + P.t2 * (next2 - old2);
-        if (dynA) { a.v += imp * ima; a.w += invIF(a, cross(P.ra, imp)); }
-        if (dynB) { b.v -= imp * imb; b.w -= invIF(b, cross(P.rb, imp)); }
+        if (dynA) { a.v += imp * ima; a.w += rowInvIF<Exact>(a, rowCross<Exact>(P.ra, imp)); }
+        if (dynB) { b.v -= imp * imb; b.w -= rowInvIF<Exact>(b, rowCross<Exact>(P.rb, imp)); }
     }
+    if (!Exact) return;
     if (c.rolling > 0.0f && P.kr1 > 0.0f && P.kr2 > 0.0f) {
         const V3 wr = a.w - b.w;
         const float o1 = c.r1Imp, o2 = c.r2Imp;
@@ -1924,8 +1964,8 @@ VXD void sweepRow(SolverBody& a, SolverBody& b, RowContact& c, const RowPrep& P,
         c.r1Imp = n1;
         c.r2Imp = n2;
         const V3 tq = P.t1 * (n1 - o1) + P.t2 * (n2 - o2);
-        if (dynA) a.w += invIF(a, tq);
-        if (dynB) b.w -= invIF(b, tq);
+        if (dynA) a.w += rowInvIF<Exact>(a, tq);
+        if (dynB) b.w -= rowInvIF<Exact>(b, tq);
     }
     if (c.spinning > 0.0f && P.ks > 0.0f) {
         const V3 wr = a.w - b.w;
@@ -1935,9 +1975,31 @@ VXD void sweepRow(SolverBody& a, SolverBody& b, RowContact& c, const RowPrep& P,
         next = vclamp(next, -limit, limit);
         c.sImp = next;
         const V3 tq = c.normal * (next - old);
-        if (dynA) a.w += invIF(a, tq);
-        if (dynB) b.w -= invIF(b, tq);
+        if (dynA) a.w += rowInvIF<Exact>(a, tq);
+        if (dynB) b.w -= rowInvIF<Exact>(b, tq);
     }
+}
+
+static __device__ __noinline__ void sweepRowExact(SolverBody& a, SolverBody& b, RowContact& c, const RowPrep& P,
+                                           bool coneBlock) {
+    sweepRowAs<true>(a, b, c, P, coneBlock);
+}
+
+VXD void sweepRow(SolverBody& a, SolverBody& b, RowContact& c, const RowPrep& P, bool coneBlock) {
+    const bool special = c.rolling > 0.0f || c.spinning > 0.0f ||
+                         negativeZeroKey(a.w.x, a.w.y, a.w.z, c.t1Imp, c.t2Imp) == INT_MIN ||
+                         negativeZeroKey(b.w.x, b.w.y, b.w.z, c.t1Imp, c.t2Imp) == INT_MIN;
+    if (special) {  // copies: only this path needs them in memory
+        SolverBody ea = a, eb = b;
+        RowContact ec = c;
+        const RowPrep ep = P;
+        sweepRowExact(ea, eb, ec, ep, coneBlock);
+        a.v = ea.v; a.w = ea.w;
+        b.v = eb.v; b.w = eb.w;
+        c = ec;
+        return;
+    }
+    sweepRowAs<false>(a, b, c, P, coneBlock);
 }
 
 }  // namespace vxb

@@ -2128,7 +2128,7 @@ VXD bool clusterStep(const SolveArgs& A, const uint32_t* start, const uint32_t* 
     return *abortFlag == 0;
 }
 
-__global__ void __launch_bounds__(kClusterThreads) solveClusterKernel(SolveArgs A, uint32_t G, const uint32_t* start,
+__global__ void __launch_bounds__(kClusterThreads, 2) solveClusterKernel(SolveArgs A, uint32_t G, const uint32_t* start,
                                                           const uint32_t* rows, const uint32_t* rowList, uint32_t R,
                                                           const uint32_t* bodyIds, uint32_t NB, const uint32_t* pred,
                                                           const uint32_t* remote, uint32_t* done, CoopState* st) {

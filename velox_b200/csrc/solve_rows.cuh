@@ -28,8 +28,6 @@
 // lane per row with the same planes (about equal for narrow colours, slower
 // for wide ones).
 #pragma once
-#include <climits>
-
 #include "geom.cuh"
 
 namespace vxb {
@@ -215,9 +213,6 @@ struct LaneBody {
     bool dyn, turns;
 };
 
-// Exact = false: zero components may carry the other sign (crossRaw).
-template <bool Exact>
-VXD V3 laneCross(const V3& a, const V3& b) { return Exact ? cross(a, b) : crossRaw(a, b); }
 template <bool Exact>
 VXD V3 laneInvI(const LaneBody& b, const V3& x) {  // invIF
     const Q4 inv{-b.frame.x, -b.frame.y, -b.frame.z, b.frame.w};
@@ -239,21 +234,10 @@ VXD V3 laneAdd(const LaneBody& b, uint32_t side, const V3& x, const V3& d) {
 template <bool Exact>
 VXD void laneImpulse(LaneBody& b, uint32_t side, const V3& arm, const V3& imp) {
     b.v = laneAdd(b, side, b.v, imp * b.im);
-    b.w = laneAdd(b, side, b.w, laneInvI<Exact>(b, laneCross<Exact>(arm, imp)));
+    b.w = laneAdd(b, side, b.w, laneInvI<Exact>(b, rowCross<Exact>(arm, imp)));
 }
 VXD void laneTorque(LaneBody& b, uint32_t side, const V3& tq) { b.w = laneAdd(b, side, b.w, laneInvI<true>(b, tq)); }
 
-// -0.0f is the smallest signed integer.
-VXD int negativeZeroKey(float a, float b, float c, float d, float e) {
-    return min(min(__float_as_int(a), min(__float_as_int(b), __float_as_int(c))),
-               min(__float_as_int(d), __float_as_int(e)));
-}
-
-// The friction impulses lie well inside the ellipse: its exact value (two
-// divisions) would not exceed 1, so nothing is rescaled. `inside` holds per
-// axis for |n| <= 0.7 max (0.49 + 0.49 plus rounding stays below 1; max is far
-// from where its square loses precision) or an axis without friction.
-VXD bool insideAxis(float n, float mx) { return (mx <= 0.0f) | ((mx > 1e-10f) & (fabsf(n) <= 0.7f * mx)); }
 // Correctly rounded x / k from y = 1 / k (correctly rounded): Markstein's
 // theorem (IBM J. Res. Dev. 34, 1990), q + (x - k q) y rounded once is the
 // quotient when q is within an ulp of it, which the first correction makes
@@ -292,20 +276,15 @@ VXD void clampToEllipse(uint32_t side, float max1, float max2, float& n1, float&
 // One sweep of one row on the pair's two lanes: sweepRow's arithmetic in the
 // same order (all 32 lanes call; `act`: this lane holds a row to solve).
 //
-// Exact = false runs it without cross's rule for the sign of zeros, for a warp
-// whose rows it provably does not reach. Zeros enter sums and products only,
-// so no non-zero value depends on their signs. A zero's sign survives
-//   in w +- dw only where w is -0, and a w that is not -0 does not become -0;
-//   in n - dot(rv, t) / k (the tangent impulses) only where n is -0;
-//   nowhere in the normal impulse: vmax returns +0.
-// Those cases and rows with rolling or spinning terms take Exact = true.
+// Exact = false as in sweepRowAs: for a warp whose rows have no -0 where it
+// matters and no rolling or spinning terms.
 template <bool Exact, bool Cone>
 VXD void laneSweep(const RowPlanes& R, bool act, uint32_t k, uint32_t side, RowRegs& r, LaneBody& b) {
     const V3 arm = f3(r.s), n = f3(r.n), t1 = f3(r.t1), t2 = f3(r.t2);
     const float k1 = r.t1.w, k2 = r.t2.w;
     float nImp = r.i.x, i1 = r.i.y, i2 = r.i.z;
     V3 ua, ub;
-    pairBoth(b.v + laneCross<Exact>(b.w, arm), side, ua, ub);
+    pairBoth(b.v + rowCross<Exact>(b.w, arm), side, ua, ub);
     const V3 rv0 = ua - ub;
     const float vn = dot(rv0, n);
     const float target = vn > 0.0f ? r.g.y : r.g.x;
@@ -323,7 +302,7 @@ VXD void laneSweep(const RowPlanes& R, bool act, uint32_t k, uint32_t side, RowR
         jn = next - nImp;
         nImp = next;
         laneImpulse<Exact>(b, side, arm, n * jn);
-        pairBoth(b.v + laneCross<Exact>(b.w, arm), side, ua, ub);
+        pairBoth(b.v + rowCross<Exact>(b.w, arm), side, ua, ub);
         const V3 rv = ua - ub;
         const float d1 = dot(rv, t1), d2 = dot(rv, t2);
         float c1, c2;
