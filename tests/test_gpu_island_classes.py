@@ -1,5 +1,5 @@
 """The island solve at the edges of its classes (tiny packs, one warp, one
-block of two sizes, the clustered grid solve) against a plain numpy solve of
+block, the grid's flow) against a plain numpy solve of
 the same contacts, and against the same islands solved next to others."""
 import numpy as np
 import pytest

@@ -104,6 +104,8 @@ struct Counters {
     uint32_t clusterColours; // most colours of a giant island
     uint32_t giantCount;     // islands the block kernels cannot hold
     uint32_t caHard;         // pairs listed for the probe's warp queries
+    uint32_t flowTooWide;    // a body with more rows than a flow link counts
+    uint32_t pad[3];
 };
 
 // Pipeline stages timed with CUDA events when timing is enabled.
@@ -143,11 +145,11 @@ struct Context {
     uint32_t planContacts = 0; // contacts of the current island plan
     uint32_t planGiants = 0;   // giant islands of the current plan
     uint32_t planLargest = 0;  // contacts of its largest island
-    bool giantLinked = false;  // dataflow links of the plan's giant islands are built
-    bool clusterBuilt = false; // spatial clusters of the plan's giant islands are built
+    bool clusterBuilt = false; // the flow plan of the giant islands is built
     bool tinyPacked = false;   // the plan's tiny islands are packed into warps
     uint32_t tinyCount = 0, tinyPackCount = 0;
-    uint32_t clusterNB = 0, clusterR = 0, clusterG = 0;  // giant bodies, rows, most colours (clustered solve)
+    uint32_t clusterNB = 0, clusterR = 0, clusterG = 0;  // giant bodies, rows, most colours (flow plan)
+    uint32_t clusterCount = 0;                           // warps that the flow plan is cut for
     uint32_t waitLimit = kSpinLimit;  // polls before a device wait gives up (vxb_context_set_wait_limit)
     cudaStream_t ownStream = nullptr;
     cudaStream_t stream = nullptr;
@@ -227,12 +229,11 @@ struct Context {
     DevBuf coopBuf;                     // CoopState of cooperative launches
     DevBuf giantBuf;                    // giant island list (solve)
     DevBuf classKeyBuf, classValBuf;    // convex pairs grouped by shape combination (narrow phase)
-    DevBuf rowBodyBuf;                  // (a, b) per solve-order row (giant islands)
+    DevBuf flowBodyBuf;                 // tagged body records (giant islands)
     DevBuf tinyBuf;                     // tiny-island flags, ranks, list, pack counts/bases/firsts
     DevBuf tinyKeyBuf;                  // tiny islands' colour counts (pack order sort)
     DevBuf clusterInfoBuf, clusterKeyBuf, clusterValBuf, clusterOfBuf, clusterCountBuf, clusterStartBuf,
         clusterRowsBuf;                 // spatial clusters of a giant island
-    DevBuf clusterLinkBuf;              // cross-cluster predecessor links + remote-successor flags
     DevBuf hardBuf;                     // narrow phase: pairs for the warp queries
     DevBuf caInfoBuf;                   // rewind pass: one record per candidate
     DevBuf tuneSaveBuf;                 // launch-shape trials: device copy of the counters

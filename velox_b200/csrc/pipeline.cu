@@ -24,6 +24,7 @@
 
 #include "context.cuh"
 #include "pair_warp.cuh"
+#include "solve_flow.cuh"
 #include "solve_rows.cuh"
 
 namespace vxb {
@@ -1308,7 +1309,7 @@ __global__ void giantCountKernel(const uint32_t* islandStart, const uint32_t* bo
     for (uint32_t isl = blockIdx.x * blockDim.x + threadIdx.x; isl < islands; isl += gridDim.x * blockDim.x) {
         const uint32_t rows = islandStart[isl + 1] - islandStart[isl];
         const uint32_t nb = isl < realIslands ? bodyStart[isl + 1] - bodyStart[isl] : 0u;
-        if (islandClassOf(nb, rows, kTinyLimit) == kGiantIsland) ++count;
+        if (solveClassOf(nb, rows, kTinyLimit) == kGiantIsland) ++count;
     }
     for (int off = 16; off > 0; off >>= 1) count += __shfl_xor_sync(0xffffffffu, count, off);
     if ((threadIdx.x & 31) == 0 && count) atomicAdd(&C->giantCount, count);
@@ -1746,220 +1747,44 @@ VXD void solveTinyPack(const SolveArgs& A, const uint32_t* list, const uint32_t*
     if (has) storeRow(*cp, rc);
 }
 
-// ---- giant islands: the whole grid on one island ----------------------------
-//
-// Islands too large for one block's shared memory run on every block of a
-// cooperative launch, with a grid barrier between colours. Mutable data that
-// other blocks wrote since the last barrier (velocities, poses, impulses, row
-// terms, frames) is read with ld.global.cg and written with st.global.cg, so
-// no SM works from a stale L1 line.
+// ---- giant islands: the plan of the grid's flow (solve_flow.cuh) ---------------
 
-VXD float4 ldcg4(const float4* p) { return __ldcg(p); }
+constexpr uint32_t kNoPred = 0xffffffffu;  // empty queue slot / no successor
 
-// Acquire load / release store at GPU scope: the dataflow's flag handoff
-// without a full fence on either side.
-VXD uint32_t ldAcquire(const uint32_t* p) {
-    uint32_t v;
-    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
-    return v;
-}
-VXD void stRelease(uint32_t* p, uint32_t v) {
-    asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
-}
-
-VXD SolverBody coherentBody(const SolveArgs& A, uint32_t id) {
-    SolverBody b;
-    b.p = f3(ldcg4(A.B.pos + id));
-    b.q = q4(ldcg4(A.B.rot + id));
-    b.v = f3(ldcg4(A.B.vel + id));
-    b.w = f3(ldcg4(A.B.ang + id));
-    b.m = loadMass(A.B, id);
-    b.sphere = shapeOf(b.m.flags) == kSphere;
-    if (isDynamic(b.m.flags)) b.frame = q4(ldcg4(A.frames + id));
-    else cacheFrame(b);
-    return b;
-}
-
-// Whole 128-byte contact records through L2 (one thread owns a row per colour).
-VXD void loadContactCoherent(const vx_contact* p, vx_contact& c) {
-    const float4* src = reinterpret_cast<const float4*>(p);
-    float4* dst = reinterpret_cast<float4*>(&c);
-#pragma unroll
-    for (int i = 0; i < (int)(sizeof(vx_contact) / 16); ++i) dst[i] = __ldcg(src + i);
-}
-
-VXD void storeContactCoherent(vx_contact* p, const vx_contact& c) {
-    const float4* src = reinterpret_cast<const float4*>(&c);
-    float4* dst = reinterpret_cast<float4*>(p);
-#pragma unroll
-    for (int i = 0; i < (int)(sizeof(vx_contact) / 16); ++i) __stcg(dst + i, src[i]);
-}
-
-// A row's prepared terms through L2 as 16-byte words: one sector per word and
-// lane, where word-sized loads would fetch each sector four times (the rows of
-// a warp lie 176 bytes apart, and L2-only loads do not keep sectors in L1).
-static_assert(sizeof(RowPrep) % 16 == 0, "prepared rows must be whole 16-byte words");
-
-VXD void coherentPrep(const RowPrep* p, RowPrep& P) {
-    const float4* s = reinterpret_cast<const float4*>(p);
-    float* d = reinterpret_cast<float*>(&P);
-#pragma unroll
-    for (int i = 0; i < (int)(sizeof(RowPrep) / 16); ++i) {
-        const float4 v = __ldcg(s + i);
-        d[4 * i + 0] = v.x;
-        d[4 * i + 1] = v.y;
-        d[4 * i + 2] = v.z;
-        d[4 * i + 3] = v.w;
-    }
-}
-
-VXD void storePrepCoherent(RowPrep* p, const RowPrep& P) {
-    float4* dst = reinterpret_cast<float4*>(p);
-    const float* src = reinterpret_cast<const float*>(&P);
-#pragma unroll
-    for (int i = 0; i < (int)(sizeof(RowPrep) / 16); ++i)
-        __stcg(dst + i, make_float4(src[4 * i + 0], src[4 * i + 1], src[4 * i + 2], src[4 * i + 3]));
-}
-
-// Inputs of one giant row that only the row itself writes (its contact
-// record and its prepared terms; the body ids are fixed): a row fetches them
-// before it waits for its predecessors, so their latency overlaps the wait.
-struct GiantRowIn {
-    uint2 ab;
-    vx_contact* cp;
-    vx_contact cc;
-    RowPrep P;
-};
-
-VXD void giantRowFetch(const SolveArgs& A, uint32_t pos, int op, GiantRowIn& in) {
-    in.ab = A.rowBodies[pos];
-    in.cp = A.contacts + A.order[pos];
-    loadContactCoherent(in.cp, in.cc);
-    if (op == 0 || op == 1) coherentPrep(A.prep + pos, in.P);
-}
-
-// op: 0 warm start, 1 velocity sweep, 2 position row, 3 prepare
-VXD void giantRowRun(const SolveArgs& A, uint32_t pos, int op, GiantRowIn& in) {
-    const uint2 ab = in.ab;
-    vx_contact* cp = in.cp;
-    vx_contact& cc = in.cc;
-    SolverBody a = coherentBody(A, ab.x), b = coherentBody(A, ab.y);
-    if (!solvedContact(a.m.flags, b.m.flags)) return;
-    RowContact r;
-    loadRow(cc, r);
-    if (op == 2) {
-        const float ima = solverInvMass(a.m), imb = solverInvMass(b.m);
-        const float invMassSum = ima + imb;
-        if (invMassSum <= 0.0f) return;
-        const V3 wa = anchorWorld(a.sphere, a.p, a.q, r.la);
-        const V3 wb = anchorWorld(b.sphere, b.p, b.q, r.lb);
-        const float gap = r.bias0 + dot(r.normal, wa - wb);
-        if (gap >= -1e-3f) return;
-        float resolve = 0.6f;
-        if (A.stackStabilization && lengthSq(a.v - b.v) < 1e-4f)
-            resolve += 0.2f * (A.stackStiffness / 1000.0f) / (1.0f + A.stackDamping * A.h);
-        const float push = -resolve * (gap + 1e-3f) / invMassSum;
-        if (isDynamic(a.m.flags) && !isAsleep(a.m.flags))
-            __stcg(A.B.pos + ab.x, pack(a.p + r.normal * (push * ima), 0.0f));
-        if (isDynamic(b.m.flags) && !isAsleep(b.m.flags))
-            __stcg(A.B.pos + ab.y, pack(b.p - r.normal * (push * imb), 0.0f));
-        return;
-    }
-    RowPrep& P = in.P;
-    if (op == 3) {
-        prepRow(a, b, r, A.h, A.coneBlock != 0, P);
-        storePrepCoherent(A.prep + pos, P);
-        return;
-    }
-    if (op == 0) warmPrepRow(a, b, r, P);
-    else sweepRow(a, b, r, P, A.coneBlock != 0);
-    if (isDynamic(a.m.flags)) { __stcg(A.B.vel + ab.x, pack(a.v, 0.0f)); __stcg(A.B.ang + ab.x, pack(a.w, 0.0f)); }
-    if (isDynamic(b.m.flags)) { __stcg(A.B.vel + ab.y, pack(b.v, 0.0f)); __stcg(A.B.ang + ab.y, pack(b.w, 0.0f)); }
-    storeRow(cc, r);
-    storeContactCoherent(cp, cc);
-}
-
-VXD void giantRow(const SolveArgs& A, uint32_t pos, int op) {
-    GiantRowIn in;
-    giantRowFetch(A, pos, op, in);
-    giantRowRun(A, pos, op, in);
-}
-
-// integrateKernel semantics (src/backend_cuda.cu:80-89) on coherent loads.
-VXD void giantIntegrateVelocity(const SolveArgs& A, uint32_t i) {
-    const Mass m = loadMass(A.B, i);
-    if (!isDynamic(m.flags) || isLocked(m.flags) || isAsleep(m.flags)) return;
-    const Q4 q = q4(ldcg4(A.B.rot + i));
-    V3 v = f3(ldcg4(A.B.vel + i));
-    V3 w = f3(ldcg4(A.B.ang + i));
-    const V3 F = f3(A.B.force[i]);
-    const V3 T = f3(A.B.torque[i]);
-    const float4 ex = A.B.extra[i];
-    v += (A.gravity * ex.y + F * solverInvMass(m)) * A.h;
-    w += invInertiaMulAt(m, T, q) * A.h;
-    v *= 1.0f / (1.0f + ex.z * A.h);
-    w *= 1.0f / (1.0f + ex.w * A.h);
-    __stcg(A.B.vel + i, pack(v, 0.0f));
-    __stcg(A.B.ang + i, pack(w, 0.0f));
-}
-
-// integrateTransformsKernel semantics (src/backend_cuda.cu:91-97) on coherent loads.
-VXD void giantIntegrateTransform(const SolveArgs& A, uint32_t i) {
-    const Mass m = loadMass(A.B, i);
-    if (isStaticBody(m.flags) || isLocked(m.flags) || isAsleep(m.flags)) return;
-    V3 p = f3(ldcg4(A.B.pos + i));
-    Q4 q = q4(ldcg4(A.B.rot + i));
-    const V3 v = f3(ldcg4(A.B.vel + i));
-    V3 w = f3(ldcg4(A.B.ang + i));
-    advanceTransform(m, p, q, v, w, A.h);
-    __stcg(A.B.pos + i, pack(p, 0.0f));
-    __stcg(A.B.rot + i, pack(q));
-    __stcg(A.B.ang + i, pack(w, 0.0f));
-}
-
-// Giant islands: every row is linked to the previous row on each of its
-// dynamic bodies (colour order; the body's last row of the previous sweep for
-// its first row). A row may run sweep u once those predecessors have
-// published sweep u (u - 1 across the wrap): the order the colour-by-colour
-// sweep imposes on every body, without a barrier per colour.
-constexpr uint32_t kNoPred = 0xffffffffu;  // no predecessor / empty queue slot
-constexpr uint32_t kWrap = 0x80000000u;    // predecessor from the previous sweep
-
-// Dataflow links of the giant islands' rows: entries (dynamic body, 2k + side)
-// of every row of a giant island, other endpoints keyed n (no link).
+// Entries (dynamic body, 2k + side) of every row of a giant island, other
+// endpoints keyed n (no link).
 __global__ void giantEntryKernel(SolveArgs A, const uint32_t* islandOf, uint32_t m, uint32_t n, uint64_t* keys,
-                                 uint32_t* vals, uint2* rowBodies);
-// For each body run of the sorted entries, the position of its last entry.
-__global__ void giantLastKernel(const uint64_t* keys, uint32_t entries, uint32_t n, uint32_t* lastOf) {
+                                 uint32_t* vals);
+// For each body run of the sorted entries, its first entry and the one behind its last.
+__global__ void flowRunKernel(const uint64_t* keys, uint32_t entries, uint32_t n, uint2* runs, Counters* C) {
+    uint32_t most = 0;
     for (uint32_t p = blockIdx.x * blockDim.x + threadIdx.x; p < entries; p += gridDim.x * blockDim.x) {
         const uint64_t key = keys[p];
-        if (key != (uint64_t)n && (p + 1 == entries || keys[p + 1] != key)) lastOf[key] = p;
+        if (key == (uint64_t)n) continue;
+        if (p == 0 || keys[p - 1] != key) runs[key].x = p;
+        if (p + 1 == entries || keys[p + 1] != key) runs[key].y = p + 1;
+        // longer runs than a link can count: some entry lies kMaxFlowDegree behind its run's start
+        if (p >= kMaxFlowDegree && keys[p - kMaxFlowDegree] == key) most = 1;
     }
+    if (most) atomicOr(&C->flowTooWide, 1u);
 }
-// pred[2k + side]: the previous row on that body in colour order, or (kWrap |
-// the body's last row) for its first row; kNoPred for no dynamic body.
-__global__ void giantPredKernel(const uint64_t* keys, const uint32_t* vals, uint32_t entries, uint32_t n,
-                                const uint32_t* lastOf, uint32_t* pred) {
+// link[2k + side]: the row's rank among its body's rows in colour order and
+// the body's row count; 0 without a dynamic body.
+__global__ void flowLinkKernel(const uint64_t* keys, const uint32_t* vals, uint32_t entries, uint32_t n,
+                               const uint2* runs, uint32_t* link) {
     for (uint32_t p = blockIdx.x * blockDim.x + threadIdx.x; p < entries; p += gridDim.x * blockDim.x) {
         const uint64_t key = keys[p];
-        uint32_t v = kNoPred;
-        if (key != (uint64_t)n)
-            v = p > 0 && keys[p - 1] == key ? (vals[p - 1] >> 1) : (kWrap | (vals[lastOf[key]] >> 1));
-        pred[vals[p]] = v;
+        uint32_t v = 0u;
+        if (key != (uint64_t)n) {
+            const uint2 r = runs[key];
+            v = (p - r.x) | (r.y - r.x) << 14;
+        }
+        link[vals[p]] = v;
     }
 }
 
-// ---- one giant island in spatial clusters -------------------------------
-//
-// The same dataflow with coarser, local steps: the island's bodies are cut
-// into as many spatial clusters (Morton order) as the grid has blocks, each
-// row belongs to the cluster of its first dynamic body, and block c runs its
-// cluster's rows colour by colour with a block barrier between colours. Rows
-// whose predecessor on a body lies in another cluster wait for that row's
-// sweep counter; all others are ordered by the block barrier. Most chain steps
-// therefore stay inside a block. A block takes its (sweep, colour) steps in
-// order, which keeps the earliest unfinished step runnable; waits are bounded.
-
+// Spatial clusters: the islands' bodies in Morton order, cut into as many
+// clusters as the grid has warps.
 VXD uint32_t spreadBits10(uint32_t v) {  // 10 bits -> every third bit
     v &= 0x3ffu;
     v = (v | (v << 16)) & 0x030000ffu;
@@ -2004,187 +1829,34 @@ VXD uint32_t segmentOf(const uint32_t* segStart, uint32_t g0, uint32_t g1, uint3
     return lo;
 }
 
-VXD uint32_t rowCluster(const SolveArgs& A, uint32_t k, const uint32_t* clusterOf) {
-    const uint2 ab = A.rowBodies[k];
-    return clusterOf[isDynamic(A.B.filt[ab.x].x) ? ab.x : ab.y];
-}
-
-// (cluster, colour slot) cell of a giant row: colour slot = colour within its
-// island. Rows of the null island (no dynamic body of their own island) go to
-// cluster 0: they are never solved and link to nothing.
-VXD uint32_t rowBlock(const SolveArgs& A, uint32_t k, const uint32_t* islandOf, const uint32_t* clusterOf) {
-    return islandOf[k] < A.realIslands ? rowCluster(A, k, clusterOf) : 0u;
-}
-
+// (warp, colour slot) cell of a giant row: the cluster of its first dynamic
+// body, colour within its island. Rows of the null island (no dynamic body of
+// their own island) have no links and go to any warp.
 VXD uint32_t rowCell(const SolveArgs& A, uint32_t k, const uint32_t* islandOf, const uint32_t* clusterOf,
-                     uint32_t G) {
+                     uint32_t clusters, uint32_t G) {
     const uint32_t isl = islandOf[k];
     const uint32_t g0 = A.islandSeg[isl], g1 = A.islandSeg[isl + 1];
-    return rowBlock(A, k, islandOf, clusterOf) * G + (segmentOf(A.segStart, g0, g1, k) - g0);
-}
-
-// Links the clustered solve waits on. A predecessor in the row's own cluster
-// ran in the same block, in an earlier (sweep, colour) step: a same-sweep
-// predecessor has a lower colour of the same island, a wrapped one belongs to
-// the previous sweep, and the block barrier after every step orders it. Only
-// predecessors in other clusters stay linked (clusterPred), and only rows that
-// such a link names publish their sweep counter (remote = 1).
-__global__ void clusterLinkKernel(SolveArgs A, const uint32_t* rowList, uint32_t R, const uint32_t* islandOf,
-                                  const uint32_t* clusterOf, const uint32_t* pred, uint32_t* clusterPred,
-                                  uint32_t* remote) {
-    for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < R; t += gridDim.x * blockDim.x) {
-        const uint32_t k = rowList[t];
-        const uint32_t own = rowBlock(A, k, islandOf, clusterOf);
-        for (int side = 0; side < 2; ++side) {
-            const uint32_t p = pred[2 * k + side];
-            uint32_t link = kNoPred;
-            if (p != kNoPred && rowBlock(A, p & ~kWrap, islandOf, clusterOf) != own) {
-                link = p;
-                remote[p & ~kWrap] = 1u;
-            }
-            clusterPred[2 * k + side] = link;
-        }
+    uint32_t owner = k % clusters;
+    if (isl < A.realIslands) {
+        const vx_contact& c = A.contacts[A.order[k]];
+        owner = clusterOf[isDynamic(A.B.filt[c.a].x) ? c.a : c.b];
     }
+    return owner * G + (segmentOf(A.segStart, g0, g1, k) - g0);
 }
 
 __global__ void clusterCountKernel(SolveArgs A, const uint32_t* rowList, uint32_t R, const uint32_t* islandOf,
-                                   const uint32_t* clusterOf, uint32_t G, uint32_t* counts) {
+                                   const uint32_t* clusterOf, uint32_t clusters, uint32_t G, uint32_t* counts) {
     for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < R; t += gridDim.x * blockDim.x)
-        atomicAdd(counts + rowCell(A, rowList[t], islandOf, clusterOf, G), 1u);
+        atomicAdd(counts + rowCell(A, rowList[t], islandOf, clusterOf, clusters, G), 1u);
 }
 
 __global__ void clusterScatterKernel(SolveArgs A, const uint32_t* rowList, uint32_t R, const uint32_t* islandOf,
-                                     const uint32_t* clusterOf, uint32_t G, const uint32_t* start, uint32_t* fill,
-                                     uint32_t* rows) {
+                                     const uint32_t* clusterOf, uint32_t clusters, uint32_t G, const uint32_t* start,
+                                     uint32_t* fill, uint32_t* rows) {
     for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < R; t += gridDim.x * blockDim.x) {
         const uint32_t k = rowList[t];
-        const uint32_t cell = rowCell(A, k, islandOf, clusterOf, G);
+        const uint32_t cell = rowCell(A, k, islandOf, clusterOf, clusters, G);
         rows[start[cell] + atomicAdd(fill + cell, 1u)] = k;
-    }
-}
-
-// Shared-memory index of a block's cluster: the start of each of its G colour
-// cells relative to the block's first row (G + 1 words, padded to 16 bytes),
-// then per row its solve position, contact index and two bodies. A step then
-// reads its rows' indices from shared memory instead of three dependent global
-// loads (cell start, row, contact index and bodies). A block whose rows do not
-// fit reads them from global memory.
-constexpr int kClusterThreads = 256;               // threads of a cluster block
-constexpr uint32_t kClusterSmemBytes = 64u * 1024u;  // its shared-memory index
-
-VXD uint32_t clusterHeadWords(uint32_t G) { return (G + 1u + 3u) & ~3u; }
-
-VXD bool clusterIndexFits(uint32_t G, uint32_t rowsInBlock) {
-    return (uint64_t)clusterHeadWords(G) * 4u + (uint64_t)rowsInBlock * 16u <= (uint64_t)kClusterSmemBytes;
-}
-
-// One unit (sweep) step of block c's cluster for colour slot gl; false = abort.
-// `pred`: the cross-cluster links (clusterLinkKernel); `remote`: rows that
-// publish their sweep counter. `resident`: the block's index is in shared
-// memory (cellStart, info); else the rows come from start/rows in global memory.
-VXD bool clusterStep(const SolveArgs& A, const uint32_t* start, const uint32_t* rows, bool resident,
-                     const uint32_t* cellStart, const uint4* info, uint32_t base, uint32_t gl, int u, int op,
-                     const uint32_t* pred, const uint32_t* remote, uint32_t* done, CoopState* st, int* abortFlag) {
-    const uint32_t i0 = resident ? cellStart[gl] : start[base + gl];
-    const uint32_t i1 = resident ? cellStart[gl + 1] : start[base + gl + 1];
-    for (uint32_t idx = i0 + threadIdx.x; idx < i1; idx += blockDim.x) {
-        uint32_t k;
-        GiantRowIn in;
-        if (resident) {
-            const uint4 r = info[idx];
-            k = r.x;
-            in.ab = make_uint2(r.z, r.w);
-            in.cp = A.contacts + r.y;
-            loadContactCoherent(in.cp, in.cc);
-            if (op == 0 || op == 1) coherentPrep(A.prep + k, in.P);
-        } else {
-            k = rows[idx];
-            giantRowFetch(A, k, op, in);
-        }
-        const uint32_t p0 = pred[2 * k], p1 = pred[2 * k + 1];
-        if (p0 != kNoPred || p1 != kNoPred) {
-            const uint32_t need0 = (p0 & kWrap) ? (uint32_t)u : (uint32_t)u + 1u;
-            const uint32_t need1 = (p1 & kWrap) ? (uint32_t)u : (uint32_t)u + 1u;
-            bool ok = true;
-            uint32_t nap = 16;
-            for (uint32_t spins = 0;; ++spins) {
-                const uint32_t d0 = p0 == kNoPred ? 0xffffffffu : ldAcquire(done + (p0 & ~kWrap));
-                const uint32_t d1 = p1 == kNoPred ? 0xffffffffu : ldAcquire(done + (p1 & ~kWrap));
-                if (d0 >= need0 && d1 >= need1) break;
-                if (spins > st->spinLimit || ((spins & 63u) == 63u && __ldcg(&st->timeout))) {
-                    atomicOr(&st->timeout, 1u);
-                    ok = false;
-                    break;
-                }
-                __nanosleep(nap);
-                if (nap < 256u) nap <<= 1;
-            }
-            if (!ok) { *abortFlag = 1; break; }
-        }
-        giantRowRun(A, k, op, in);
-        if (remote[k]) stRelease(done + k, (uint32_t)u + 1u);
-    }
-    __syncthreads();
-    return *abortFlag == 0;
-}
-
-__global__ void __launch_bounds__(kClusterThreads, 2) solveClusterKernel(SolveArgs A, uint32_t G, const uint32_t* start,
-                                                          const uint32_t* rows, const uint32_t* rowList, uint32_t R,
-                                                          const uint32_t* bodyIds, uint32_t NB, const uint32_t* pred,
-                                                          const uint32_t* remote, uint32_t* done, CoopState* st) {
-    extern __shared__ uint4 clusterSmem[];  // kClusterSmemBytes: the block's cluster index
-    __shared__ int abortFlag;
-    const uint32_t tid = blockIdx.x * blockDim.x + threadIdx.x, stride = gridDim.x * blockDim.x;
-    const uint32_t base = blockIdx.x * G;
-    const uint32_t s0 = start[base], s1 = start[base + G];
-    const bool resident = G > 0 && clusterIndexFits(G, s1 - s0);
-    uint32_t* cellStart = reinterpret_cast<uint32_t*>(clusterSmem);
-    uint4* info = clusterSmem + clusterHeadWords(G) / 4u;
-    if (resident) {
-        for (uint32_t t = threadIdx.x; t <= G; t += blockDim.x) cellStart[t] = start[base + t] - s0;
-        for (uint32_t i = threadIdx.x; i < s1 - s0; i += blockDim.x) {
-            const uint32_t k = rows[s0 + i];
-            const uint2 ab = A.rowBodies[k];
-            info[i] = make_uint4(k, A.order[k], ab.x, ab.y);
-        }
-    }
-    if (threadIdx.x == 0) abortFlag = 0;
-    __syncthreads();
-    if (A.positionIterations > 0) {
-        for (uint32_t t = tid; t < R; t += stride) __stcg(done + rowList[t], 0u);
-        if (!gridSync(&st->bar, &st->timeout, st->spinLimit)) return;
-        for (int u = 0; u < A.positionIterations; ++u)
-            for (uint32_t gl = 0; gl < G; ++gl)
-                if (!clusterStep(A, start, rows, resident, cellStart, info, base, gl, u, 2, pred, remote, done, st,
-                                 &abortFlag))
-                    return;
-        gridSync(&st->bar, &st->timeout, st->spinLimit);
-        return;
-    }
-    for (int s = 0; s < A.substeps; ++s) {
-        for (uint32_t t = tid; t < NB; t += stride) {
-            const uint32_t id = bodyIds[t];
-            if (A.integrate && s > 0) giantIntegrateVelocity(A, id);
-            __stcg(A.frames + id, pack(inertiaFrameAt(loadMass(A.B, id), q4(ldcg4(A.B.rot + id)))));
-        }
-        if (!gridSync(&st->bar, &st->timeout, st->spinLimit)) return;
-        for (uint32_t t = tid; t < R; t += stride) {
-            const uint32_t k = rowList[t];
-            giantRow(A, k, 3);
-            __stcg(done + k, 0u);
-        }
-        if (!gridSync(&st->bar, &st->timeout, st->spinLimit)) return;
-        const int warmUnits = A.warmStart && s == 0 ? 1 : 0;
-        for (int u = 0; u < warmUnits + A.sweeps; ++u)
-            for (uint32_t gl = 0; gl < G; ++gl)
-                if (!clusterStep(A, start, rows, resident, cellStart, info, base, gl, u, u < warmUnits ? 0 : 1, pred,
-                                 remote, done, st, &abortFlag))
-                    return;
-        if (!gridSync(&st->bar, &st->timeout, st->spinLimit)) return;
-        if (A.integrate) {
-            for (uint32_t t = tid; t < NB; t += stride) giantIntegrateTransform(A, bodyIds[t]);
-            if (!gridSync(&st->bar, &st->timeout, st->spinLimit)) return;
-        }
     }
 }
 
@@ -2192,15 +1864,14 @@ __global__ void __launch_bounds__(kClusterThreads, 2) solveClusterKernel(SolveAr
 VXD bool isGiant(const SolveArgs& A, uint32_t isl) {
     const uint32_t rows = A.islandStart[isl + 1] - A.islandStart[isl];
     const uint32_t nb = isl < A.realIslands ? A.bodyStart[isl + 1] - A.bodyStart[isl] : 0u;
-    return islandClassOf(nb, rows, A.tinyLimit) == kGiantIsland;
+    return solveClassOf(nb, rows, A.tinyLimit) == kGiantIsland;
 }
 
 __global__ void giantEntryKernel(SolveArgs A, const uint32_t* islandOf, uint32_t m, uint32_t n, uint64_t* keys,
-                                 uint32_t* vals, uint2* rowBodies) {
+                                 uint32_t* vals) {
     for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < m; k += gridDim.x * blockDim.x) {
         const bool giant = isGiant(A, islandOf[k]);
         const vx_contact& c = A.contacts[A.order[k]];
-        rowBodies[k] = make_uint2(c.a, c.b);
         const uint32_t fa = A.B.filt[c.a].x, fb = A.B.filt[c.b].x;
         const bool solved = giant && solvedContact(fa, fb);
         keys[2 * k] = solved && isDynamic(fa) ? c.a : n;
@@ -3259,7 +2930,6 @@ static int buildIslands(Context& c, const vx_contact* cs, uint32_t m, IslandPlan
     const uint32_t n = c.n;
     plan.contacts = m;
     c.planContacts = m;
-    c.giantLinked = false;
     c.clusterBuilt = false;
     c.tinyPacked = false;
     VXB_TRY(ensure(c, c.parentBuf, (size_t)n * 4));
@@ -3410,6 +3080,73 @@ static int launchIslands(Context& c, const SolveArgs& A) {
     return VXB_OK;
 }
 
+// Plan of the giant islands' flow, once per island plan: every row's links on
+// its bodies, the bodies' clusters and the warps' rows in colour order.
+static int buildFlow(Context& c, const SolveArgs& A, uint32_t clusters) {
+    const uint32_t m = c.planContacts, n = c.n;
+    VXB_TRY(ensure(c, c.fpKeyBuf, (size_t)m * 16 + 64));
+    VXB_TRY(ensure(c, c.fpValBuf, (size_t)m * 8 + 64));
+    VXB_TRY(ensure(c, c.fpSlotBuf, (size_t)m * 8 + 64));
+    VXB_TRY(ensure(c, c.fpRunStartBuf, (size_t)n * 8 + 64));
+    VXB_TRY(ensure(c, c.flowBodyBuf, (size_t)n * 64 + 64));
+    uint64_t* keys = P<uint64_t>(c.fpKeyBuf);
+    uint32_t* vals = P<uint32_t>(c.fpValBuf);
+    const uint32_t* islandOf = P<uint32_t>(c.fpIslandBuf);
+    VXB_CUDA(c, cudaMemsetAsync(&c.dCounters->flowTooWide, 0, 4, c.stream));
+    LAUNCH(c, giantEntryKernel, blocksFor(m, 256), 256, A, islandOf, m, n, keys, vals);
+    VXB_TRY(sortPairs(c, keys, vals, 2 * m, bitsFor(n)));
+    LAUNCH(c, flowRunKernel, blocksFor(2 * m, 256), 256, keys, 2 * m, n, P<uint2>(c.fpRunStartBuf), c.dCounters);
+    LAUNCH(c, flowLinkKernel, blocksFor(2 * m, 256), 256, keys, vals, 2 * m, n,
+           (const uint2*)P<uint2>(c.fpRunStartBuf), P<uint32_t>(c.fpSlotBuf));
+    VXB_TRY(ensure(c, c.clusterInfoBuf, ((size_t)n * 3 + (size_t)m * 3 + 128) * 4));
+    uint32_t* bodyFlags = P<uint32_t>(c.clusterInfoBuf);
+    uint32_t* bodyRank = bodyFlags + n + 16;
+    uint32_t* bodyPos = bodyRank + n + 16;
+    uint32_t* rowFlags = bodyPos + n + 16;
+    uint32_t* rowRank = rowFlags + m + 16;
+    uint32_t* rowList = rowRank + m + 16;
+    VXB_CUDA(c, cudaMemsetAsync(&c.dCounters->clusterColours, 0, 4, c.stream));
+    LAUNCH(c, giantMemberKernel, blocksFor(std::max(n, m), 256), 256, A, P<uint64_t>(c.bodyKeyBuf), n, islandOf, m,
+           bodyFlags, rowFlags, c.dCounters);
+    VXB_TRY(exclusiveScan(c, bodyFlags, bodyRank, n, &c.dCounters->clusterBodies));
+    VXB_TRY(exclusiveScan(c, rowFlags, rowRank, m, &c.dCounters->clusterRows));
+    LAUNCH(c, compactKernel, blocksFor(n, 256), 256, bodyFlags, bodyRank, n, bodyPos);
+    LAUNCH(c, compactKernel, blocksFor(m, 256), 256, rowFlags, rowRank, m, rowList);
+    VXB_TRY(readCounters(c));
+    c.clusterNB = c.hostCounters.clusterBodies;
+    c.clusterR = c.hostCounters.clusterRows;
+    c.clusterG = c.hostCounters.clusterColours;
+    c.clusterCount = clusters;
+    c.clusterBuilt = true;
+    const uint32_t nb = c.clusterNB, R = c.clusterR, G = c.clusterG, cells = clusters * G;
+    if (nb == 0 || R == 0 || G == 0) {
+        c.clusterR = 0;
+        return VXB_OK;
+    }
+    VXB_TRY(ensure(c, c.clusterKeyBuf, (size_t)nb * 8 + 64));
+    VXB_TRY(ensure(c, c.clusterValBuf, (size_t)nb * 4 + 64));
+    VXB_TRY(ensure(c, c.clusterOfBuf, (size_t)n * 4 + 64));
+    VXB_TRY(ensure(c, c.clusterCountBuf, (size_t)cells * 8 + 64));
+    VXB_TRY(ensure(c, c.clusterStartBuf, ((size_t)cells + 1) * 4 + 64));
+    VXB_TRY(ensure(c, c.clusterRowsBuf, (size_t)R * 4 + 64));
+    uint32_t* counts = P<uint32_t>(c.clusterCountBuf);
+    uint32_t* fill = counts + cells;
+    uint32_t* start = P<uint32_t>(c.clusterStartBuf);
+    const uint32_t* clusterOf = P<uint32_t>(c.clusterOfBuf);
+    LAUNCH(c, clusterBodyKeyKernel, blocksFor(nb, 256), 256, A, (const uint32_t*)bodyPos, nb,
+           (const Counters*)c.dCounters, P<uint64_t>(c.clusterKeyBuf), P<uint32_t>(c.clusterValBuf));
+    VXB_TRY(sortPairs(c, P<uint64_t>(c.clusterKeyBuf), P<uint32_t>(c.clusterValBuf), nb, 30));
+    LAUNCH(c, clusterOfBodyKernel, blocksFor(nb, 256), 256, (const uint32_t*)P<uint32_t>(c.clusterValBuf), nb, clusters,
+           P<uint32_t>(c.clusterOfBuf));
+    VXB_CUDA(c, cudaMemsetAsync(counts, 0, (size_t)cells * 8, c.stream));
+    LAUNCH(c, clusterCountKernel, blocksFor(R, 256), 256, A, (const uint32_t*)rowList, R, islandOf, clusterOf, clusters,
+           G, counts);
+    VXB_TRY(exclusiveScan(c, counts, start, cells, start + cells));
+    LAUNCH(c, clusterScatterKernel, blocksFor(R, 256), 256, A, (const uint32_t*)rowList, R, islandOf, clusterOf,
+           clusters, G, (const uint32_t*)start, fill, P<uint32_t>(c.clusterRowsBuf));
+    return VXB_OK;
+}
+
 static int launchSolve(Context& c, const SolveArgs& A) {
     if (A.islands == 0) return VXB_OK;
     // tiny islands: pack them into warps once per island plan
@@ -3453,7 +3190,6 @@ static int launchSolve(Context& c, const SolveArgs& A) {
     }
     if (c.planLargest > kTinyLimit) VXB_TRY(launchIslands<kSmallIsland>(c, A));
     if (c.planLargest >= (uint32_t)kSmallBodies) VXB_TRY(launchIslands<kMediumIsland>(c, A));
-    if (c.planLargest >= (uint32_t)kMediumBodies) VXB_TRY(launchIslands<kLargeIsland>(c, A));
     // giant islands: list them, then one cooperative launch over all of them
     VXB_TRY(ensure(c, c.giantBuf, ((size_t)A.islands + 1) * 4 + 64));
     VXB_TRY(ensure(c, c.coopBuf, sizeof(CoopState)));
@@ -3465,100 +3201,24 @@ static int launchSolve(Context& c, const SolveArgs& A) {
     LAUNCH(c, giantListKernel, std::min<uint32_t>(blocksFor(A.islands, 256), (uint32_t)c.smCount * 4), 256, A, list,
            &st->rounds);
     c.stats.giantIslands = std::max(c.stats.giantIslands, giants);
-    // dataflow links of the giant islands' rows (once per island plan)
-    const uint32_t m = c.planContacts;
-    VXB_TRY(ensure(c, c.fpKeyBuf, (size_t)m * 16 + 64));
-    VXB_TRY(ensure(c, c.fpValBuf, (size_t)m * 8 + 64));
-    VXB_TRY(ensure(c, c.fpSlotBuf, (size_t)m * 8 + 64));
-    VXB_TRY(ensure(c, c.fpColorBuf, (size_t)m * 4 + 64));
-    VXB_TRY(ensure(c, c.fpRunStartBuf, (size_t)c.n * 4 + 64));
-    VXB_TRY(ensure(c, c.rowBodyBuf, (size_t)m * 8 + 64));
-    uint32_t* pred = P<uint32_t>(c.fpSlotBuf);
-    uint32_t* done = P<uint32_t>(c.fpColorBuf);
-    if (!c.giantLinked) {
-        uint64_t* keys = P<uint64_t>(c.fpKeyBuf);
-        uint32_t* vals = P<uint32_t>(c.fpValBuf);
-        LAUNCH(c, giantEntryKernel, blocksFor(m, 256), 256, A, P<uint32_t>(c.fpIslandBuf), m, c.n, keys, vals,
-               P<uint2>(c.rowBodyBuf));
-        VXB_TRY(sortPairs(c, keys, vals, 2 * m, bitsFor(c.n)));
-        LAUNCH(c, giantLastKernel, blocksFor(2 * m, 256), 256, keys, 2 * m, c.n, P<uint32_t>(c.fpRunStartBuf));
-        LAUNCH(c, giantPredKernel, blocksFor(2 * m, 256), 256, keys, vals, 2 * m, c.n,
-               P<uint32_t>(c.fpRunStartBuf), pred);
-        c.giantLinked = true;
-    }
-    SolveArgs G = A;
-    G.rowBodies = P<uint2>(c.rowBodyBuf);
-    if (c.cooperative) {
-        // the giant islands in spatial clusters, one per block of the cooperative grid
-        int perSm = 0;
-        VXB_CUDA(c, cudaFuncSetAttribute(solveClusterKernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                          (int)kClusterSmemBytes));
-        VXB_CUDA(c, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSm, solveClusterKernel, kClusterThreads,
-                                                                  kClusterSmemBytes));
-        const uint32_t clusters = (uint32_t)(perSm * c.smCount);
-        const uint32_t n = c.n;
-        VXB_TRY(ensure(c, c.clusterInfoBuf, ((size_t)n * 3 + (size_t)m * 3 + 64) * 4));
-        uint32_t* bodyFlags = P<uint32_t>(c.clusterInfoBuf);
-        uint32_t* bodyRank = bodyFlags + n + 16;
-        uint32_t* bodyPos = bodyRank + n + 16;
-        uint32_t* rowFlags = bodyPos + n + 16;
-        uint32_t* rowRank = rowFlags + m + 16;
-        uint32_t* rowList = rowRank + m + 16;
-        if (clusters > 0 && !c.clusterBuilt) {
-            VXB_CUDA(c, cudaMemsetAsync(&c.dCounters->clusterColours, 0, 4, c.stream));
-            LAUNCH(c, giantMemberKernel, blocksFor(std::max(n, m), 256), 256, G, P<uint64_t>(c.bodyKeyBuf), n,
-                   (const uint32_t*)P<uint32_t>(c.fpIslandBuf), m, bodyFlags, rowFlags, c.dCounters);
-            VXB_TRY(exclusiveScan(c, bodyFlags, bodyRank, n, &c.dCounters->clusterBodies));
-            VXB_TRY(exclusiveScan(c, rowFlags, rowRank, m, &c.dCounters->clusterRows));
-            LAUNCH(c, compactKernel, blocksFor(n, 256), 256, bodyFlags, bodyRank, n, bodyPos);
-            LAUNCH(c, compactKernel, blocksFor(m, 256), 256, rowFlags, rowRank, m, rowList);
-            VXB_TRY(readCounters(c));
-            c.clusterNB = c.hostCounters.clusterBodies;
-            c.clusterR = c.hostCounters.clusterRows;
-            c.clusterG = c.hostCounters.clusterColours;
-            const uint32_t nb = c.clusterNB, R = c.clusterR, Gc = c.clusterG, cells = clusters * Gc;
-            if (nb > 0 && R > 0 && Gc > 0) {
-                VXB_TRY(ensure(c, c.clusterKeyBuf, (size_t)nb * 8 + 64));
-                VXB_TRY(ensure(c, c.clusterValBuf, (size_t)nb * 4 + 64));
-                VXB_TRY(ensure(c, c.clusterOfBuf, (size_t)n * 4 + 64));
-                VXB_TRY(ensure(c, c.clusterCountBuf, (size_t)cells * 8 + 64));
-                VXB_TRY(ensure(c, c.clusterStartBuf, ((size_t)cells + 1) * 4 + 64));
-                VXB_TRY(ensure(c, c.clusterRowsBuf, (size_t)R * 4 + 64));
-                uint32_t* counts = P<uint32_t>(c.clusterCountBuf);
-                uint32_t* fill = counts + cells;
-                uint32_t* start = P<uint32_t>(c.clusterStartBuf);
-                LAUNCH(c, clusterBodyKeyKernel, blocksFor(nb, 256), 256, G, (const uint32_t*)bodyPos, nb,
-                       (const Counters*)c.dCounters, P<uint64_t>(c.clusterKeyBuf), P<uint32_t>(c.clusterValBuf));
-                VXB_TRY(sortPairs(c, P<uint64_t>(c.clusterKeyBuf), P<uint32_t>(c.clusterValBuf), nb, 30));
-                LAUNCH(c, clusterOfBodyKernel, blocksFor(nb, 256), 256, (const uint32_t*)P<uint32_t>(c.clusterValBuf),
-                       nb, clusters, P<uint32_t>(c.clusterOfBuf));
-                VXB_CUDA(c, cudaMemsetAsync(counts, 0, (size_t)cells * 8, c.stream));
-                LAUNCH(c, clusterCountKernel, blocksFor(R, 256), 256, G, (const uint32_t*)rowList, R,
-                       (const uint32_t*)P<uint32_t>(c.fpIslandBuf), (const uint32_t*)P<uint32_t>(c.clusterOfBuf), Gc,
-                       counts);
-                VXB_TRY(exclusiveScan(c, counts, start, cells, start + cells));
-                LAUNCH(c, clusterScatterKernel, blocksFor(R, 256), 256, G, (const uint32_t*)rowList, R,
-                       (const uint32_t*)P<uint32_t>(c.fpIslandBuf), (const uint32_t*)P<uint32_t>(c.clusterOfBuf), Gc,
-                       (const uint32_t*)start, fill, P<uint32_t>(c.clusterRowsBuf));
-                VXB_TRY(ensure(c, c.clusterLinkBuf, (size_t)m * 12 + 64));
-                uint32_t* remote = P<uint32_t>(c.clusterLinkBuf) + 2 * (size_t)m;
-                VXB_CUDA(c, cudaMemsetAsync(remote, 0, (size_t)m * 4, c.stream));
-                LAUNCH(c, clusterLinkKernel, blocksFor(R, 256), 256, G, (const uint32_t*)rowList, R,
-                       (const uint32_t*)P<uint32_t>(c.fpIslandBuf), (const uint32_t*)P<uint32_t>(c.clusterOfBuf),
-                       (const uint32_t*)pred, P<uint32_t>(c.clusterLinkBuf), remote);
-                c.clusterBuilt = true;
-            }
-        }
-        if (clusters > 0 && c.clusterBuilt) {
+    int perSm = 0;
+    auto* flow = A.coneBlock ? solveFlowKernel<true> : solveFlowKernel<false>;
+    VXB_CUDA(c, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSm, flow, kFlowThreads, 0));
+    perSm = std::min(perSm, kFlowBlocksPerSm);
+    const uint32_t clusters = (uint32_t)(perSm * c.smCount) * (kFlowThreads / 32);
+    if (c.cooperative && clusters > 0) {
+        if (!c.clusterBuilt || c.clusterCount != clusters) VXB_TRY(buildFlow(c, A, clusters));
+        if (c.clusterR > 0 && !c.hostCounters.flowTooWide) {
+            FlowArgs F;
+            F.start = P<uint32_t>(c.clusterStartBuf);
+            F.rows = P<uint32_t>(c.clusterRowsBuf);
+            F.link = P<uint32_t>(c.fpSlotBuf);
+            F.bodyIds = P<uint32_t>(c.clusterValBuf);
+            F.body = P<float4>(c.flowBodyBuf);
+            F.bodies = c.clusterNB;
+            F.colours = c.clusterG;
             VXB_TRY(resetCoop(c, st));
-            const int rcc = launchCooperativeSmem(c, 0, kClusterSmemBytes, solveClusterKernel, kClusterThreads, G,
-                                                  c.clusterG,
-                                              (const uint32_t*)P<uint32_t>(c.clusterStartBuf),
-                                              (const uint32_t*)P<uint32_t>(c.clusterRowsBuf), (const uint32_t*)rowList,
-                                              c.clusterR, (const uint32_t*)P<uint32_t>(c.clusterValBuf), c.clusterNB,
-                                              (const uint32_t*)P<uint32_t>(c.clusterLinkBuf),
-                                              (const uint32_t*)(P<uint32_t>(c.clusterLinkBuf) + 2 * (size_t)m), done,
-                                              st);
+            const int rcc = launchCooperativeSmem(c, perSm, 0, flow, kFlowThreads, A, F, st);
             if (rcc != VXB_ERR_UNSUPPORTED) {
                 VXB_TRY(rcc);
                 // a timed-out wait reaches the host with the step's final counter read

@@ -22,8 +22,7 @@
 // A step fell from 3.8 us (256 threads, a row per thread, 128- and 176-byte
 // records read at the start of the step) to 1.2 us on an island of 400 rows in
 // 25 colours. Solve stage of one step: 13.3 -> 5.4 ms for 64 islands of 2,400
-// rows (31 colours, 8 substeps), 13.0 -> 7.9 ms for one of 10,500 rows and
-// 1,000 bodies (49 colours), 6.7 -> 4.3 ms for one of 3,500 rows in a heap.
+// rows (31 colours, 8 substeps), 4.8 -> 1.9 ms for one of 310 rows (20 colours).
 // Measured and not kept: cross's sign rule behind a branch (20 % slower), one
 // lane per row with the same planes (about equal for narrow colours, slower
 // for wide ones).
@@ -90,24 +89,20 @@ struct SolveArgs {
     int coneBlock;
     uint32_t tinyLimit;
     int positionIterations;  // position-correction mode when > 0
-    RowPrep* prep;           // per solve-order row, rebuilt every substep (giant islands)
-    float4* planes;          // per solve-order row terms of the block solve (RowPlanes)
+    RowPrep* prep;           // per solve-order row, rebuilt every substep (giant islands without a cooperative grid)
+    float4* planes;          // per row terms of the block solve and the grid's flow (RowPlanes)
     uint32_t rows;           // rows of the plan (the planes' stride)
     float4* frames;          // per body inertia frame, rebuilt every substep (global path)
     int stackStabilization;
     float stackStiffness, stackDamping;
     uint32_t* fault;         // set when the island plan is inconsistent (Counters::planFault)
-    const uint2* rowBodies;  // per solve-order row: (a, b) of its contact (giant islands)
 };
 
 VXD bool solvedContact(uint32_t fa, uint32_t fb) { return !isSensor(fa) && !isSensor(fb); }
 
 // Island classes by what a block of the class holds (islandClassOf). Small: one
 // warp, many per SM. Medium: several blocks per SM. Large: one block per SM
-// (64 bytes of shared memory per body: 3,072 bodies fit 197 KB), for islands
-// whose colours are too narrow to pay for a grid-wide solve: 7.9 against 13.0
-// ms in the clustered solve for 10,500 rows in 49 colours. Beyond that, where
-// a colour's rows no longer fit one SM's issue slots, the clustered solve.
+// (the colouring's; the solve takes them as giants). Giant: the whole grid.
 constexpr int kSmallThreads = 32, kSmallBodies = 64, kSmallRows = 256;
 constexpr int kMediumThreads = 256, kMediumBodies = 512, kMediumRows = 3072;
 constexpr int kLargeThreads = 512, kLargeBodies = 3072, kLargeRows = 16384;
@@ -119,6 +114,16 @@ VXD int islandClassOf(uint32_t nb, uint32_t rows, uint32_t tinyLimit) {
     if (nb <= (uint32_t)kMediumBodies && rows <= (uint32_t)kMediumRows) return kMediumIsland;
     if (nb <= (uint32_t)kLargeBodies && rows <= (uint32_t)kLargeRows) return kLargeIsland;
     return kGiantIsland;
+}
+
+// The solve's classes: large islands (one block's shared memory would hold
+// them) run as the grid's flow, too. Solve stage of one step, one 512-thread
+// block against the flow: 10,500 rows in 49 colours 7.9 / 4.8 ms, 6,100 in 40
+// 5.5 / 4.1 ms, 3,500 in 17 4.1 / 3.2 ms. Medium islands stay in their blocks:
+// 64 of 2,400 rows 5.4 / 7.2 ms, one of 310 1.9 / 2.6 ms.
+VXD int solveClassOf(uint32_t nb, uint32_t rows, uint32_t tinyLimit) {
+    const int cls = islandClassOf(nb, rows, tinyLimit);
+    return cls == kLargeIsland ? kGiantIsland : cls;
 }
 
 template <int Class>
@@ -560,6 +565,54 @@ VXD int bodyWord(const SolveArgs& A, const uint32_t* localIdx, uint32_t b0, uint
     return ~(int)id;
 }
 
+// A row's pose terms into the planes (all but its arms and impulses) for
+// substep s; returns its bits.
+template <bool Cone>
+VXD uint32_t storeRowPlanes(const RowPlanes& R, uint32_t k, const RowContact& rc, const RowPrep& P, bool solved, int s) {
+    R.n[k] = pack(rc.normal, solved ? P.kNormal : 0.0f);
+    R.t1[k] = pack(P.t1, P.k1);
+    R.t2[k] = pack(P.t2, P.k2);
+    float closing = P.targetBase, parting = P.targetBase;
+    if (rc.vn0 < -1.0f) {
+        parting = vmax(P.targetBase, -rc.restitution * rc.vn0);
+        if (P.liveGap <= 0.0f) closing = parting;
+    }
+    R.g[k] = make_float4(closing, parting, rc.friction1, rc.friction2);
+    R.aux[k] = Cone ? make_float4(P.kN1, P.kN2, P.k12, 0.0f)
+                    : make_float4(1.0f / P.kNormal, 1.0f / P.k1, 1.0f / P.k2, 0.0f);
+    const bool ext = rc.rolling > 0.0f || rc.spinning > 0.0f;
+    const bool recip = quotientBase(P.kNormal) &&
+                       (!(P.k1 > 0.0f && P.k2 > 0.0f) || (quotientBase(P.k1) && quotientBase(P.k2)));
+    if (ext)
+        for (int side = 0; side < 2; ++side) {
+            float4* E = R.ext + 2 * (2 * (size_t)k + side);
+            E[0] = make_float4(P.kr1, P.kr2, P.ks, rc.rolling);
+            if (s == 0) E[1] = make_float4(rc.spinning, rc.r1Imp, rc.r2Imp, rc.sImp);
+        }
+    return (ext ? kRowExt : 0u) | (solved ? kRowSolved : 0u) | (recip ? kRowRecip : 0u);
+}
+
+// The sweeps set a contact's point to these poses' anchors; a warm start
+// without sweeps only for rows that carry impulses.
+VXD bool setsPoint(const SolveArgs& A, int s, bool solved, const RowContact& rc) {
+    return solved && (A.sweeps > 0 ||
+                      (A.warmStart && s == 0 && !(rc.nImp <= 0.0f && rc.t1Imp == 0.0f && rc.t2Imp == 0.0f &&
+                                                  rc.r1Imp == 0.0f && rc.r2Imp == 0.0f && rc.sImp == 0.0f)));
+}
+
+VXD void storeRowImpulses(const RowPlanes& R, uint32_t k, vx_contact& c) {
+    const float4 imp = R.imp[2 * (size_t)k];
+    c.normalImpulse = imp.x;
+    c.tangentImpulse1 = imp.y;
+    c.tangentImpulse2 = imp.z;
+    if (__float_as_uint(imp.w) & kRowExt) {
+        const float4 e1 = R.ext[4 * (size_t)k + 1];
+        c.rollingImpulse1 = e1.y;
+        c.rollingImpulse2 = e1.z;
+        c.spinningImpulse = e1.w;
+    }
+}
+
 template <int Class, bool Cone>
 __global__ void __launch_bounds__(ClassShape<Class>::kThreads, ClassShape<Class>::kBlocksPerSm)
     solveIslandKernel(SolveArgs A, uint32_t* localIdx) {
@@ -577,7 +630,7 @@ __global__ void __launch_bounds__(ClassShape<Class>::kThreads, ClassShape<Class>
         const uint32_t b0 = isl < A.realIslands ? A.bodyStart[isl] : 0u;
         const uint32_t b1 = isl < A.realIslands ? A.bodyStart[isl + 1] : 0u;
         const uint32_t nb = b1 - b0;
-        if (islandClassOf(nb, s1 - s0, A.tinyLimit) != Class) continue;
+        if (solveClassOf(nb, s1 - s0, A.tinyLimit) != Class) continue;
         const uint32_t g0 = A.islandSeg[isl], colours = A.islandSeg[isl + 1] - g0;
         const uint32_t* seg = A.segStart + g0;
         if (colours < (uint32_t)ClassShape<Class>::kSegments) {
@@ -658,40 +711,14 @@ __global__ void __launch_bounds__(ClassShape<Class>::kThreads, ClassShape<Class>
                 RowPrep P;
                 prepRow(a, b, rc, A.h, Cone, P);
                 const bool solved = solvedContact(a.m.flags, b.m.flags);
-                R.n[k] = pack(rc.normal, solved ? P.kNormal : 0.0f);
-                R.t1[k] = pack(P.t1, P.k1);
-                R.t2[k] = pack(P.t2, P.k2);
-                float closing = P.targetBase, parting = P.targetBase;
-                if (rc.vn0 < -1.0f) {
-                    parting = vmax(P.targetBase, -rc.restitution * rc.vn0);
-                    if (P.liveGap <= 0.0f) closing = parting;
-                }
-                R.g[k] = make_float4(closing, parting, rc.friction1, rc.friction2);
-                R.aux[k] = Cone ? make_float4(P.kN1, P.kN2, P.k12, 0.0f)
-                                : make_float4(1.0f / P.kNormal, 1.0f / P.k1, 1.0f / P.k2, 0.0f);
+                const uint32_t bits = storeRowPlanes<Cone>(R, k, rc, P, solved, s);
                 R.side[2 * (size_t)k] = pack(P.ra, __int_as_float(la));
                 R.side[2 * (size_t)k + 1] = pack(P.rb, __int_as_float(lb));
-                const bool ext = rc.rolling > 0.0f || rc.spinning > 0.0f;
-                const bool recip = quotientBase(P.kNormal) && (!(P.k1 > 0.0f && P.k2 > 0.0f) ||
-                                                               (quotientBase(P.k1) && quotientBase(P.k2)));
-                const uint32_t bits = (ext ? kRowExt : 0u) | (solved ? kRowSolved : 0u) | (recip ? kRowRecip : 0u);
                 float4 imp = make_float4(rc.nImp, rc.t1Imp, rc.t2Imp, 0.0f);
                 if (s > 0) imp = R.imp[2 * (size_t)k];
                 imp.w = __uint_as_float(bits);
                 R.imp[2 * (size_t)k] = R.imp[2 * (size_t)k + 1] = imp;
-                if (ext)
-                    for (int side = 0; side < 2; ++side) {
-                        float4* E = R.ext + 2 * (2 * (size_t)k + side);
-                        E[0] = make_float4(P.kr1, P.kr2, P.ks, rc.rolling);
-                        if (s == 0) E[1] = make_float4(rc.spinning, rc.r1Imp, rc.r2Imp, rc.sImp);
-                    }
-                // the sweeps set the contact's point to these poses' anchors; a warm start
-                // without sweeps only for rows that carry impulses
-                if (solved && (A.sweeps > 0 ||
-                               (A.warmStart && s == 0 &&
-                                !(rc.nImp <= 0.0f && rc.t1Imp == 0.0f && rc.t2Imp == 0.0f && rc.r1Imp == 0.0f &&
-                                  rc.r2Imp == 0.0f && rc.sImp == 0.0f))))
-                    c.point = vx_vec3{P.point.x, P.point.y, P.point.z};
+                if (setsPoint(A, s, solved, rc)) c.point = vx_vec3{P.point.x, P.point.y, P.point.z};
             }
             islandBarrier<Threads>();
             if (A.warmStart && s == 0) runColours<Threads, kRowWarm, Cone>(A, R, T, seg, colours, 1);
@@ -717,17 +744,7 @@ __global__ void __launch_bounds__(ClassShape<Class>::kThreads, ClassShape<Class>
             A.B.ang[id] = pack(f3(T.w[t]), 0.0f);
         }
         for (uint32_t k = s0 + threadIdx.x; k < s1; k += Threads) {
-            vx_contact& c = A.contacts[A.order[k]];
-            const float4 imp = R.imp[2 * (size_t)k];
-            c.normalImpulse = imp.x;
-            c.tangentImpulse1 = imp.y;
-            c.tangentImpulse2 = imp.z;
-            if (__float_as_uint(imp.w) & kRowExt) {
-                const float4 e1 = R.ext[4 * (size_t)k + 1];
-                c.rollingImpulse1 = e1.y;
-                c.rollingImpulse2 = e1.z;
-                c.spinningImpulse = e1.w;
-            }
+            storeRowImpulses(R, k, A.contacts[A.order[k]]);
         }
         islandBarrier<Threads>();
     }
