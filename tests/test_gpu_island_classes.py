@@ -86,3 +86,30 @@ def test_islands_of_every_class_side_by_side(ctx):
         for name in ("position", "orientation", "velocity", "angularVelocity"):
             assert np.array_equal(both[name][at:at + n], alone[name][1:]), (n, name)
         at += n
+
+
+def test_many_small_islands_on_one_warp_each(ctx):
+    """More small islands than the GPU holds on four warps each: every one solves as it does alone, bit for bit."""
+    n, islands = 12, 640
+    part = chain(n)[0]
+    ground, part = part[:1], part[1:]
+    parts = [part.copy() for _ in range(islands)]
+    for i, p in enumerate(parts):  # worlds keep the islands apart at equal coordinates
+        p["velocity"][:, 0] += 0.001 * (i % 7)
+    soup = vb.make_soup(np.zeros((0, 3)), np.zeros(0))
+    many = np.concatenate([np.concatenate([ground, p]) for p in parts]).astype(vb.BODY)
+    many = vb.binding.records(many, vb.BODY).copy()
+    worlds = np.repeat(np.arange(islands, dtype=np.uint32), n + 1)
+    c = vb.Context(0)
+    c.load(many, soup, worlds)
+    c.configure(dt=4 * H, substeps=4, gravity=(0.0, -9.81, 0.0))
+    c.step(1)
+    got = c.read_bodies()
+    for i in (0, 3, 6, islands - 1):
+        alone = vb.binding.records(np.concatenate([ground, parts[i]]).astype(vb.BODY), vb.BODY).copy()
+        c.load(alone, soup)
+        c.step(1)
+        want = c.read_bodies()
+        at = i * (n + 1)
+        for name in ("position", "orientation", "velocity", "angularVelocity"):
+            assert np.array_equal(got[name][at:at + n + 1], want[name]), (i, name)

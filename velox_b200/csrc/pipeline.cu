@@ -1108,9 +1108,7 @@ __global__ void colorFinishKernel(const uint32_t* order, uint32_t m, const uint3
 // contact bids on its bodies (2.2 ms for the 10,500, 1.1 ms for the 2,400).
 template <int Class>
 struct ColorShape {
-    static constexpr int kRows = Class == kSmallIsland    ? kSmallRows
-                                 : Class == kMediumIsland ? kMediumRows
-                                                          : kLargeRows;
+    static constexpr int kRows = ClassShape<Class>::kRows;
     static constexpr int kBodies = ClassShape<Class>::kBodies;
     static_assert(kBodies < 0xfff && 2 * kRows < 0xffff, "12-bit body words, 16-bit list positions");
     static constexpr size_t kSmem = (size_t)kBodies * 16 + (size_t)kRows * 10;
@@ -3188,7 +3186,11 @@ static int launchSolve(Context& c, const SolveArgs& A) {
             A, (const uint32_t*)tList, (const uint32_t*)tFirst, (const Counters*)c.dCounters, P<uint32_t>(c.localIdxBuf));
         ++c.launches;
     }
-    if (c.planLargest > kTinyLimit) VXB_TRY(launchIslands<kSmallIsland>(c, A));
+    if (c.planLargest > kTinyLimit) {
+        // four warps an island while the GPU holds them all at once
+        const bool few = A.islands <= (uint32_t)(c.smCount * ClassShape<kSmallWide>::kBlocksPerSm);
+        VXB_TRY(few ? launchIslands<kSmallWide>(c, A) : launchIslands<kSmallIsland>(c, A));
+    }
     if (c.planLargest >= (uint32_t)kSmallBodies) VXB_TRY(launchIslands<kMediumIsland>(c, A));
     // giant islands: list them, then one cooperative launch over all of them
     VXB_TRY(ensure(c, c.giantBuf, ((size_t)A.islands + 1) * 4 + 64));

@@ -30,7 +30,7 @@ namespace vxb {
 
 constexpr int kFlowThreads = 128;
 constexpr int kFlowBlocksPerSm = 3;
-constexpr uint32_t kMaxFlowDegree = 16383;  // rows of one body (14 bits beside its rank)
+constexpr uint32_t kMaxFlowDegree = kRowLinkMask;  // rows of one body that a link counts
 
 struct FlowArgs {
     const uint32_t* start;    // first slot of each (warp, colour) cell
@@ -59,11 +59,6 @@ VXD void stRelaxed16(float4* p, const V3& v, uint32_t tag) {
                  "l"(lo), "l"(hi)
                  : "memory");
 }
-
-// Row bits of a flow row (imp.w): kRowExt, kRowSolved, kRowRecip, kRowTurns
-// (the lane's body may turn), then rank and degree on the lane's body.
-constexpr uint32_t kRowTurns = 8u;
-constexpr int kRowLinkShift = 4;
 
 struct FlowRegs {
     RowRegs r;
@@ -113,7 +108,7 @@ VXD bool flowRow(const SolveArgs& A, const FlowArgs& F, const RowPlanes& R, bool
     const uint32_t bits = __float_as_uint(r.i.w);
     act = act && (bits & kRowSolved);
     const int li = act ? __float_as_int(r.s.w) : kAtRest;
-    const uint32_t rank = (bits >> kRowLinkShift) & kMaxFlowDegree, degree = bits >> (kRowLinkShift + 14);
+    const uint32_t rank = (bits >> kRowLinkShift) & kRowLinkMask, degree = bits >> kRowDegreeShift;
     const uint32_t tag = u * degree + rank;
     float4* rec = F.body + 4 * (size_t)(li >= 0 ? li : 0);
     float4 tv = make_float4(0.0f, 0.0f, 0.0f, 0.0f), tw = tv;

@@ -101,12 +101,15 @@ struct SolveArgs {
 VXD bool solvedContact(uint32_t fa, uint32_t fb) { return !isSensor(fa) && !isSensor(fb); }
 
 // Island classes by what a block of the class holds (islandClassOf). Small: one
-// warp, many per SM. Medium: several blocks per SM. Large: one block per SM
-// (the colouring's; the solve takes them as giants). Giant: the whole grid.
+// warp, many per SM, or four warps (kSmallWide) where the GPU holds all islands
+// at once. Medium: several blocks per SM. Large: one block per SM (the
+// colouring's; the solve takes them as giants). Giant: the whole grid.
 constexpr int kSmallThreads = 32, kSmallBodies = 64, kSmallRows = 256;
+constexpr int kSmallWideThreads = 128;  // few small islands: four warps each
 constexpr int kMediumThreads = 256, kMediumBodies = 512, kMediumRows = 3072;
 constexpr int kLargeThreads = 512, kLargeBodies = 3072, kLargeRows = 16384;
-enum IslandClass : int { kTinyIsland = 0, kSmallIsland, kMediumIsland, kLargeIsland, kGiantIsland };
+enum IslandClass : int { kTinyIsland = 0, kSmallIsland, kMediumIsland, kLargeIsland, kGiantIsland,
+                         kSmallWide };  // kSmallIsland's islands on four warps
 
 VXD int islandClassOf(uint32_t nb, uint32_t rows, uint32_t tinyLimit) {
     if (rows <= tinyLimit) return kTinyIsland;
@@ -128,15 +131,23 @@ VXD int solveClassOf(uint32_t nb, uint32_t rows, uint32_t tinyLimit) {
 
 template <int Class>
 struct ClassShape {
+    static constexpr bool kSmall = Class == kSmallIsland || Class == kSmallWide;
     static constexpr int kThreads = Class == kSmallIsland    ? kSmallThreads
+                                    : Class == kSmallWide    ? kSmallWideThreads
                                     : Class == kMediumIsland ? kMediumThreads
                                                              : kLargeThreads;
-    static constexpr int kBodies = Class == kSmallIsland    ? kSmallBodies
-                                   : Class == kMediumIsland ? kMediumBodies
-                                                            : kLargeBodies;
-    static constexpr int kBlocksPerSm = Class == kSmallIsland ? 16 : Class == kMediumIsland ? 2 : 1;
-    static constexpr int kSegments = Class == kSmallIsland ? 64 : 256;  // colour starts kept in shared memory
-    static constexpr size_t kSmem = (size_t)kBodies * 4 * sizeof(float4) + (size_t)kSegments * sizeof(uint32_t);
+    static constexpr int kBodies = kSmall ? kSmallBodies : Class == kMediumIsland ? kMediumBodies : kLargeBodies;
+    static constexpr int kRows = kSmall ? kSmallRows : Class == kMediumIsland ? kMediumRows : kLargeRows;
+    static constexpr int kBlocksPerSm = Class == kSmallIsland    ? 16
+                                        : Class == kSmallWide    ? 4
+                                        : Class == kMediumIsland ? 2
+                                                                 : 1;
+    static constexpr int kSegments = kSmall ? 64 : 256;  // colour starts kept in shared memory
+    // dataflow (several warps): rows of a batch, a table of batches
+    static constexpr bool kFlow = kThreads > 32;
+    static constexpr int kBatch = kSmall ? 8 : 16;
+    static constexpr size_t kSmem = (size_t)kBodies * 4 * sizeof(float4) + (size_t)kSegments * sizeof(uint32_t) +
+                                    (kFlow ? (size_t)kRows * sizeof(uint16_t) : 0);
 };
 
 // The planes of one block's island, indexed by solve position. Velocity mode:
@@ -158,6 +169,10 @@ struct ClassShape {
 // global memory in every sweep, 300 cycles on the step's critical path.
 constexpr int kPlaneWords = 13;
 constexpr uint32_t kRowExt = 1u, kRowSolved = 2u, kRowRecip = 4u;
+// Dataflow rows: the lane's body may turn; then the row's rank among its
+// body's rows and the body's row count, 14 bits each.
+constexpr uint32_t kRowTurns = 8u, kRowLinkMask = 0x3fffu;
+constexpr int kRowLinkShift = 4, kRowDegreeShift = kRowLinkShift + 14;
 constexpr int kAtRest = INT_MIN;
 struct RowPlanes {
     float4 *n, *t1, *t2, *g, *aux, *side, *imp, *ext;
@@ -530,6 +545,143 @@ VXD void runColours(const SolveArgs& A, const RowPlanes& R, const BodyTable& T, 
     }
 }
 
+// ---- several warps on one island: a dataflow over the body table ------------
+//
+// Colour order only constrains rows that share a dynamic body, so with several
+// warps the colours need no barrier: the table's velocities end in a tag that
+// counts the body's row updates since the substep's start, and a row, which
+// knows its rank among its body's rows, waits for the two tags it must find.
+// The rows are cut into batches of one colour, taken by the warps in turn; a
+// batch's predecessors all lie in earlier batches, so the waits end (each is
+// bounded all the same). Solve stage of one step against the colour barrier:
+// 5.3 -> 4.5 ms with 64 islands of 2,400 rows, 1.9 -> 1.6 ms with one of 310;
+// 24 steps of 128 islands of 34 rows on four warps instead of one 27 -> 22 ms.
+// Batches of 8 or 4 rows were slower (7.2 and 12.6 ms for the 64: more batches
+// poll), as was sleeping between polls.
+constexpr uint32_t kTableWaitLimit = 1u << 22;  // polls of about 50 cycles
+
+VXD float4 ldTable(const float4* p) {
+    float4 v;
+    asm volatile("ld.volatile.shared.v4.f32 {%0, %1, %2, %3}, [%4];"
+                 : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
+                 : "r"((uint32_t)__cvta_generic_to_shared(p))
+                 : "memory");
+    return v;
+}
+VXD void stTable(float4* p, const V3& v, uint32_t tag) {
+    asm volatile("st.volatile.shared.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"((uint32_t)__cvta_generic_to_shared(p)),
+                 "f"(v.x), "f"(v.y), "f"(v.z), "f"(__uint_as_float(tag))
+                 : "memory");
+}
+
+// One batch (all 32 lanes call). u: the sweep counted from the substep's
+// start. Returns false when a wait gave up.
+template <bool Cone>
+VXD bool tableRow(const SolveArgs& A, const RowPlanes& R, const BodyTable& T, bool act, uint32_t k, uint32_t side,
+                  uint32_t u, bool warm, RowRegs& r, volatile int* dead) {
+    const uint32_t bits = __float_as_uint(r.i.w);
+    act = act && (bits & kRowSolved);
+    const int li = act ? __float_as_int(r.s.w) : kAtRest;
+    const uint32_t rank = (bits >> kRowLinkShift) & kRowLinkMask, degree = bits >> kRowDegreeShift;
+    const uint32_t tag = u * degree + rank;
+    LaneBody b;
+    b.dyn = li >= 0;
+    b.turns = b.dyn && (bits & kRowTurns);
+    b.im = 0.0f;
+    b.v = b.w = b.invI = V3{0.0f, 0.0f, 0.0f};
+    b.frame = Q4{0.0f, 0.0f, 0.0f, 1.0f};
+    if (li >= 0) {
+        const float4 ti = T.i[li];
+        b.frame = q4(T.f[li]);
+        b.invI = f3(ti);
+        b.im = ti.w;
+    } else if (li != kAtRest) {
+        b.v = f3(A.B.vel[~li]);
+        b.w = f3(A.B.ang[~li]);
+    }
+    bool ok = li < 0;
+    for (uint32_t spins = 0;; ++spins) {
+        if (!ok) {
+            const float4 tv = ldTable(T.v + li), tw = ldTable(T.w + li);
+            ok = __float_as_uint(tv.w) == tag && __float_as_uint(tw.w) == tag;
+            b.v = f3(tv);
+            b.w = f3(tw);
+        }
+        if (__all_sync(0xffffffffu, ok)) break;
+        if (spins > kTableWaitLimit) {
+            atomicOr(A.fault, 1u);
+            *dead = 1;
+        }
+        if ((spins & 63u) == 63u && __any_sync(0xffffffffu, *dead != 0)) return false;
+    }
+    const V3 arm = f3(r.s), n = f3(r.n);
+    if (warm) {
+        if (act) {
+            const vx_contact& c = A.contacts[A.order[k]];
+            const float r1 = c.rollingImpulse1, r2 = c.rollingImpulse2, sp = c.spinningImpulse;
+            const V3 t1 = f3(r.t1), t2 = f3(r.t2);
+            if (!(r.i.x <= 0.0f && r.i.y == 0.0f && r.i.z == 0.0f && r1 == 0.0f && r2 == 0.0f && sp == 0.0f)) {
+                laneImpulse<true>(b, side, arm, n * r.i.x + t1 * r.i.y + t2 * r.i.z);
+                laneTorque(b, side, t1 * r1 + t2 * r2 + n * sp);
+            }
+        }
+    } else {
+        const bool solve = act && !(r.n.w <= 0.0f);
+        const uint32_t plain = Cone ? 0u : kRowRecip;
+        const bool special = solve && ((bits & (kRowExt | plain)) != plain ||
+                                       negativeZeroKey(b.w.x, b.w.y, b.w.z, r.i.y, r.i.z) == INT_MIN);
+        const float4 imp = r.i;
+        const V3 v0 = b.v, w0 = b.w;
+        if (__any_sync(0xffffffffu, special)) laneSweep<true, Cone>(R, solve, k, side, r, b);
+        else laneSweep<false, Cone>(R, solve, k, side, r, b);
+        if (!solve) {  // a row without normal mass passes its bodies on
+            r.i = imp;
+            b.v = v0;
+            b.w = w0;
+        } else {
+            R.imp[2 * (size_t)k + side] = r.i;
+        }
+    }
+    if (li >= 0) {
+        stTable(T.v + li, b.v, tag + 1u);
+        stTable(T.w + li, b.w, tag + 1u);
+    }
+    return true;
+}
+
+// `units` passes over the island's batches, of which the first `warmUnits`
+// warm-start. batches: first row (12 bits, from s0) | rows - 1 << 12.
+template <int Threads, bool Cone>
+VXD void runBatches(const SolveArgs& A, const RowPlanes& R, const BodyTable& T, const uint16_t* batches,
+                    uint32_t count, uint32_t s0, uint32_t units, uint32_t warmUnits, volatile int* dead) {
+    constexpr uint32_t kWarps = Threads / 32;
+    const uint32_t warp = threadIdx.x >> 5, pair = (threadIdx.x & 31u) >> 1, side = threadIdx.x & 1u;
+    if (warp >= count) return;
+    RowRegs even, odd;  // the current and the next batch, in turn
+    even.s = even.n = even.t1 = even.t2 = even.g = even.i = even.y = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    odd = even;
+    uint32_t at = warp, u = 0, word = batches[at];
+    if (pair <= word >> 12) loadRowRegs<kRowSweep>(R, s0 + (word & 0xfffu) + pair, side, even);
+    bool alive = true;
+    auto batch = [&](RowRegs& now, RowRegs& then) {
+        const bool wrap = at + kWarps >= count;
+        const uint32_t nat = wrap ? warp : at + kWarps, nu = wrap ? u + 1u : u, nword = batches[nat];
+        if (nu < units && pair <= nword >> 12)
+            loadRowRegs<kRowSweep>(R, s0 + (nword & 0xfffu) + pair, side, then);
+        alive = tableRow<Cone>(A, R, T, pair <= word >> 12, s0 + (word & 0xfffu) + pair, side, u, u < warmUnits, now,
+                               dead);
+        if (nat == at) then.i = now.i;  // the warp's only batch: its impulses were just updated
+        at = nat;
+        u = nu;
+        word = nword;
+    };
+    while (u < units && alive) {
+        batch(even, odd);
+        if (u >= units || !alive) break;
+        batch(odd, even);
+    }
+}
+
 // The body of a row for prepRow: pose and mass from global memory, the frame
 // from the table.
 VXD SolverBody tableBody(const SolveArgs& A, const BodyTable& T, int li, uint32_t id) {
@@ -624,13 +776,17 @@ __global__ void __launch_bounds__(ClassShape<Class>::kThreads, ClassShape<Class>
     T.f = T.w + kBodies;
     T.i = T.f + kBodies;
     uint32_t* segShared = reinterpret_cast<uint32_t*>(T.i + kBodies);
+    uint16_t* batches = reinterpret_cast<uint16_t*>(segShared + ClassShape<Class>::kSegments);  // kFlow only
+    constexpr bool kFlow = ClassShape<Class>::kFlow;
+    __shared__ uint32_t batchCount;
+    __shared__ int dead;
     const RowPlanes R = rowPlanes(A);
     for (uint32_t isl = blockIdx.x; isl < A.islands; isl += gridDim.x) {
         const uint32_t s0 = A.islandStart[isl], s1 = A.islandStart[isl + 1];
         const uint32_t b0 = isl < A.realIslands ? A.bodyStart[isl] : 0u;
         const uint32_t b1 = isl < A.realIslands ? A.bodyStart[isl + 1] : 0u;
         const uint32_t nb = b1 - b0;
-        if (solveClassOf(nb, s1 - s0, A.tinyLimit) != Class) continue;
+        if (solveClassOf(nb, s1 - s0, A.tinyLimit) != (Class == kSmallWide ? (int)kSmallIsland : Class)) continue;
         const uint32_t g0 = A.islandSeg[isl], colours = A.islandSeg[isl + 1] - g0;
         const uint32_t* seg = A.segStart + g0;
         if (colours < (uint32_t)ClassShape<Class>::kSegments) {
@@ -646,11 +802,56 @@ __global__ void __launch_bounds__(ClassShape<Class>::kThreads, ClassShape<Class>
             if (position) {
                 T.v[t] = pack(f3(A.B.pos[id]), isAsleep(m.flags) ? 1.0f : 0.0f);
             } else {
-                T.v[t] = pack(f3(A.B.vel[id]), isRotationLocked(m.flags) ? 1.0f : 0.0f);
+                T.v[t] = pack(f3(A.B.vel[id]), !kFlow && isRotationLocked(m.flags) ? 1.0f : 0.0f);
                 T.w[t] = A.B.ang[id];
             }
         }
         islandBarrier<Threads>();
+        if (kFlow && !position) {
+            // ranks of the rows on their bodies, colour by colour (a colour has one row a body)
+            uint32_t* seen = reinterpret_cast<uint32_t*>(T.f);  // the frames come later
+            for (uint32_t t = threadIdx.x; t < nb; t += Threads) seen[t] = 0u;
+            if (threadIdx.x == 0u) dead = 0;
+            for (uint32_t k = s0 + threadIdx.x; k < s1; k += Threads) {
+                const vx_contact& c = A.contacts[A.order[k]];
+                const bool solved = solvedContact(A.B.filt[c.a].x, A.B.filt[c.b].x);
+                const int la = bodyWord(A, localIdx, b0, nb, c.a, false), lb = bodyWord(A, localIdx, b0, nb, c.b, false);
+                R.side[2 * (size_t)k].w = __int_as_float(solved ? la : kAtRest);
+                R.side[2 * (size_t)k + 1].w = __int_as_float(solved ? lb : kAtRest);
+            }
+            islandBarrier<Threads>();
+            for (uint32_t c = 0; c < colours; ++c) {
+                for (uint32_t x = 2u * seg[c] + threadIdx.x; x < 2u * seg[c + 1]; x += Threads) {
+                    const int li = __float_as_int(R.side[x].w);
+                    if (li >= 0) R.imp[x].w = __uint_as_float(seen[li]++ << kRowLinkShift);
+                }
+                islandBarrier<Threads>();
+            }
+            for (uint32_t x = 2u * s0 + threadIdx.x; x < 2u * s1; x += Threads) {
+                const int li = __float_as_int(R.side[x].w);
+                R.imp[x].w = __uint_as_float(li >= 0 ? __float_as_uint(R.imp[x].w) | seen[li] << kRowDegreeShift : 0u);
+            }
+            if (threadIdx.x < 32u) {  // the batches of each colour, one lane a colour
+                constexpr uint32_t kBatch = ClassShape<Class>::kBatch;
+                uint32_t base = 0u;
+                for (uint32_t c0 = 0; c0 < colours; c0 += 32u) {
+                    const uint32_t c = c0 + threadIdx.x;
+                    const uint32_t from = c < colours ? seg[c] : 0u, to = c < colours ? seg[c + 1] : 0u;
+                    const uint32_t need = (to - from + kBatch - 1u) / kBatch;
+                    uint32_t incl = need;
+                    for (int off = 1; off < 32; off <<= 1) {
+                        const uint32_t y = __shfl_up_sync(0xffffffffu, incl, off);
+                        if ((int)threadIdx.x >= off) incl += y;
+                    }
+                    uint32_t at = base + incl - need;
+                    for (uint32_t k = from; k < to; k += kBatch)
+                        batches[at++] = (uint16_t)((k - s0) | (min(kBatch, to - k) - 1u) << 12);
+                    base += __shfl_sync(0xffffffffu, incl, 31);
+                }
+                if (threadIdx.x == 0u) batchCount = base;
+            }
+            islandBarrier<Threads>();
+        }
         if (position) {
             for (uint32_t k = s0 + threadIdx.x; k < s1; k += Threads) {
                 const vx_contact& c = A.contacts[A.order[k]];
@@ -692,13 +893,14 @@ __global__ void __launch_bounds__(ClassShape<Class>::kThreads, ClassShape<Class>
                     T.v[t] = pack(v, tv.w);
                     T.w[t] = pack(w, 0.0f);
                 }
+                if (kFlow) T.v[t].w = T.w[t].w = 0.0f;  // fresh tags
                 T.f[t] = pack(inertiaFrameAt(m, q));
             }
             islandBarrier<Threads>();
             for (uint32_t k = s0 + threadIdx.x; k < s1; k += Threads) {
                 vx_contact& c = A.contacts[A.order[k]];
                 int la, lb;
-                if (s == 0) {
+                if (s == 0 && !kFlow) {
                     la = bodyWord(A, localIdx, b0, nb, c.a, false);
                     lb = bodyWord(A, localIdx, b0, nb, c.b, false);
                 } else {
@@ -716,13 +918,30 @@ __global__ void __launch_bounds__(ClassShape<Class>::kThreads, ClassShape<Class>
                 R.side[2 * (size_t)k + 1] = pack(P.rb, __int_as_float(lb));
                 float4 imp = make_float4(rc.nImp, rc.t1Imp, rc.t2Imp, 0.0f);
                 if (s > 0) imp = R.imp[2 * (size_t)k];
-                imp.w = __uint_as_float(bits);
-                R.imp[2 * (size_t)k] = R.imp[2 * (size_t)k + 1] = imp;
+                uint32_t wordA = bits, wordB = bits;
+                if (kFlow) {
+                    const uint32_t link = ~((1u << kRowLinkShift) - 1u);
+                    wordA |= (__float_as_uint(R.imp[2 * (size_t)k].w) & link) |
+                             (isRotationLocked(a.m.flags) ? 0u : kRowTurns);
+                    wordB |= (__float_as_uint(R.imp[2 * (size_t)k + 1].w) & link) |
+                             (isRotationLocked(b.m.flags) ? 0u : kRowTurns);
+                }
+                imp.w = __uint_as_float(wordA);
+                R.imp[2 * (size_t)k] = imp;
+                imp.w = __uint_as_float(wordB);
+                R.imp[2 * (size_t)k + 1] = imp;
                 if (setsPoint(A, s, solved, rc)) c.point = vx_vec3{P.point.x, P.point.y, P.point.z};
             }
             islandBarrier<Threads>();
-            if (A.warmStart && s == 0) runColours<Threads, kRowWarm, Cone>(A, R, T, seg, colours, 1);
-            runColours<Threads, kRowSweep, Cone>(A, R, T, seg, colours, A.sweeps);
+            const bool warm = A.warmStart && s == 0;
+            if constexpr (kFlow) {
+                runBatches<Threads, Cone>(A, R, T, batches, batchCount, s0, (warm ? 1u : 0u) + (uint32_t)A.sweeps,
+                                          warm ? 1u : 0u, &dead);
+                islandBarrier<Threads>();
+            } else {
+                if (warm) runColours<Threads, kRowWarm, Cone>(A, R, T, seg, colours, 1);
+                runColours<Threads, kRowSweep, Cone>(A, R, T, seg, colours, A.sweeps);
+            }
             if (A.integrate) {
                 for (uint32_t t = threadIdx.x; t < nb; t += Threads) {
                     const uint32_t id = A.bodyOrder[b0 + t];
