@@ -50,6 +50,15 @@ int injectedFailure(Context& c) {
     return VXB_OK;
 }
 
+void releaseStreams(Context& c) {
+    for (int s = 0; s < 2; ++s) {
+        if (c.joinEvent[s]) cudaEventDestroy(c.joinEvent[s]);
+        if (c.side[s]) cudaStreamDestroy(c.side[s]);
+    }
+    if (c.forkEvent) cudaEventDestroy(c.forkEvent);
+    if (c.ownStream) cudaStreamDestroy(c.ownStream);
+}
+
 int ensureCounters(Context& c) {
     TRY(vxb::ensure(c, c.countersBuf, sizeof(vxb::Counters)));
     c.dCounters = reinterpret_cast<vxb::Counters*>(c.countersBuf.ptr);
@@ -103,10 +112,14 @@ int vxb_context_create(int device, vxb_context** out) {
         return VXB_ERR_DEVICE_LOST;
     }
     c.stream = c.ownStream;
-    if (ensureCounters(c) != VXB_OK) {
-        cudaStreamDestroy(c.ownStream);
+    bool forks = cudaEventCreateWithFlags(&c.forkEvent, cudaEventDisableTiming) == cudaSuccess;
+    for (int s = 0; s < 2; ++s)
+        forks = forks && cudaStreamCreateWithFlags(&c.side[s], cudaStreamNonBlocking) == cudaSuccess &&
+                cudaEventCreateWithFlags(&c.joinEvent[s], cudaEventDisableTiming) == cudaSuccess;
+    if (!forks || ensureCounters(c) != VXB_OK) {
+        releaseStreams(c);
         delete ctx;
-        return VXB_ERR_OOM;
+        return forks ? VXB_ERR_OOM : VXB_ERR_DEVICE_LOST;
     }
     c.tuner.init(device, c.smCount);
     *out = ctx;
@@ -140,7 +153,7 @@ void vxb_context_destroy(vxb_context* ctx) {
                            &c.countersBuf};
     for (vxb::DevBuf* b : bufs)
         if (b->ptr) cudaFree(b->ptr);
-    if (c.ownStream) cudaStreamDestroy(c.ownStream);
+    releaseStreams(c);
     delete ctx;
 }
 

@@ -153,6 +153,8 @@ struct Context {
     uint32_t waitLimit = kSpinLimit;  // polls before a device wait gives up (vxb_context_set_wait_limit)
     cudaStream_t ownStream = nullptr;
     cudaStream_t stream = nullptr;
+    cudaStream_t side[2] = {};  // forked from and joined to `stream` within a call (launchSolve)
+    cudaEvent_t forkEvent = nullptr, joinEvent[2] = {};
     std::string lastError;
     uint64_t launches = 0;
     uint64_t hostSyncs = 0;  // blocking reads of device counts (the stream drains)

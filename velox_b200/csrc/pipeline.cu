@@ -3145,9 +3145,8 @@ static int buildFlow(Context& c, const SolveArgs& A, uint32_t clusters) {
     return VXB_OK;
 }
 
-static int launchSolve(Context& c, const SolveArgs& A) {
-    if (A.islands == 0) return VXB_OK;
-    // tiny islands: pack them into warps once per island plan
+// Tiny islands: packed into warps once per island plan, then one launch.
+static int launchTiny(Context& c, const SolveArgs& A) {
     const uint32_t islands = A.islands, chunksCap = (islands + kPackChunk - 1) / kPackChunk + 1;
     VXB_TRY(ensure(c, c.tinyBuf, ((size_t)islands * 4 + (size_t)chunksCap * 2 + 64) * 4));
     uint32_t* tFlags = P<uint32_t>(c.tinyBuf);
@@ -3186,30 +3185,74 @@ static int launchSolve(Context& c, const SolveArgs& A) {
             A, (const uint32_t*)tList, (const uint32_t*)tFirst, (const Counters*)c.dCounters, P<uint32_t>(c.localIdxBuf));
         ++c.launches;
     }
-    if (c.planLargest > kTinyLimit) {
-        // four warps an island while the GPU holds them all at once
-        const bool few = A.islands <= (uint32_t)(c.smCount * ClassShape<kSmallWide>::kBlocksPerSm);
-        VXB_TRY(few ? launchIslands<kSmallWide>(c, A) : launchIslands<kSmallIsland>(c, A));
-    }
-    if (c.planLargest >= (uint32_t)kSmallBodies) VXB_TRY(launchIslands<kMediumIsland>(c, A));
-    // giant islands: list them, then one cooperative launch over all of them
-    VXB_TRY(ensure(c, c.giantBuf, ((size_t)A.islands + 1) * 4 + 64));
+    return VXB_OK;
+}
+
+// Runs `work` on the context's side stream `s`, forked from its stream at
+// `forkEvent`; the caller joins with joinSide before anything depends on it.
+template <class Work>
+static int onSide(Context& c, int s, Work work) {
+    VXB_CUDA(c, cudaStreamWaitEvent(c.side[s], c.forkEvent, 0));
+    const cudaStream_t own = c.stream;
+    c.stream = c.side[s];
+    const int rc = work();
+    c.stream = own;
+    VXB_CUDA(c, cudaEventRecord(c.joinEvent[s], c.side[s]));
+    return rc;
+}
+static int joinSide(Context& c, int s) {
+    VXB_CUDA(c, cudaStreamWaitEvent(c.stream, c.joinEvent[s], 0));
+    return VXB_OK;
+}
+
+// The classes' kernels touch different islands (their rows, bodies and
+// planes), so tiny and small islands run beside the medium ones: one after
+// the other, each class waited for the last's longest chain. Solve stage of one
+// step, in turn -> side by side: a lattice of 65 bodies as it falls apart
+// 1.65 -> 1.41 ms, 187,000 tiny islands beside some small ones 5.7 -> 5.1 ms,
+// heaps of 3,000 and 40,000 bodies 3.0 -> 2.5 and 4.3 -> 3.8 ms; one class alone
+// (the pyramids) stays at 4.5 ms. The flow starts after the join: it reuses the
+// planes and fills the GPU.
+static int launchSolve(Context& c, const SolveArgs& A) {
+    if (A.islands == 0) return VXB_OK;
+    VXB_TRY(ensure(c, c.localIdxBuf, (size_t)c.n * 4 + 16));
     VXB_TRY(ensure(c, c.coopBuf, sizeof(CoopState)));
+    const uint32_t giants = c.planGiants;  // counted with the island plan
+    int perSm = 0;
+    uint32_t clusters = 0;
+    auto* flow = A.coneBlock ? solveFlowKernel<true> : solveFlowKernel<false>;
+    if (giants && c.cooperative) {  // (its sorts and scans share scratch with the tiny islands' packing)
+        VXB_CUDA(c, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSm, flow, kFlowThreads, 0));
+        perSm = std::min(perSm, kFlowBlocksPerSm);
+        clusters = (uint32_t)(perSm * c.smCount) * (kFlowThreads / 32);
+        if (clusters > 0 && (!c.clusterBuilt || c.clusterCount != clusters)) VXB_TRY(buildFlow(c, A, clusters));
+    }
+    VXB_CUDA(c, cudaEventRecord(c.forkEvent, c.stream));
+    const int tinyStatus = onSide(c, 0, [&] { return launchTiny(c, A); });
+    int smallStatus = VXB_OK;
+    if (c.planLargest > kTinyLimit)
+        smallStatus = onSide(c, 1, [&] {
+            // four warps an island while the GPU holds them all at once
+            const bool few = A.islands <= (uint32_t)(c.smCount * ClassShape<kSmallWide>::kBlocksPerSm);
+            return few ? launchIslands<kSmallWide>(c, A) : launchIslands<kSmallIsland>(c, A);
+        });
+    int mediumStatus = VXB_OK;
+    if (c.planLargest >= (uint32_t)kSmallBodies) mediumStatus = launchIslands<kMediumIsland>(c, A);
+    VXB_TRY(joinSide(c, 0));
+    if (c.planLargest > kTinyLimit) VXB_TRY(joinSide(c, 1));
+    VXB_TRY(tinyStatus);
+    VXB_TRY(smallStatus);
+    VXB_TRY(mediumStatus);
+    if (!giants) return VXB_OK;
+    // giant islands: list them, then one cooperative launch over all of them
     CoopState* st = P<CoopState>(c.coopBuf);
+    VXB_TRY(ensure(c, c.giantBuf, ((size_t)A.islands + 1) * 4 + 64));
     uint32_t* list = P<uint32_t>(c.giantBuf);
     VXB_TRY(resetCoop(c, st));
-    const uint32_t giants = c.planGiants;  // counted with the island plan
-    if (!giants) return VXB_OK;
     LAUNCH(c, giantListKernel, std::min<uint32_t>(blocksFor(A.islands, 256), (uint32_t)c.smCount * 4), 256, A, list,
            &st->rounds);
     c.stats.giantIslands = std::max(c.stats.giantIslands, giants);
-    int perSm = 0;
-    auto* flow = A.coneBlock ? solveFlowKernel<true> : solveFlowKernel<false>;
-    VXB_CUDA(c, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSm, flow, kFlowThreads, 0));
-    perSm = std::min(perSm, kFlowBlocksPerSm);
-    const uint32_t clusters = (uint32_t)(perSm * c.smCount) * (kFlowThreads / 32);
-    if (c.cooperative && clusters > 0) {
-        if (!c.clusterBuilt || c.clusterCount != clusters) VXB_TRY(buildFlow(c, A, clusters));
+    if (clusters > 0) {
         if (c.clusterR > 0 && !c.hostCounters.flowTooWide) {
             FlowArgs F;
             F.start = P<uint32_t>(c.clusterStartBuf);
