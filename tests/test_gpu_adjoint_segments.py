@@ -10,17 +10,21 @@ import velox_b200 as vb
 pytestmark = pytest.mark.gpu
 
 
-def gradients(worlds, steps, every):
+def taped(ctx, worlds, steps, every):
     specs, pool = vb.generate_scene(5, seed=3, size=worlds)
     bodies, hull, faces = vb.bodies_from_specs(specs, pool)
+    ctx.load(bodies, vb.make_soup(hull, faces), world_of=np.ascontiguousarray(specs["world"], np.uint32))
+    ctx.configure(substeps=4)
+    ctx.tape_begin(steps, every)
+    ctx.step(steps)
+    seed = np.random.default_rng(1).normal(size=(len(bodies), 13)).astype(np.float32)
+    return ctx.adjoint_backward(seed)
+
+
+def gradients(worlds, steps, every):
     ctx = vb.Context(0)
     try:
-        ctx.load(bodies, vb.make_soup(hull, faces), world_of=np.ascontiguousarray(specs["world"], np.uint32))
-        ctx.configure(substeps=4)
-        ctx.tape_begin(steps, every)
-        ctx.step(steps)
-        seed = np.random.default_rng(1).normal(size=(len(bodies), 13)).astype(np.float32)
-        return ctx.adjoint_backward(seed)
+        return taped(ctx, worlds, steps, every)
     finally:
         ctx.close()
 
@@ -34,3 +38,20 @@ def test_gradients_do_not_depend_on_the_tape(worlds, steps, spacings):
     for every in spacings[1:]:
         for x, y in zip(first, gradients(worlds, steps, every)):
             assert np.array_equal(x, y), every
+
+
+# A context's tapes share memory from one to the next: larger, smaller, after
+# an untaped world (which gives it back) and after vxb_tape_end.
+@pytest.mark.parametrize("between", ["nothing", "untaped", "end"])
+def test_tapes_of_one_context_are_independent(ctx, between):
+    for worlds, steps, every in [(20, 5, 2), (3, 9, 4), (40, 5, 5), (20, 5, 2)]:
+        for x, y in zip(gradients(worlds, steps, every), taped(ctx, worlds, steps, every)):
+            assert np.array_equal(x, y), (worlds, steps, every)
+        if between == "untaped":
+            specs, pool = vb.generate_scene(5, seed=4, size=7)
+            bodies, hull, faces = vb.bodies_from_specs(specs, pool)
+            for _ in range(2):
+                ctx.load(bodies, vb.make_soup(hull, faces), world_of=np.ascontiguousarray(specs["world"], np.uint32))
+                ctx.step(1)
+        elif between == "end":
+            ctx.tape_end()

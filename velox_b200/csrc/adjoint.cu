@@ -73,6 +73,10 @@ constexpr uint32_t kNoColour = 0x7fffffffu;
 // and each step again with one: a third more row updates (backward pass of 128
 // rollouts of 24 steps 126 against 186 ms, of 1,024 of 10 steps 65 against 98).
 constexpr size_t kSegmentTapeLimit = (size_t)4 << 30;
+// Memory an ended tape may hold for the next one (the scratch above with the
+// allocator's half on top). Freeing and allocating it for each pass of a loop
+// over load, tape and backward took 0 to 50 of 200 ms, now and then a second (128 rollouts of 24 steps: now 177 each time).
+constexpr size_t kTapeKeepLimit = (size_t)6 << 30;
 
 inline uint32_t gridFor(uint64_t items, int threads) {
     uint64_t b = (items + threads - 1) / threads;
@@ -84,11 +88,7 @@ int growKeep(Context& c, DevBuf& b, size_t bytes, size_t keep) {
     if (bytes <= b.bytes && b.ptr) return VXB_OK;
     void* fresh = nullptr;
     const size_t want = std::max(bytes, b.bytes * 2) + 256;
-    cudaError_t e = cudaMalloc(&fresh, want);
-    if (e != cudaSuccess) {
-        cudaGetLastError();
-        return cudaStatus(c, e, "cudaMalloc (tape)");
-    }
+    AD_TRY(allocate(c, b, &fresh, want));
     if (b.ptr && keep) AD_CUDA(c, cudaMemcpyAsync(fresh, b.ptr, keep, cudaMemcpyDeviceToDevice, c.stream));
     if (b.ptr) {
         AD_CUDA(c, cudaStreamSynchronize(c.stream));
@@ -1193,6 +1193,7 @@ int tapeBegin(Context& c, uint32_t steps, uint32_t every) {
     if (c.n == 0) return fail(c, VXB_ERR_INVALID, "tape: no bodies loaded");
     Tape& T = c.tape;
     T.active = true;
+    T.begun = true;
     T.steps = steps;
     T.every = every;
     T.recorded = 0;
@@ -1205,14 +1206,21 @@ int tapeBegin(Context& c, uint32_t steps, uint32_t every) {
     return VXB_OK;
 }
 
-int tapeEnd(Context& c) {
+// keep: the buffers stay up to kTapeKeepLimit in sum. A load after a world that
+// was never taped keeps none, so a program that stops taping gets the memory back.
+int tapeEnd(Context& c, bool keep) {
     Tape& T = c.tape;
     T.active = false;
     T.recorded = 0;
     T.stepStart.assign(1, 0u);
     if (T.contacts.ptr || T.ckpt.ptr || T.scratch.ptr || T.branches.ptr) cudaStreamSynchronize(c.stream);
-    for (DevBuf* b : {&T.contacts, &T.src, &T.color, &T.worldStart, &T.ckpt, &T.flags, &T.scratch, &T.host,
+    size_t held = 0;
+    for (DevBuf* b : {&T.scratch, &T.contacts, &T.src, &T.color, &T.worldStart, &T.ckpt, &T.flags, &T.host,
                       &T.branches}) {
+        if (keep && held + b->bytes <= kTapeKeepLimit) {
+            held += b->bytes;
+            continue;
+        }
         if (b->ptr) cudaFree(b->ptr);
         b->ptr = nullptr;
         b->bytes = 0;

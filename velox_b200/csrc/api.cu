@@ -361,7 +361,8 @@ int vxb_world_load(vxb_context* ctx, const vx_body* bodies, uint32_t n, const vx
                 return vxb::fail(c, VXB_ERR_INVALID, "body " + std::to_string(i) + ": " + why);
     }
     TRY(ensureCounters(c));
-    vxb::tapeEnd(c);  // a tape belongs to the world it recorded
+    vxb::tapeEnd(c, c.tape.begun);  // a tape belongs to the world it recorded
+    c.tape.begun = false;
     c.backendContacts = 0;  // a new world: no coloured Backend contacts
     c.backendColored = false;
     TRY(vxb::loadBodies(c, bodies, n, worldOfBody, true));
@@ -510,7 +511,7 @@ int vxb_tape_begin(vxb_context* ctx, uint32_t steps, uint32_t checkpointEvery) {
     GUARD(ctx);
     Context& c = ctx->impl;
     if (!c.configured) return vxb::fail(c, VXB_ERR_INVALID, "vxb_world_configure was not called");
-    TRY(vxb::tapeEnd(c));
+    TRY(vxb::tapeEnd(c, true));
     return vxb::tapeBegin(c, steps, checkpointEvery);
 }
 

@@ -54,6 +54,7 @@ struct DeviceSnapshot {
 // Recording of the device world's steps for the adjoint (adjoint.cu).
 struct Tape {
     bool active = false;
+    bool begun = false;  // since the last world load
     uint32_t steps = 0, every = 0, recorded = 0;
     std::vector<uint32_t> stepStart{0u};  // first contact of each recorded step (+ total)
     DevBuf contacts;    // vx_contact per contact, after warm-start matching
@@ -346,7 +347,9 @@ bool finiteValues(const float* v, size_t count);
 
 // Adjoint (adjoint.cu): tape hooks of the device world's step, and the backward pass.
 int tapeBegin(Context& c, uint32_t steps, uint32_t every);
-int tapeEnd(Context& c);
+// keep: the memory stays for the next tape, within bounds (adjoint.cu).
+int tapeEnd(Context& c, bool keep = false);
+int allocate(Context& c, const DevBuf& b, void** out, size_t bytes);
 int tapeStepBegin(Context& c);
 int tapeBeforeMatch(Context& c, const vx_contact* cs, uint32_t m, const vx_contact* prev, const uint64_t* prevKeys,
                     uint32_t mPrev);

@@ -52,16 +52,33 @@ int cudaStatus(Context& c, cudaError_t e, const char* what) {
     return fail(c, VXB_ERR_INVALID, msg);
 }
 
+// cudaMalloc for `b`. When memory is short, what the tape holds without using
+// it goes back first: everything of an ended tape, the scratch of a live one.
+int allocate(Context& c, const DevBuf& b, void** out, size_t bytes) {
+    cudaError_t e = cudaMalloc(out, bytes);
+    if (e == cudaErrorMemoryAllocation) {
+        cudaGetLastError();
+        if (!c.tape.active) {
+            tapeEnd(c);
+        } else if (&b != &c.tape.scratch && c.tape.scratch.ptr) {
+            cudaFree(c.tape.scratch.ptr);
+            c.tape.scratch = DevBuf{};
+        }
+        e = cudaMalloc(out, bytes);
+    }
+    if (e != cudaSuccess) cudaGetLastError();
+    return e == cudaSuccess ? VXB_OK : cudaStatus(c, e, "cudaMalloc");
+}
+
 int ensure(Context& c, DevBuf& b, size_t bytes) {
     if (bytes <= b.bytes && b.ptr) return VXB_OK;
     if (b.ptr) cudaFree(b.ptr);
     b.ptr = nullptr;
     b.bytes = 0;
     size_t want = bytes + bytes / 2 + 256;
-    cudaError_t e = cudaMalloc(&b.ptr, want);
-    if (e != cudaSuccess) {
-        cudaGetLastError();
-        return cudaStatus(c, e, "cudaMalloc");
+    if (const int rc = allocate(c, b, &b.ptr, want)) {
+        b.ptr = nullptr;
+        return rc;
     }
     b.bytes = want;
     return VXB_OK;
