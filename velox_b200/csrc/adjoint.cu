@@ -71,11 +71,13 @@ constexpr uint32_t kNoColour = 0x7fffffffu;
 // recomputes it (64 bytes per row update: 1.4 GB for 1,024 worlds of 34 rows and
 // 10 steps a segment). Beyond it the segment runs forward once without a tape
 // and each step again with one: a third more row updates (backward pass of 128
-// rollouts of 24 steps 126 against 186 ms, of 1,024 of 10 steps 65 against 98).
+// rollouts of 24 steps 126 against 186 ms, of 1,024 of 10 steps 65 against 98,
+// both with the rows' state in global memory).
 constexpr size_t kSegmentTapeLimit = (size_t)4 << 30;
 // Memory an ended tape may hold for the next one (the scratch above with the
 // allocator's half on top). Freeing and allocating it for each pass of a loop
-// over load, tape and backward took 0 to 50 of 200 ms, now and then a second (128 rollouts of 24 steps: now 177 each time).
+// over load, tape and backward took 0 to 50 of 200 ms, now and then a second
+// (128 rollouts of 24 steps).
 constexpr size_t kTapeKeepLimit = (size_t)6 << 30;
 
 inline uint32_t gridFor(uint64_t items, int threads) {
@@ -285,9 +287,11 @@ struct AdjArgs {
     size_t worldBytes;
     size_t tapeBytes;              // bytes of one step's tape (sub .. lamInit); its slots lie one after another
     int segmentTape;               // a slot per step of a segment: the segment runs forward once
-    // offsets inside a world's slice
-    size_t oSt, oSub, oEnd, oCorr, oRin, oPush, oLam, oLamInit, oPrep, oPbar, oOrder, oCstart, oLamb0, oLamb1,
-        oCur, oAdj, oGm;
+    size_t hotOffset, hotBytes;    // what every row update touches (oLam ..): in the slice or in shared memory
+    int hotShared;
+    // offsets inside a world's slice, and inside its hot part
+    size_t oSt, oSub, oEnd, oCorr, oRin, oPush, oLamInit;
+    size_t oLam, oPrep, oPbar, oOrder, oCstart, oLamb0, oLamb1, oCur, oAdj, oGm;
 };
 
 struct WorldView {
@@ -313,16 +317,18 @@ VXD WorldView carve(const AdjArgs& A, uint32_t w) {
     char* base = A.scratch + (size_t)w * A.worldBytes;
     WorldView V;
     V.st = reinterpret_cast<float4*>(base + A.oSt);
-    V.lam = reinterpret_cast<float4*>(base + A.oLam);
-    V.prep = reinterpret_cast<RowPrep*>(base + A.oPrep);
-    V.pbar = reinterpret_cast<PrepBar*>(base + A.oPbar);
-    V.order = reinterpret_cast<uint32_t*>(base + A.oOrder);
-    V.cstart = reinterpret_cast<uint32_t*>(base + A.oCstart);
-    V.lamb[0] = reinterpret_cast<float4*>(base + A.oLamb0);
-    V.lamb[1] = reinterpret_cast<float4*>(base + A.oLamb1);
-    V.cur = reinterpret_cast<float4*>(base + A.oCur);
-    V.adj = reinterpret_cast<BodyBar*>(base + A.oAdj);
-    V.gm = reinterpret_cast<float2*>(base + A.oGm);
+    extern __shared__ float4 hotShared[];
+    char* hot = A.hotShared ? reinterpret_cast<char*>(hotShared) + (threadIdx.x / 32) * A.hotBytes : base + A.hotOffset;
+    V.lam = reinterpret_cast<float4*>(hot + A.oLam);
+    V.prep = reinterpret_cast<RowPrep*>(hot + A.oPrep);
+    V.pbar = reinterpret_cast<PrepBar*>(hot + A.oPbar);
+    V.order = reinterpret_cast<uint32_t*>(hot + A.oOrder);
+    V.cstart = reinterpret_cast<uint32_t*>(hot + A.oCstart);
+    V.lamb[0] = reinterpret_cast<float4*>(hot + A.oLamb0);
+    V.lamb[1] = reinterpret_cast<float4*>(hot + A.oLamb1);
+    V.cur = reinterpret_cast<float4*>(hot + A.oCur);
+    V.adj = reinterpret_cast<BodyBar*>(hot + A.oAdj);
+    V.gm = reinterpret_cast<float2*>(hot + A.oGm);
     return V;
 }
 
@@ -1042,7 +1048,17 @@ struct WorldRun {
     }
 };
 
-__global__ void __launch_bounds__(128) adjointKernel(AdjArgs A) {
+// One warp a world. A row update waits on what the last one wrote (velocities,
+// impulses, prepared rows, adjoints): that part of a world's memory lies in
+// shared memory while an SM's worlds fit there, up to the 8 warps that its
+// registers hold; beyond that in the scratch. 128 rollouts of 24 steps, scratch
+// -> shared: 127 -> 96 ms, 1,024 of 10 steps 63 -> 47 ms. Then a warp's
+// instructions bound it (3.6 cycles each, a third of it issue); held to 128
+// registers it spilled (96 against 92 ms, 47 against 45).
+constexpr size_t kAdjointShared = (size_t)220 << 10;
+constexpr uint32_t kAdjointWarpsPerSm = 8;
+
+__global__ void __launch_bounds__(128, 2) adjointKernel(const __grid_constant__ AdjArgs A) {
     const uint32_t w = blockIdx.x * (blockDim.x / 32) + threadIdx.x / 32;
     if (w >= A.worlds) return;
     WorldRun R(A, w);
@@ -1363,20 +1379,23 @@ int adjointBackward(Context& c, const float* seed, float* grad, float* gradInv, 
     A.oCur = o; o += al(4 * NBs * 16);
     A.oAdj = o; o += al(NBs * sizeof(BodyBar));
     A.oGm = o; o += al(NBs * 8);
-    // (offsets behind the tape so far are relative to its end)
-    const size_t rest = o;
-    size_t* behind[] = {&A.oLam, &A.oPrep, &A.oPbar, &A.oOrder, &A.oCstart, &A.oLamb0, &A.oLamb1, &A.oCur, &A.oAdj, &A.oGm};
+    const size_t rest = A.hotBytes = o;
     A.segmentTape = (afterTape + segmentExtra + rest) * worlds <= kSegmentTapeLimit ? 1 : 0;
     if (A.segmentTape && ensure(c, T.scratch, (afterTape + segmentExtra + rest) * worlds) != VXB_OK) A.segmentTape = 0;
     if (A.segmentTape) afterTape += segmentExtra;
-    for (size_t* off : behind) *off += afterTape;
+    A.hotOffset = afterTape;
     A.worldBytes = afterTape + rest;
     if (!A.segmentTape) AD_TRY(ensure(c, T.scratch, A.worldBytes * worlds));
     A.scratch = PT<char>(T.scratch);
     // few worlds: one per SM before they share one
     const uint32_t perSm = (worlds + (uint32_t)c.smCount - 1) / (uint32_t)c.smCount;
     const int worldsPerBlock = (int)std::min<uint32_t>(4u, std::max<uint32_t>(1u, perSm));
-    AD_LAUNCH(c, adjointKernel, (worlds + worldsPerBlock - 1) / worldsPerBlock, 32 * worldsPerBlock, A);
+    A.hotShared = A.hotBytes * std::min<uint32_t>(perSm, kAdjointWarpsPerSm) <= kAdjointShared &&
+                  A.hotBytes * worldsPerBlock <= kAdjointShared;
+    const size_t smem = A.hotShared ? A.hotBytes * worldsPerBlock : 0;
+    AD_CUDA(c, cudaFuncSetAttribute(adjointKernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kAdjointShared));
+    adjointKernel<<<(worlds + worldsPerBlock - 1) / worldsPerBlock, 32 * worldsPerBlock, smem, c.stream>>>(A);
+    ++c.launches;
     AD_CUDA(c, cudaGetLastError());
     if (grad) AD_CUDA(c, cudaMemcpyAsync(grad, dGrad, (size_t)n * 13 * 4, cudaMemcpyDeviceToHost, c.stream));
     if (gradInv) AD_CUDA(c, cudaMemcpyAsync(gradInv, dGradInv, (size_t)n * 2 * 4, cudaMemcpyDeviceToHost, c.stream));
