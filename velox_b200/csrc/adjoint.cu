@@ -67,8 +67,8 @@ constexpr uint32_t kBrRestitution = 1, kBrResMax = 2, kBrClamp = 4, kBrFriction 
                    kBrEllipse = 64, kBrSkip = 128;
 constexpr uint32_t kNoColour = 0x7fffffffu;
 
-// Scratch up to which a backward pass tapes every step of a segment while it
-// recomputes it (64 bytes per row update: 1.4 GB for 1,024 worlds of 34 rows and
+// Scratch up to which a backward pass tapes every step of all segments at once
+// (see AdjointPart), else of one segment while it recomputes it (64 bytes per row update: 1.4 GB for 1,024 worlds of 34 rows and
 // 10 steps a segment). Beyond it the segment runs forward once without a tape
 // and each step again with one: a third more row updates (backward pass of 128
 // rollouts of 24 steps 126 against 186 ms, of 1,024 of 10 steps 65 against 98,
@@ -1058,12 +1058,36 @@ struct WorldRun {
 constexpr size_t kAdjointShared = (size_t)220 << 10;
 constexpr uint32_t kAdjointWarpsPerSm = 8;
 
+// A segment's recomputation starts at its checkpoint and so needs no other
+// segment: while the GPU has warps to spare and the scratch holds every step's
+// tape, all segments are recomputed at once, a warp each (kRecompute), and the
+// reverse follows over the finished tapes (kReverse). Otherwise a world's warp
+// takes them in turn (kInTurn). 128 rollouts of 24 steps in three segments: 92 ->
+// 76 ms; with one segment or 8 worlds an SM there is nothing to overlap.
+enum AdjointPart : int { kInTurn = 0, kRecompute, kReverse };
+
+template <int Part>
 __global__ void __launch_bounds__(128, 2) adjointKernel(const __grid_constant__ AdjArgs A) {
-    const uint32_t w = blockIdx.x * (blockDim.x / 32) + threadIdx.x / 32;
-    if (w >= A.worlds) return;
+    const uint32_t item = blockIdx.x * (blockDim.x / 32) + threadIdx.x / 32;
+    if (item >= (Part == kRecompute ? A.worlds * A.J : A.worlds)) return;
+    const uint32_t w = Part == kRecompute ? item % A.worlds : item;
     WorldRun R(A, w);
     if (R.nb > A.NB) {
         if (R.lane == 0) atomicOr(A.flags + w, (uint32_t)VXB_ADJ_UNSUPPORTED);
+        return;
+    }
+    auto recompute = [&](uint32_t seg, uint32_t t0, uint32_t t1, uint32_t slot0) {
+        R.loadCheckpoint(seg, R.V.cur);
+        for (uint32_t t = t0; t < t1; ++t) {
+            R.copyState(R.V.st + (size_t)(t - slot0) * 4 * A.NB, R.V.cur);
+            if (A.segmentTape) R.tapeSlot(t - slot0);
+            R.forwardStep(t, A.segmentTape != 0);
+        }
+        if (!R.matchesCheckpoint(seg + 1, R.V.cur) && R.lane == 0) atomicOr(A.flags + w, (uint32_t)VXB_ADJ_DIVERGED);
+    };
+    if constexpr (Part == kRecompute) {
+        const uint32_t seg = item / A.worlds;
+        recompute(seg, seg * A.every, min(A.steps, (seg + 1u) * A.every), 0u);
         return;
     }
     // seeds, zeroed accumulators
@@ -1085,20 +1109,14 @@ __global__ void __launch_bounds__(128, 2) adjointKernel(const __grid_constant__ 
     for (int seg = (int)A.J - 1; seg >= 0; --seg) {
         const uint32_t t0 = (uint32_t)seg * A.every;
         const uint32_t t1 = min(A.steps, t0 + A.every);
-        R.loadCheckpoint((uint32_t)seg, R.V.cur);
-        for (uint32_t t = t0; t < t1; ++t) {
-            R.copyState(R.V.st + (size_t)(t - t0) * 4 * A.NB, R.V.cur);
-            if (A.segmentTape) R.tapeSlot(t - t0);
-            R.forwardStep(t, A.segmentTape != 0);
-        }
-        if (!R.matchesCheckpoint((uint32_t)seg + 1, R.V.cur) && R.lane == 0)
-            atomicOr(A.flags + w, (uint32_t)VXB_ADJ_DIVERGED);
+        const uint32_t slot0 = Part == kInTurn ? t0 : 0u;  // step of the first tape slot
+        if constexpr (Part == kInTurn) recompute((uint32_t)seg, t0, t1, t0);
         for (int t = (int)t1 - 1; t >= (int)t0; --t) {
-            const float4* start = R.V.st + (size_t)(t - t0) * 4 * A.NB;
+            const float4* start = R.V.st + (size_t)((uint32_t)t - slot0) * 4 * A.NB;
             if (A.segmentTape) {
                 uint32_t c0;
                 const uint32_t m = R.rowsOf((uint32_t)t, c0);
-                R.tapeSlot((uint32_t)t - t0);
+                R.tapeSlot((uint32_t)t - slot0);
                 R.buildOrder(c0, m);
             } else {
                 R.copyState(R.V.cur, start);
@@ -1380,22 +1398,43 @@ int adjointBackward(Context& c, const float* seed, float* grad, float* gradInv, 
     A.oAdj = o; o += al(NBs * sizeof(BodyBar));
     A.oGm = o; o += al(NBs * 8);
     const size_t rest = A.hotBytes = o;
-    A.segmentTape = (afterTape + segmentExtra + rest) * worlds <= kSegmentTapeLimit ? 1 : 0;
-    if (A.segmentTape && ensure(c, T.scratch, (afterTape + segmentExtra + rest) * worlds) != VXB_OK) A.segmentTape = 0;
-    if (A.segmentTape) afterTape += segmentExtra;
+    // few worlds: one per SM before they share one
+    auto perBlock = [&](uint32_t warps) {
+        return std::min<uint32_t>(4u, std::max<uint32_t>(1u, (warps + (uint32_t)c.smCount - 1) / (uint32_t)c.smCount));
+    };
+    const uint32_t perSm = (worlds + (uint32_t)c.smCount - 1) / (uint32_t)c.smCount, segments = worlds * A.J;
+    A.hotShared = A.hotBytes * std::min<uint32_t>(perSm, kAdjointWarpsPerSm) <= kAdjointShared &&
+                  A.hotBytes * perBlock(worlds) <= kAdjointShared;
+    // every step's tape at once, or one segment's, or one step's
+    const size_t wholeExtra = al((size_t)steps * 4 * NBs * 16) - tape0 + A.tapeBytes * (steps - 1);
+    const bool whole = A.J > 1 && A.hotShared && A.hotBytes * perBlock(segments) <= kAdjointShared &&
+                       perSm < kAdjointWarpsPerSm &&
+                       (afterTape + wholeExtra + rest) * worlds <= kSegmentTapeLimit &&
+                       ensure(c, T.scratch, (afterTape + wholeExtra + rest) * worlds) == VXB_OK;
+    A.segmentTape = whole || ((afterTape + segmentExtra + rest) * worlds <= kSegmentTapeLimit &&
+                              ensure(c, T.scratch, (afterTape + segmentExtra + rest) * worlds) == VXB_OK);
+    if (whole) {
+        const size_t states = al((size_t)steps * 4 * NBs * 16) - tape0;
+        for (size_t* off : {&A.oSub, &A.oEnd, &A.oCorr, &A.oRin, &A.oPush, &A.oLamInit}) *off += states;
+    }
+    if (A.segmentTape) afterTape += whole ? wholeExtra : segmentExtra;
     A.hotOffset = afterTape;
     A.worldBytes = afterTape + rest;
     if (!A.segmentTape) AD_TRY(ensure(c, T.scratch, A.worldBytes * worlds));
     A.scratch = PT<char>(T.scratch);
-    // few worlds: one per SM before they share one
-    const uint32_t perSm = (worlds + (uint32_t)c.smCount - 1) / (uint32_t)c.smCount;
-    const int worldsPerBlock = (int)std::min<uint32_t>(4u, std::max<uint32_t>(1u, perSm));
-    A.hotShared = A.hotBytes * std::min<uint32_t>(perSm, kAdjointWarpsPerSm) <= kAdjointShared &&
-                  A.hotBytes * worldsPerBlock <= kAdjointShared;
-    const size_t smem = A.hotShared ? A.hotBytes * worldsPerBlock : 0;
-    AD_CUDA(c, cudaFuncSetAttribute(adjointKernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kAdjointShared));
-    adjointKernel<<<(worlds + worldsPerBlock - 1) / worldsPerBlock, 32 * worldsPerBlock, smem, c.stream>>>(A);
-    ++c.launches;
+    auto launch = [&](auto* kernel, uint32_t warps) {
+        const uint32_t block = perBlock(warps);
+        AD_CUDA(c, cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kAdjointShared));
+        kernel<<<(warps + block - 1) / block, 32 * block, A.hotShared ? A.hotBytes * block : 0, c.stream>>>(A);
+        ++c.launches;
+        return (int)VXB_OK;
+    };
+    if (whole) {
+        AD_TRY(launch(adjointKernel<kRecompute>, segments));
+        AD_TRY(launch(adjointKernel<kReverse>, worlds));
+    } else {
+        AD_TRY(launch(adjointKernel<kInTurn>, worlds));
+    }
     AD_CUDA(c, cudaGetLastError());
     if (grad) AD_CUDA(c, cudaMemcpyAsync(grad, dGrad, (size_t)n * 13 * 4, cudaMemcpyDeviceToHost, c.stream));
     if (gradInv) AD_CUDA(c, cudaMemcpyAsync(gradInv, dGradInv, (size_t)n * 2 * 4, cudaMemcpyDeviceToHost, c.stream));
