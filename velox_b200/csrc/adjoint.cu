@@ -68,11 +68,12 @@ constexpr uint32_t kBrRestitution = 1, kBrResMax = 2, kBrClamp = 4, kBrFriction 
 constexpr uint32_t kNoColour = 0x7fffffffu;
 
 // Scratch up to which a backward pass tapes every step of all segments at once
-// (see AdjointPart), else of one segment while it recomputes it (64 bytes per row update: 1.4 GB for 1,024 worlds of 34 rows and
-// 10 steps a segment). Beyond it the segment runs forward once without a tape
-// and each step again with one: a third more row updates (backward pass of 128
-// rollouts of 24 steps 126 against 186 ms, of 1,024 of 10 steps 65 against 98,
-// both with the rows' state in global memory).
+// (AdjointPart below), else of one segment while it recomputes it (64 bytes per
+// row update: 1.4 GB for 1,024 worlds of 34 rows and 10 steps a segment). Beyond
+// it the segment runs forward once without a tape and each step again with one:
+// a third more row updates (backward pass of 128 rollouts of 24 steps 126 against
+// 186 ms, of 1,024 of 10 steps 65 against 98, both with the rows' state in global
+// memory).
 constexpr size_t kSegmentTapeLimit = (size_t)4 << 30;
 // Memory an ended tape may hold for the next one (the scratch above with the
 // allocator's half on top). Freeing and allocating it for each pass of a loop
