@@ -1316,7 +1316,7 @@ __global__ void bodyStartKernel(const uint64_t* keys, uint32_t n, uint32_t* body
     }
 }
 
-// Islands the block kernels cannot hold (solveClusterKernel's share), counted
+// Islands the block kernels cannot hold (the grid's flow), counted
 // for the host's single read of the plan.
 __global__ void giantCountKernel(const uint32_t* islandStart, const uint32_t* bodyStart, uint32_t islands,
                                  uint32_t realIslands, Counters* C) {
