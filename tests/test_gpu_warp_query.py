@@ -49,3 +49,22 @@ def test_warp_query_equals_the_thread_query(ctx, seed, hull_points, spread, qual
     thread = ctx.distance(body, soup, pairs, path=1)
     assert (thread[:, 10] == 1).sum() > 500
     assert np.array_equal(warp.view(np.uint32), thread.view(np.uint32))
+
+
+# Hulls of many points on a sphere, deep in one another: EPA removes faces and
+# reuses their slots in nearly every iteration, with horizons on both sides of
+# 32 edges. Lanes pass vertices, faces and edges through shared memory, so the
+# same bits must come back from every run.
+@pytest.mark.parametrize("points", [24, 70])
+def test_reused_face_slots(ctx, points):
+    body, soup, pairs = scene(5, 4, 0.05)
+    rng = np.random.default_rng(points)
+    n = len(body)
+    body["shape"], body["radius"] = 5, 0.5
+    body["hullFirst"], body["hullCount"] = np.arange(n) * points, points
+    d = rng.normal(size=(n * points, 3))
+    soup = vb.make_soup(0.5 * d / np.linalg.norm(d, axis=1, keepdims=True), np.zeros(0))
+    thread = ctx.distance(body, soup, pairs, path=1)
+    assert (thread[:, 10] == 1).sum() > 4000
+    for _ in range(3):
+        assert np.array_equal(ctx.distance(body, soup, pairs, path=0).view(np.uint32), thread.view(np.uint32))

@@ -379,6 +379,9 @@ static __device__ __noinline__ bool epaWarp(const Simplex& s, GjkResult& result)
             open[chunk] = __ballot_sync(kFullWarp, i < (uint32_t)faceCount && (sees || !(ids & kValid)));
             horizon(W, __ballot_sync(kFullWarp, sees), ids, edgeCount, myEdge, spilled);
         }
+        // The new vertex and the cleared faces are other lanes' writes (votes and
+        // shuffles order no memory), and the new faces reuse slots just read.
+        __syncwarp();
         // the horizon's new faces, in order, into the lowest open slots, then behind the last
         uint32_t made = 0u, opened = 0u;
         for (int chunk = 0; chunk < kEpaFaces / 32; ++chunk) opened += (uint32_t)__popc(open[chunk]);
