@@ -113,3 +113,34 @@ def test_many_small_islands_on_one_warp_each(ctx):
         at = i * (n + 1)
         for name in ("position", "orientation", "velocity", "angularVelocity"):
             assert np.array_equal(got[name][at:at + n + 1], want[name]), (i, name)
+
+
+# Rows of one body wait for one another through the tags in shared memory: equal
+# worlds solved by many blocks at once, again and again, end in equal bits (a
+# heap of 36 spheres is a small island, on four warps; one of 180 a medium one).
+@pytest.mark.parametrize("layers", [1, 5])
+def test_equal_crowded_islands_end_equal(ctx, layers):
+    per, worlds = 36 * layers, 200
+    k = np.arange(per)
+    s = np.zeros(per + 1, SPEC)
+    s["orientation"] = (0, 0, 0, 1)
+    s["shape"][0] = 1
+    s["planeNormal"][0] = (0, 1, 0)
+    s["mass"][1:], s["radius"][1:], s["friction"][1:] = 1.0, 0.5, 0.5
+    s["position"][1:] = np.stack([k % 6, k // 36, k // 6 % 6], 1) * 0.985 + (0.0, 0.49, 0.0)
+    s["velocity"][1:] = np.random.default_rng(layers).normal(0.0, 0.3, (per, 3))
+    bodies, hull, faces = vb.bodies_from_specs(s, np.zeros((0, 3), np.float32))
+    many = vb.binding.records(np.concatenate([bodies] * worlds).astype(vb.BODY), vb.BODY).copy()
+    world_of = np.repeat(np.arange(worlds, dtype=np.uint32), per + 1)
+    first = None
+    for _ in range(3):
+        ctx.load(many, vb.make_soup(hull, faces), world_of)
+        ctx.configure(dt=4 * H, substeps=4, gravity=(0.0, -9.81, 0.0))
+        ctx.step(1)
+        assert ctx.stats()["giantIslands"] == 0
+        got = ctx.read_bodies()
+        for name in ("position", "orientation", "velocity", "angularVelocity"):
+            x = got[name].reshape(worlds, per + 1, -1)
+            first = first or {}
+            first.setdefault(name, x[0].copy())
+            assert np.array_equal(x, np.broadcast_to(first[name], x.shape)), name

@@ -560,17 +560,24 @@ VXD void runColours(const SolveArgs& A, const RowPlanes& R, const BodyTable& T, 
 // poll), as was sleeping between polls.
 constexpr uint32_t kTableWaitLimit = 1u << 22;  // polls of about 50 cycles
 
+// Whole 16-byte accesses: a vector access is four scalar ones in any order to
+// the memory model, a .b128 one is a single access, so a body's velocity
+// arrives with the tag that announces it.
 VXD float4 ldTable(const float4* p) {
-    float4 v;
-    asm volatile("ld.volatile.shared.v4.f32 {%0, %1, %2, %3}, [%4];"
-                 : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
+    unsigned long long lo, hi;
+    asm volatile("{\n\t.reg .b128 t;\n\tld.relaxed.cta.shared.b128 t, [%2];\n\tmov.b128 {%0, %1}, t;\n\t}"
+                 : "=l"(lo), "=l"(hi)
                  : "r"((uint32_t)__cvta_generic_to_shared(p))
                  : "memory");
-    return v;
+    return make_float4(__uint_as_float((uint32_t)lo), __uint_as_float((uint32_t)(lo >> 32)),
+                       __uint_as_float((uint32_t)hi), __uint_as_float((uint32_t)(hi >> 32)));
 }
 VXD void stTable(float4* p, const V3& v, uint32_t tag) {
-    asm volatile("st.volatile.shared.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"((uint32_t)__cvta_generic_to_shared(p)),
-                 "f"(v.x), "f"(v.y), "f"(v.z), "f"(__uint_as_float(tag))
+    const unsigned long long lo = (unsigned long long)__float_as_uint(v.y) << 32 | __float_as_uint(v.x);
+    const unsigned long long hi = (unsigned long long)tag << 32 | __float_as_uint(v.z);
+    asm volatile("{\n\t.reg .b128 t;\n\tmov.b128 t, {%1, %2};\n\tst.relaxed.cta.shared.b128 [%0], t;\n\t}" ::"r"(
+                     (uint32_t)__cvta_generic_to_shared(p)),
+                 "l"(lo), "l"(hi)
                  : "memory");
 }
 
