@@ -3069,6 +3069,8 @@ static SolveArgs solveArgs(Context& c, vx_contact* cs, const IslandPlan& plan) {
     A.realIslands = plan.realIslands;
     A.tinyLimit = kTinyLimit;
     A.fault = &c.dCounters->planFault;
+    A.timeout = &c.dCounters->timeout;
+    A.waitLimit = c.waitLimit;
     A.prep = P<RowPrep>(c.prepBuf);
     A.planes = P<float4>(c.planeBuf);
     A.rows = plan.contacts;

@@ -96,6 +96,8 @@ struct SolveArgs {
     int stackStabilization;
     float stackStiffness, stackDamping;
     uint32_t* fault;         // set when the island plan is inconsistent (Counters::planFault)
+    uint32_t* timeout;       // set when a row's wait gave up (Counters::timeout)
+    uint32_t waitLimit;      // polls before it does (Context::waitLimit)
 };
 
 VXD bool solvedContact(uint32_t fa, uint32_t fb) { return !isSensor(fa) && !isSensor(fb); }
@@ -558,8 +560,6 @@ VXD void runColours(const SolveArgs& A, const RowPlanes& R, const BodyTable& T, 
 // 24 steps of 128 islands of 34 rows on four warps instead of one 27 -> 22 ms.
 // Batches of 8 or 4 rows were slower (7.2 and 12.6 ms for the 64: more batches
 // poll), as was sleeping between polls.
-constexpr uint32_t kTableWaitLimit = 1u << 22;  // polls of about 50 cycles
-
 // Whole 16-byte accesses: a vector access is four scalar ones in any order to
 // the memory model, a .b128 one is a single access, so a body's velocity
 // arrives with the tag that announces it.
@@ -615,8 +615,8 @@ VXD bool tableRow(const SolveArgs& A, const RowPlanes& R, const BodyTable& T, bo
             b.w = f3(tw);
         }
         if (__all_sync(0xffffffffu, ok)) break;
-        if (spins > kTableWaitLimit) {
-            atomicOr(A.fault, 1u);
+        if (spins > A.waitLimit) {
+            atomicOr(A.timeout, 1u);
             *dead = 1;
         }
         if ((spins & 63u) == 63u && __any_sync(0xffffffffu, *dead != 0)) return false;
@@ -818,7 +818,8 @@ __global__ void __launch_bounds__(ClassShape<Class>::kThreads, ClassShape<Class>
             // ranks of the rows on their bodies, colour by colour (a colour has one row a body)
             uint32_t* seen = reinterpret_cast<uint32_t*>(T.f);  // the frames come later
             for (uint32_t t = threadIdx.x; t < nb; t += Threads) seen[t] = 0u;
-            if (threadIdx.x == 0u) dead = 0;
+            // (a wait that gave up on another island ends this one's at once)
+            if (threadIdx.x == 0u) dead = *static_cast<volatile uint32_t*>(A.timeout) != 0u;
             for (uint32_t k = s0 + threadIdx.x; k < s1; k += Threads) {
                 const vx_contact& c = A.contacts[A.order[k]];
                 const bool solved = solvedContact(A.B.filt[c.a].x, A.B.filt[c.b].x);
