@@ -147,8 +147,8 @@ void vxb_context_destroy(vxb_context* ctx) {
                            &c.bodyValBuf, &c.islandBodyStartBuf, &c.caFlagBuf, &c.caBodyMarkBuf, &c.caCandBuf, &c.caSpecBuf,
                            &c.localIdxBuf, &c.prepBuf, &c.planeBuf, &c.frameBuf, &c.fpKeyBuf, &c.fpValBuf,
                            &c.fpSlotBuf, &c.fpColorBuf, &c.fpRunStartBuf, &c.fpIslandBuf, &c.coopBuf,
-                           &c.giantBuf, &c.classKeyBuf, &c.classValBuf, &c.flowBodyBuf, &c.tinyBuf, &c.tinyKeyBuf, &c.clusterInfoBuf, &c.clusterKeyBuf,
-                           &c.clusterValBuf, &c.clusterOfBuf, &c.clusterCountBuf, &c.clusterStartBuf,
+                           &c.giantBuf, &c.classKeyBuf, &c.classValBuf, &c.flowBodyBuf, &c.flowDegreeBuf, &c.tinyBuf, &c.tinyKeyBuf, &c.clusterInfoBuf, &c.clusterKeyBuf,
+                           &c.clusterValBuf, &c.clusterOfBuf, &c.flowColourBuf, &c.clusterStartBuf,
                            &c.clusterRowsBuf, &c.hardBuf, &c.caInfoBuf, &c.tuneSaveBuf,
                            &c.countersBuf};
     for (vxb::DevBuf* b : bufs)

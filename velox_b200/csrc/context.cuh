@@ -105,8 +105,7 @@ struct Counters {
     uint32_t clusterColours; // most colours of a giant island
     uint32_t giantCount;     // islands the block kernels cannot hold
     uint32_t caHard;         // pairs listed for the probe's warp queries
-    uint32_t flowTooWide;    // a body with more rows than a flow link counts
-    uint32_t pad[3];
+    uint32_t pad[4];
 };
 
 // Pipeline stages timed with CUDA events when timing is enabled.
@@ -232,10 +231,10 @@ struct Context {
     DevBuf coopBuf;                     // CoopState of cooperative launches
     DevBuf giantBuf;                    // giant island list (solve)
     DevBuf classKeyBuf, classValBuf;    // convex pairs grouped by shape combination (narrow phase)
-    DevBuf flowBodyBuf;                 // tagged body records (giant islands)
+    DevBuf flowBodyBuf, flowDegreeBuf;  // tagged body records, rows per body (giant islands)
     DevBuf tinyBuf;                     // tiny-island flags, ranks, list, pack counts/bases/firsts
     DevBuf tinyKeyBuf;                  // tiny islands' colour counts (pack order sort)
-    DevBuf clusterInfoBuf, clusterKeyBuf, clusterValBuf, clusterOfBuf, clusterCountBuf, clusterStartBuf,
+    DevBuf clusterInfoBuf, clusterKeyBuf, clusterValBuf, clusterOfBuf, flowColourBuf, clusterStartBuf,
         clusterRowsBuf;                 // spatial clusters of a giant island
     DevBuf hardBuf;                     // narrow phase: pairs for the warp queries
     DevBuf caInfoBuf;                   // rewind pass: one record per candidate

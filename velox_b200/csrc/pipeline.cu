@@ -1770,31 +1770,22 @@ constexpr uint32_t kNoPred = 0xffffffffu;  // empty queue slot / no successor
 // endpoints keyed n (no link).
 __global__ void giantEntryKernel(SolveArgs A, const uint32_t* islandOf, uint32_t m, uint32_t n, uint64_t* keys,
                                  uint32_t* vals);
-// For each body run of the sorted entries, its first entry and the one behind its last.
-__global__ void flowRunKernel(const uint64_t* keys, uint32_t entries, uint32_t n, uint2* runs, Counters* C) {
-    uint32_t most = 0;
+// For each body run of the sorted entries, its first entry.
+__global__ void flowRunKernel(const uint64_t* keys, uint32_t entries, uint32_t n, uint32_t* first) {
     for (uint32_t p = blockIdx.x * blockDim.x + threadIdx.x; p < entries; p += gridDim.x * blockDim.x) {
         const uint64_t key = keys[p];
-        if (key == (uint64_t)n) continue;
-        if (p == 0 || keys[p - 1] != key) runs[key].x = p;
-        if (p + 1 == entries || keys[p + 1] != key) runs[key].y = p + 1;
-        // longer runs than a link can count: some entry lies kMaxFlowDegree behind its run's start
-        if (p >= kMaxFlowDegree && keys[p - kMaxFlowDegree] == key) most = 1;
+        if (key != (uint64_t)n && (p == 0 || keys[p - 1] != key)) first[key] = p;
     }
-    if (most) atomicOr(&C->flowTooWide, 1u);
 }
-// link[2k + side]: the row's rank among its body's rows in colour order and
-// the body's row count; 0 without a dynamic body.
+// rank[2k + side]: the row's rank among its body's rows in colour order, 0
+// without a dynamic body; degree: the body's rows.
 __global__ void flowLinkKernel(const uint64_t* keys, const uint32_t* vals, uint32_t entries, uint32_t n,
-                               const uint2* runs, uint32_t* link) {
+                               const uint32_t* first, uint32_t* rank, uint32_t* degree) {
     for (uint32_t p = blockIdx.x * blockDim.x + threadIdx.x; p < entries; p += gridDim.x * blockDim.x) {
         const uint64_t key = keys[p];
-        uint32_t v = 0u;
-        if (key != (uint64_t)n) {
-            const uint2 r = runs[key];
-            v = (p - r.x) | (r.y - r.x) << 14;
-        }
-        link[vals[p]] = v;
+        const uint32_t v = key != (uint64_t)n ? p - first[key] : 0u;
+        rank[vals[p]] = v;
+        if (key != (uint64_t)n && (p + 1 == entries || keys[p + 1] != key)) degree[key] = v + 1u;
     }
 }
 
@@ -1844,34 +1835,36 @@ VXD uint32_t segmentOf(const uint32_t* segStart, uint32_t g0, uint32_t g1, uint3
     return lo;
 }
 
-// (warp, colour slot) cell of a giant row: the cluster of its first dynamic
-// body, colour within its island. Rows of the null island (no dynamic body of
-// their own island) have no links and go to any warp.
-VXD uint32_t rowCell(const SolveArgs& A, uint32_t k, const uint32_t* islandOf, const uint32_t* clusterOf,
-                     uint32_t clusters, uint32_t G) {
-    const uint32_t isl = islandOf[k];
-    const uint32_t g0 = A.islandSeg[isl], g1 = A.islandSeg[isl + 1];
-    uint32_t owner = k % clusters;
-    if (isl < A.realIslands) {
-        const vx_contact& c = A.contacts[A.order[k]];
-        owner = clusterOf[isDynamic(A.B.filt[c.a].x) ? c.a : c.b];
-    }
-    return owner * G + (segmentOf(A.segStart, g0, g1, k) - g0);
-}
-
-__global__ void clusterCountKernel(SolveArgs A, const uint32_t* rowList, uint32_t R, const uint32_t* islandOf,
-                                   const uint32_t* clusterOf, uint32_t clusters, uint32_t G, uint32_t* counts) {
-    for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < R; t += gridDim.x * blockDim.x)
-        atomicAdd(counts + rowCell(A, rowList[t], islandOf, clusterOf, clusters, G), 1u);
-}
-
-__global__ void clusterScatterKernel(SolveArgs A, const uint32_t* rowList, uint32_t R, const uint32_t* islandOf,
-                                     const uint32_t* clusterOf, uint32_t clusters, uint32_t G, const uint32_t* start,
-                                     uint32_t* fill, uint32_t* rows) {
+// Sort key of a giant row: its warp (the cluster of its first dynamic body),
+// then its colour within its island. Rows of the null island (no dynamic body
+// of their own island) have no links and go to any warp. Sorted rather than
+// counted into a table of warps x colours: a body of 20,000 rows has as many
+// colours, which made the table 0.6 GB.
+__global__ void flowKeyKernel(SolveArgs A, const uint32_t* rowList, uint32_t R, const uint32_t* islandOf,
+                              const uint32_t* clusterOf, uint32_t clusters, int colourBits, uint64_t* keys,
+                              uint32_t* rows) {
     for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < R; t += gridDim.x * blockDim.x) {
-        const uint32_t k = rowList[t];
-        const uint32_t cell = rowCell(A, k, islandOf, clusterOf, clusters, G);
-        rows[start[cell] + atomicAdd(fill + cell, 1u)] = k;
+        const uint32_t k = rowList[t], isl = islandOf[k];
+        const uint32_t g0 = A.islandSeg[isl], g1 = A.islandSeg[isl + 1];
+        uint32_t owner = k % clusters;
+        if (isl < A.realIslands) {
+            const vx_contact& c = A.contacts[A.order[k]];
+            owner = clusterOf[isDynamic(A.B.filt[c.a].x) ? c.a : c.b];
+        }
+        keys[t] = (uint64_t)owner << colourBits | (segmentOf(A.segStart, g0, g1, k) - g0);
+        rows[t] = k;
+    }
+}
+// Colour and warp ranges of the sorted rows.
+__global__ void flowStartKernel(const uint64_t* keys, uint32_t R, uint32_t clusters, int colourBits, uint32_t* colour,
+                                uint32_t* start) {
+    for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < R; t += gridDim.x * blockDim.x) {
+        const uint64_t key = keys[t];
+        colour[t] = (uint32_t)key & ((1u << colourBits) - 1u);
+        const uint32_t w = (uint32_t)(key >> colourBits);
+        for (uint32_t x = t ? (uint32_t)(keys[t - 1] >> colourBits) + 1u : 0u; x <= w; ++x) start[x] = t;
+        if (t + 1 == R)
+            for (uint32_t x = w + 1u; x <= clusters; ++x) start[x] = R;
     }
 }
 
@@ -3104,17 +3097,17 @@ static int buildFlow(Context& c, const SolveArgs& A, uint32_t clusters) {
     VXB_TRY(ensure(c, c.fpKeyBuf, (size_t)m * 16 + 64));
     VXB_TRY(ensure(c, c.fpValBuf, (size_t)m * 8 + 64));
     VXB_TRY(ensure(c, c.fpSlotBuf, (size_t)m * 8 + 64));
-    VXB_TRY(ensure(c, c.fpRunStartBuf, (size_t)n * 8 + 64));
+    VXB_TRY(ensure(c, c.fpRunStartBuf, (size_t)n * 4 + 64));
+    VXB_TRY(ensure(c, c.flowDegreeBuf, (size_t)n * 4 + 64));
     VXB_TRY(ensure(c, c.flowBodyBuf, (size_t)n * 64 + 64));
     uint64_t* keys = P<uint64_t>(c.fpKeyBuf);
     uint32_t* vals = P<uint32_t>(c.fpValBuf);
     const uint32_t* islandOf = P<uint32_t>(c.fpIslandBuf);
-    VXB_CUDA(c, cudaMemsetAsync(&c.dCounters->flowTooWide, 0, 4, c.stream));
     LAUNCH(c, giantEntryKernel, blocksFor(m, 256), 256, A, islandOf, m, n, keys, vals);
     VXB_TRY(sortPairs(c, keys, vals, 2 * m, bitsFor(n)));
-    LAUNCH(c, flowRunKernel, blocksFor(2 * m, 256), 256, keys, 2 * m, n, P<uint2>(c.fpRunStartBuf), c.dCounters);
+    LAUNCH(c, flowRunKernel, blocksFor(2 * m, 256), 256, keys, 2 * m, n, P<uint32_t>(c.fpRunStartBuf));
     LAUNCH(c, flowLinkKernel, blocksFor(2 * m, 256), 256, keys, vals, 2 * m, n,
-           (const uint2*)P<uint2>(c.fpRunStartBuf), P<uint32_t>(c.fpSlotBuf));
+           (const uint32_t*)P<uint32_t>(c.fpRunStartBuf), P<uint32_t>(c.fpSlotBuf), P<uint32_t>(c.flowDegreeBuf));
     VXB_TRY(ensure(c, c.clusterInfoBuf, ((size_t)n * 3 + (size_t)m * 3 + 128) * 4));
     uint32_t* bodyFlags = P<uint32_t>(c.clusterInfoBuf);
     uint32_t* bodyRank = bodyFlags + n + 16;
@@ -3135,7 +3128,7 @@ static int buildFlow(Context& c, const SolveArgs& A, uint32_t clusters) {
     c.clusterG = c.hostCounters.clusterColours;
     c.clusterCount = clusters;
     c.clusterBuilt = true;
-    const uint32_t nb = c.clusterNB, R = c.clusterR, G = c.clusterG, cells = clusters * G;
+    const uint32_t nb = c.clusterNB, R = c.clusterR, G = c.clusterG;
     if (nb == 0 || R == 0 || G == 0) {
         c.clusterR = 0;
         return VXB_OK;
@@ -3143,24 +3136,21 @@ static int buildFlow(Context& c, const SolveArgs& A, uint32_t clusters) {
     VXB_TRY(ensure(c, c.clusterKeyBuf, (size_t)nb * 8 + 64));
     VXB_TRY(ensure(c, c.clusterValBuf, (size_t)nb * 4 + 64));
     VXB_TRY(ensure(c, c.clusterOfBuf, (size_t)n * 4 + 64));
-    VXB_TRY(ensure(c, c.clusterCountBuf, (size_t)cells * 8 + 64));
-    VXB_TRY(ensure(c, c.clusterStartBuf, ((size_t)cells + 1) * 4 + 64));
+    VXB_TRY(ensure(c, c.flowColourBuf, (size_t)R * 4 + 64));
+    VXB_TRY(ensure(c, c.clusterStartBuf, ((size_t)clusters + 1) * 4 + 64));
     VXB_TRY(ensure(c, c.clusterRowsBuf, (size_t)R * 4 + 64));
-    uint32_t* counts = P<uint32_t>(c.clusterCountBuf);
-    uint32_t* fill = counts + cells;
-    uint32_t* start = P<uint32_t>(c.clusterStartBuf);
     const uint32_t* clusterOf = P<uint32_t>(c.clusterOfBuf);
     LAUNCH(c, clusterBodyKeyKernel, blocksFor(nb, 256), 256, A, (const uint32_t*)bodyPos, nb,
            (const Counters*)c.dCounters, P<uint64_t>(c.clusterKeyBuf), P<uint32_t>(c.clusterValBuf));
     VXB_TRY(sortPairs(c, P<uint64_t>(c.clusterKeyBuf), P<uint32_t>(c.clusterValBuf), nb, 30));
     LAUNCH(c, clusterOfBodyKernel, blocksFor(nb, 256), 256, (const uint32_t*)P<uint32_t>(c.clusterValBuf), nb, clusters,
            P<uint32_t>(c.clusterOfBuf));
-    VXB_CUDA(c, cudaMemsetAsync(counts, 0, (size_t)cells * 8, c.stream));
-    LAUNCH(c, clusterCountKernel, blocksFor(R, 256), 256, A, (const uint32_t*)rowList, R, islandOf, clusterOf, clusters,
-           G, counts);
-    VXB_TRY(exclusiveScan(c, counts, start, cells, start + cells));
-    LAUNCH(c, clusterScatterKernel, blocksFor(R, 256), 256, A, (const uint32_t*)rowList, R, islandOf, clusterOf,
-           clusters, G, (const uint32_t*)start, fill, P<uint32_t>(c.clusterRowsBuf));
+    const int colourBits = bitsFor(G - 1);
+    LAUNCH(c, flowKeyKernel, blocksFor(R, 256), 256, A, (const uint32_t*)rowList, R, islandOf, clusterOf, clusters,
+           colourBits, keys, P<uint32_t>(c.clusterRowsBuf));
+    VXB_TRY(sortPairs(c, keys, P<uint32_t>(c.clusterRowsBuf), R, colourBits + bitsFor(clusters - 1)));
+    LAUNCH(c, flowStartKernel, blocksFor(R, 256), 256, (const uint64_t*)keys, R, clusters, colourBits,
+           P<uint32_t>(c.flowColourBuf), P<uint32_t>(c.clusterStartBuf));
     return VXB_OK;
 }
 
@@ -3272,15 +3262,16 @@ static int launchSolve(Context& c, const SolveArgs& A) {
            &st->rounds);
     c.stats.giantIslands = std::max(c.stats.giantIslands, giants);
     if (clusters > 0) {
-        if (c.clusterR > 0 && !c.hostCounters.flowTooWide) {
+        if (c.clusterR > 0) {
             FlowArgs F;
             F.start = P<uint32_t>(c.clusterStartBuf);
             F.rows = P<uint32_t>(c.clusterRowsBuf);
-            F.link = P<uint32_t>(c.fpSlotBuf);
+            F.colour = P<uint32_t>(c.flowColourBuf);
+            F.rank = P<uint32_t>(c.fpSlotBuf);
+            F.degree = P<uint32_t>(c.flowDegreeBuf);
             F.bodyIds = P<uint32_t>(c.clusterValBuf);
             F.body = P<float4>(c.flowBodyBuf);
             F.bodies = c.clusterNB;
-            F.colours = c.clusterG;
             VXB_TRY(resetCoop(c, st));
             const int rcc = launchCooperativeSmem(c, perSm, 0, flow, kFlowThreads, A, F, st);
             if (rcc != VXB_ERR_UNSUPPORTED) {

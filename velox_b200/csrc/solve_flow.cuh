@@ -30,16 +30,17 @@ namespace vxb {
 
 constexpr int kFlowThreads = 128;
 constexpr int kFlowBlocksPerSm = 3;
-constexpr uint32_t kMaxFlowDegree = kRowLinkMask;  // rows of one body that a link counts
+constexpr uint32_t kLastColour = 65535;  // colours past it share a segment (the colour key's 16 bits)
 
 struct FlowArgs {
-    const uint32_t* start;    // first slot of each (warp, colour) cell
+    const uint32_t* start;    // first slot of each warp (warps + 1)
     const uint32_t* rows;     // slot -> solve position
-    const uint32_t* link;     // 2 per solve position: rank | degree << 14 on its bodies a and b (0: no link)
+    const uint32_t* colour;   // slot -> colour within its island
+    const uint32_t* rank;     // 2 per solve position: rank among the rows of its bodies a and b (0: no dynamic body)
+    const uint32_t* degree;   // body -> its rows
     const uint32_t* bodyIds;  // the islands' bodies
     float4* body;             // 4 per body: velocity | tag, angular velocity | tag, frame, inverse inertia | mass
     uint32_t bodies;
-    uint32_t colours;         // cells per warp
 };
 
 // The whole 16 bytes in one access, coherent over the GPU.
@@ -63,6 +64,7 @@ VXD void stRelaxed16(float4* p, const V3& v, uint32_t tag) {
 struct FlowRegs {
     RowRegs r;
     float4 frame, inertia;
+    uint32_t degree;
 };
 
 template <int Op>
@@ -78,7 +80,10 @@ VXD void loadFlowRegs(const RowPlanes& R, const FlowArgs& F, uint32_t slot, uint
         x.r.t2 = R.t2[slot];
         if (li >= 0) x.frame = __ldcg(F.body + 4 * (size_t)li + 2);
     }
-    if (li >= 0) x.inertia = __ldcg(F.body + 4 * (size_t)li + 3);
+    if (li >= 0) {
+        x.inertia = __ldcg(F.body + 4 * (size_t)li + 3);
+        x.degree = F.degree[li];
+    }
 }
 
 // Waits until every lane's body record carries the lane's tag; false when a
@@ -108,8 +113,7 @@ VXD bool flowRow(const SolveArgs& A, const FlowArgs& F, const RowPlanes& R, bool
     const uint32_t bits = __float_as_uint(r.i.w);
     act = act && (bits & kRowSolved);
     const int li = act ? __float_as_int(r.s.w) : kAtRest;
-    const uint32_t rank = (bits >> kRowLinkShift) & kRowLinkMask, degree = bits >> kRowDegreeShift;
-    const uint32_t tag = u * degree + rank;
+    const uint32_t tag = u * x.degree + (bits >> kRowLinkShift);
     float4* rec = F.body + 4 * (size_t)(li >= 0 ? li : 0);
     float4 tv = make_float4(0.0f, 0.0f, 0.0f, 0.0f), tw = tv;
     if (!awaitTags<Op != kRowPosition>(rec, li >= 0, tag, tv, tw, st)) return false;
@@ -190,6 +194,7 @@ VXD void runFlow(const SolveArgs& A, const FlowArgs& F, const RowPlanes& R, uint
     FlowRegs even, odd;  // the current and the next batch, in turn
     even.r.s = even.r.n = even.r.t1 = even.r.t2 = even.r.g = even.r.i = even.r.y = even.frame = even.inertia =
         make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    even.degree = 0u;
     odd = even;
     uint32_t i = s0, u = 0;
     if (i + pair < s1) loadFlowRegs<Op>(R, F, i + pair, side, even);
@@ -199,7 +204,8 @@ VXD void runFlow(const SolveArgs& A, const FlowArgs& F, const RowPlanes& R, uint
         const bool valid = i + pair < s1;
         const uint32_t colour = __float_as_uint(now.r.y.w);
         const uint32_t first = __shfl_sync(0xffffffffu, colour, 0);
-        const uint32_t count = (uint32_t)__popc(__ballot_sync(0xffffffffu, valid && colour == first)) >> 1;
+        uint32_t count = (uint32_t)__popc(__ballot_sync(0xffffffffu, valid && colour == first)) >> 1;
+        if (first == kLastColour) count = 1u;  // rows of this one may share a body: in order, one by one
         const bool wrap = i + count >= s1;
         const uint32_t ni = wrap ? s0 : i + count, nu = wrap ? u + 1u : u;
         if (nu < units && ni + pair < s1) loadFlowRegs<Op>(R, F, ni + pair, side, then);
@@ -241,18 +247,9 @@ __global__ void __launch_bounds__(kFlowThreads, kFlowBlocksPerSm) solveFlowKerne
                                                                                   CoopState* st) {
     const uint32_t tid = blockIdx.x * blockDim.x + threadIdx.x, stride = gridDim.x * blockDim.x;
     const uint32_t warp = tid >> 5, lane = threadIdx.x & 31u;
-    const uint32_t s0 = F.start[warp * F.colours], s1 = F.start[(warp + 1u) * F.colours];
+    const uint32_t s0 = F.start[warp], s1 = F.start[warp + 1u];
     const RowPlanes R = rowPlanes(A);
-    const uint32_t cell0 = warp * F.colours;
-    auto colourOf = [&](uint32_t slot) {  // last cell of the warp that starts at or before the slot
-        uint32_t lo = 0, hi = F.colours;
-        while (hi - lo > 1u) {
-            const uint32_t mid = (lo + hi) >> 1;
-            if (F.start[cell0 + mid] <= slot) lo = mid; else hi = mid;
-        }
-        return lo;
-    };
-    auto linkBits = [&](uint32_t k, uint32_t side) { return F.link[2 * (size_t)k + side] << kRowLinkShift; };
+    auto linkBits = [&](uint32_t k, uint32_t side) { return F.rank[2 * (size_t)k + side] << kRowLinkShift; };
     if (A.positionIterations > 0) {
         for (uint32_t t = tid; t < F.bodies; t += stride) {
             const uint32_t id = F.bodyIds[t];
@@ -275,7 +272,7 @@ __global__ void __launch_bounds__(kFlowThreads, kFlowBlocksPerSm) solveFlowKerne
             if (A.stackStabilization && lengthSq(f3(A.B.vel[c.a]) - f3(A.B.vel[c.b])) < 1e-4f)
                 resolve += 0.2f * (A.stackStiffness / 1000.0f) / (1.0f + A.stackDamping * A.h);
             R.g[slot] = make_float4(resolve, solverInvMass(ma) + solverInvMass(mb), 0.0f, 0.0f);
-            R.aux[slot] = make_float4(0.0f, 0.0f, 0.0f, __uint_as_float(colourOf(slot)));
+            R.aux[slot] = make_float4(0.0f, 0.0f, 0.0f, __uint_as_float(F.colour[slot]));
             const uint32_t solved = solvedContact(ma.flags, mb.flags) ? kRowSolved : 0u;
             R.imp[2 * (size_t)slot] =
                 make_float4(0.0f, 0.0f, 0.0f, __uint_as_float(solved | (isAsleep(ma.flags) ? kRowTurns : 0u) | linkBits(k, 0)));
@@ -345,7 +342,7 @@ __global__ void __launch_bounds__(kFlowThreads, kFlowBlocksPerSm) solveFlowKerne
             prepRow(a, b, rc, A.h, Cone, P);
             const bool solved = solvedContact(a.m.flags, b.m.flags);
             const uint32_t bits = storeRowPlanes<Cone>(R, slot, rc, P, solved, s);
-            R.aux[slot].w = __uint_as_float(colourOf(slot));
+            R.aux[slot].w = __uint_as_float(F.colour[slot]);
             R.side[2 * (size_t)slot] = pack(P.ra, __int_as_float(flowWord(A, c.a, a.m.flags, false)));
             R.side[2 * (size_t)slot + 1] = pack(P.rb, __int_as_float(flowWord(A, c.b, b.m.flags, false)));
             float4 imp = make_float4(rc.nImp, rc.t1Imp, rc.t2Imp, 0.0f);

@@ -171,8 +171,9 @@ struct ClassShape {
 // global memory in every sweep, 300 cycles on the step's critical path.
 constexpr int kPlaneWords = 13;
 constexpr uint32_t kRowExt = 1u, kRowSolved = 2u, kRowRecip = 4u;
-// Dataflow rows: the lane's body may turn; then the row's rank among its
-// body's rows and the body's row count, 14 bits each.
+// Dataflow rows: the lane's body may turn; above it the row's rank among its
+// body's rows, in a block 14 bits of it and 14 of the body's row count (at most
+// kMediumRows), in the grid's flow 28 bits (the count lies with the body).
 constexpr uint32_t kRowTurns = 8u, kRowLinkMask = 0x3fffu;
 constexpr int kRowLinkShift = 4, kRowDegreeShift = kRowLinkShift + 14;
 constexpr int kAtRest = INT_MIN;
