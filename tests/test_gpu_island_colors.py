@@ -1,6 +1,8 @@
 """Colouring of islands at the edges of their classes, bit for bit against the
 serial greedy rule in plain Python (src/backend_cuda.cu:603-630 of the
 reference): one thread, one warp, blocks of two sizes, the grid."""
+import time
+
 import numpy as np
 import pytest
 
@@ -66,3 +68,28 @@ def test_colors_equal_the_serial_rule(ctx, bodies, rows, hub, seed):
     want = greedy(contacts, body["motionType"] == 2, body["sensor"] != 0)
     assert np.array_equal(colors, want)
     assert count == want.max() + 1
+
+
+# Rows of one body: lists of up to 64 are sorted by a thread, longer ones picked
+# in order by a warp. One warp, both block sizes.
+@pytest.mark.parametrize("length", [64, 65, 250, 3000, 16384])
+def test_long_lists_keep_their_order(ctx, length):
+    rng = np.random.default_rng(length)
+    bodies = min(length // 2 + 2, 3000)
+    body = np.zeros(bodies, vb.BODY)
+    body["orientation"] = body["inertiaOrientation"] = (0, 0, 0, 1)
+    body["radius"], body["invMass"], body["motionType"] = 0.5, 1.0, 2
+    hub = bodies // 2  # the first end of some rows, the second of others
+    other = np.concatenate([np.delete(np.arange(bodies), hub), rng.integers(0, bodies, length)])
+    other = other[other != hub][:length]
+    contacts = np.zeros(len(other), vb.CONTACT)
+    contacts["a"], contacts["b"] = np.sort(np.stack([other, np.full(len(other), hub)], 1), axis=1).T
+    contacts = contacts[np.lexsort((contacts["b"], contacts["a"]))]
+    times = []
+    for _ in range(3):
+        start = time.perf_counter()
+        colors, count = ctx.color(body, contacts)
+        times.append(time.perf_counter() - start)
+    assert np.array_equal(colors, greedy(contacts, body["motionType"] == 2, body["sensor"] != 0))
+    assert count == len(other)
+    assert min(times) < 0.06  # 8 ms for the longest, 109 ms when its thread sorts it

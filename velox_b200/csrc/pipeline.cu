@@ -1123,6 +1123,10 @@ __global__ void colorFinishKernel(const uint32_t* order, uint32_t m, const uint3
 // 2,400 contacts, 3.2 -> 0.41 ms with one of 3,500, 2.7 -> 0.64 ms with one of
 // 10,500. Measured and not kept: block-wide rounds in which every waiting
 // contact bids on its bodies (2.2 ms for the 10,500, 1.1 ms for the 2,400).
+// A body's list is filled in any order and sorted by its thread while it is
+// short; sorting a hub's there took most of the call (call on an island of 4,000
+// rows of one body 31 ms, of 16,384 109 ms), so a warp picks a list of more than
+// 64 rows out of the island's rows in order (2.3 and 8.3 ms).
 template <int Class>
 struct ColorShape {
     static constexpr int kRows = ClassShape<Class>::kRows;
@@ -1139,6 +1143,7 @@ __global__ void __launch_bounds__(ClassShape<Class>::kThreads)
     constexpr int Threads = ClassShape<Class>::kThreads, kBodies = ColorShape<Class>::kBodies;
     constexpr int kRows = ColorShape<Class>::kRows;
     constexpr uint32_t kNone = 0xfffu, kPred = 1u << 24;
+    constexpr int kLongList = 64;
     extern __shared__ unsigned long long colorSmem[];
     unsigned long long* mask = colorSmem;
     uint32_t* next = reinterpret_cast<uint32_t*>(mask + kBodies);  // spill counter past 64 colours; entry counts first
@@ -1203,12 +1208,28 @@ __global__ void __launch_bounds__(ClassShape<Class>::kThreads)
         for (uint32_t t = threadIdx.x; t < nb; t += Threads) {
             // (nearly sorted: the threads took the rows in ascending batches)
             const int from = head[t], to = stop[t];
+            if (to - from > kLongList) continue;
             for (int x = from + 1; x < to; ++x) {
                 const uint16_t v = list[x];
                 int y = x - 1;
                 while (y >= from && list[y] > v) { list[y + 1] = list[y]; --y; }
                 list[y + 1] = v;
             }
+        }
+        for (uint32_t t = threadIdx.x >> 5; t < nb; t += Threads / 32) {  // a longer list: picked in order by a warp
+            uint32_t at = head[t];
+            if ((int)(stop[t] - at) <= kLongList) continue;
+            for (uint32_t r0 = 0; r0 < count; r0 += 32u) {
+                const uint32_t word = r0 + lane < count ? rows[r0 + lane] : 0xffffffu;
+                const bool mine = (word & 0xfffu) == t || ((word >> 12) & 0xfffu) == t;
+                const unsigned m = __ballot_sync(0xffffffffu, mine);
+                if (mine) list[at + __popc(m & laneMaskLt())] = (uint16_t)(r0 + lane);
+                at += __popc(m);
+            }
+        }
+        islandBarrier<Threads>();
+        for (uint32_t t = threadIdx.x; t < nb; t += Threads) {
+            const int from = head[t], to = stop[t];
             for (int x = from + 1; x < to; ++x) atomicAdd(rows + list[x], kPred);
             next[t] = 64u;
         }
