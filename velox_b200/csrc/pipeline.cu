@@ -2670,6 +2670,12 @@ int loadBodies(Context& c, const vx_body* bodies, uint32_t n, const uint32_t* wo
                       &c.sortKeysAlt})
         VXB_TRY(ensure(c, *b, mcap * 8 + 64));
     VXB_TRY(ensure(c, c.sortValsAlt, std::max<size_t>(mcap, (size_t)c.pairCap) * 4 + 64));
+    // The rows' planes and the listed pairs, two a body: grown with the contacts
+    // of a world's first steps, they were freed and allocated a dozen times each
+    // (solve stage of steps 6 to 25 of 4,096 worlds 15.3 -> 9.7 ms; a free now and
+    // then takes tens of ms more).
+    VXB_TRY(ensure(c, c.planeBuf, ((size_t)2 * n + 4096) * kRowPlaneBytes + 256));
+    VXB_TRY(ensure(c, c.hardBuf, ((size_t)2 * n + 4096) * (4 + sizeof(HardResult)) + 64));
     c.prevCount = 0;
     c.stepContacts = 0;
     VXB_TRY(sleepLoad(c, bodies, n));
@@ -3085,10 +3091,8 @@ static SolveArgs solveArgs(Context& c, vx_contact* cs, const IslandPlan& plan) {
     A.fault = &c.dCounters->planFault;
     A.timeout = &c.dCounters->timeout;
     A.waitLimit = c.waitLimit;
-    A.prep = P<RowPrep>(c.prepBuf);
     A.planes = P<float4>(c.planeBuf);
     A.rows = plan.contacts;
-    A.frames = P<float4>(c.frameBuf);
     return A;
 }
 
@@ -3304,21 +3308,19 @@ static int launchSolve(Context& c, const SolveArgs& A) {
         }
     }
     // no cooperative grid (or no solvable giant rows): one block per giant island
-    LAUNCH(c, solveGiantBlockKernel, giants, kGiantBlockThreads, A, (const uint32_t*)list);
+    SolveArgs G = A;
+    VXB_TRY(ensure(c, c.prepBuf, (size_t)A.rows * sizeof(RowPrep) + 256));
+    VXB_TRY(ensure(c, c.frameBuf, (size_t)c.n * 16 + 256));
+    G.prep = P<RowPrep>(c.prepBuf);
+    G.frames = P<float4>(c.frameBuf);
+    LAUNCH(c, solveGiantBlockKernel, giants, kGiantBlockThreads, G, (const uint32_t*)list);
     return VXB_OK;
 }
 
 // Substep loop over islands + contact-free bodies (advanceSubsteps).
-static int solveBuffers(Context& c, uint32_t m) {
-    VXB_TRY(ensure(c, c.prepBuf, (size_t)m * sizeof(RowPrep) + 256));
-    VXB_TRY(ensure(c, c.planeBuf, (size_t)m * kPlaneWords * sizeof(float4) + 256));
-    VXB_TRY(ensure(c, c.frameBuf, (size_t)c.n * 16 + 256));
-    return VXB_OK;
-}
-
 static int runSubsteps(Context& c, vx_contact* cs, const IslandPlan& plan, const V3& g, float h, int substeps,
                        const vx_solver_options& o, bool warmStart, bool integrate) {
-    VXB_TRY(solveBuffers(c, plan.contacts + 1));
+    VXB_TRY(ensure(c, c.planeBuf, ((size_t)plan.contacts + 1) * kRowPlaneBytes + 256));
     SolveArgs A = solveArgs(c, cs, plan);
     A.gravity = g;
     A.h = h;

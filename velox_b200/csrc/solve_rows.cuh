@@ -90,9 +90,9 @@ struct SolveArgs {
     uint32_t tinyLimit;
     int positionIterations;  // position-correction mode when > 0
     RowPrep* prep;           // per solve-order row, rebuilt every substep (giant islands without a cooperative grid)
+    float4* frames;          // per body inertia frame, rebuilt every substep (the same)
     float4* planes;          // per row terms of the block solve and the grid's flow (RowPlanes)
     uint32_t rows;           // rows of the plan (the planes' stride)
-    float4* frames;          // per body inertia frame, rebuilt every substep (global path)
     int stackStabilization;
     float stackStiffness, stackDamping;
     uint32_t* fault;         // set when the island plan is inconsistent (Counters::planFault)
@@ -169,7 +169,7 @@ struct ClassShape {
 // for a body outside it (never moved here) kAtRest when its velocities are
 // zero, else the complement of its id: a body that is not at rest is read from
 // global memory in every sweep, 300 cycles on the step's critical path.
-constexpr int kPlaneWords = 13;
+constexpr size_t kRowPlaneBytes = 13 * sizeof(float4);
 constexpr uint32_t kRowExt = 1u, kRowSolved = 2u, kRowRecip = 4u;
 // Dataflow rows: the lane's body may turn; above it the row's rank among its
 // body's rows, in a block 14 bits of it and 14 of the body's row count (at most
