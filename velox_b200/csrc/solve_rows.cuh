@@ -280,7 +280,7 @@ VXD bool quotientRange(float x) {
 VXD bool quotientBase(float k) { return k >= 9.5e-10f && k <= 1.0e9f; }
 
 VXD float axisShare(float n, float mx) {  // (a zero numerator would cost the slow division)
-    return mx <= 0.0f || (n == 0.0f && mx > 1e-10f) ? 0.0f : n * n / (mx * mx);
+    return !(mx > 0.0f) || (n == 0.0f && mx > 1e-10f) ? 0.0f : n * n / (mx * mx);
 }
 // Both lanes hold the same impulses; each divides one axis (all 32 lanes call).
 VXD void clampToEllipse(uint32_t side, float max1, float max2, float& n1, float& n2) {
