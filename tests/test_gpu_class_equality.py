@@ -85,3 +85,27 @@ def test_classes_agree(ctx, mode, friction):
         for name in ("normalImpulse", "tangentImpulse1", "tangentImpulse2", "rollingImpulse1", "rollingImpulse2",
                      "spinningImpulse"):
             assert np.array_equal(bits(real[name]), bits(rows[name])), (idle, name)
+
+
+# A body that the velocity solve drives to infinity: the position correction
+# passes its gap on in every class alike.
+def test_not_a_number_spreads_alike(ctx):
+    masks = []
+    for n in (40, 200, 700):
+        s = np.zeros(n + 1, vb.binding.SPEC)
+        s["orientation"] = (0, 0, 0, 1)
+        s["shape"][n], s["planeNormal"][n] = 1, (0, 1, 0)  # last: contacts are written back with a < b
+        s["mass"][:n], s["radius"][:n] = 1.0, 0.5
+        s["position"][:n, 0], s["position"][:n, 1] = np.arange(n) * 0.995, 0.498
+        bodies, hull, faces = vb.bodies_from_specs(s, np.zeros((0, 3), np.float32))
+        ctx.load(bodies, vb.make_soup(hull, faces))
+        ctx.configure(dt=4 * H, substeps=4)
+        ctx.step(1)
+        contacts = ctx.read_contacts()
+        contacts["normalImpulse"][(contacts["a"] == 20) & (contacts["b"] == 21)] = np.inf
+        ctx.write_contacts(contacts)
+        ctx.step(1)
+        assert (ctx.stats()["giantIslands"] == 1) == (n == 700)
+        masks.append(np.isfinite(ctx.read_bodies()["position"]).all(axis=1)[:35])
+    assert not masks[0].all() and masks[0].any()
+    assert np.array_equal(masks[0], masks[1]) and np.array_equal(masks[0], masks[2])

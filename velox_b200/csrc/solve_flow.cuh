@@ -125,7 +125,8 @@ VXD bool flowRow(const SolveArgs& A, const FlowArgs& F, const RowPlanes& R, bool
         pairBoth(p + arm, side, wa, wb);
         const float gap = r.n.w + dot(n, wa - wb);
         if (act && li >= 0) {
-            if (r.g.y > 0.0f && gap < -1e-3f && !(bits & kRowTurns)) {  // (kRowTurns: asleep, in this mode)
+            // (as laneRow's step, a gap that is not a number included; kRowTurns: asleep, in this mode)
+            if (!(r.g.y <= 0.0f) && !(gap >= -1e-3f) && !(bits & kRowTurns)) {
                 const float push = -r.g.x * (gap + 1e-3f) / r.g.y;
                 const V3 d = n * (push * x.inertia.w);
                 p = side ? p - d : p + d;
