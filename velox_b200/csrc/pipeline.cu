@@ -1709,8 +1709,9 @@ VXD void solveTinyPack(const SolveArgs& A, const uint32_t* list, const uint32_t*
         idb = cp->b;
         const uint32_t fa = A.B.filt[ida].x, fb = A.B.filt[idb].x;
         live = solvedContact(fa, fb);
-        if (isDynamic(fa)) la = (int)localIdx[ida];
-        if (isDynamic(fb)) lb = (int)localIdx[idb];
+        // (a sensor's row lies in the null island, which owns no bodies)
+        if (live && isDynamic(fa)) la = (int)localIdx[ida];
+        if (live && isDynamic(fb)) lb = (int)localIdx[idb];
         // a dynamic body outside its island's slots means an inconsistent plan: report it, never index smem
         if (la >= 0 && ((uint32_t)la < myBase || (uint32_t)la >= myBase + myNb || ids[la] != ida)) {
             atomicOr(A.fault, 1u);
