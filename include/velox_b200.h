@@ -310,7 +310,15 @@ int vxb_world_snapshot_write(vxb_context* ctx, const void* in, uint64_t size);
  * vxb_world_step for those steps (they are recorded: contacts after matching,
  * body checkpoints every k steps), then vxb_adjoint_backward. The backward
  * pass recomputes each k-step segment from its checkpoint (bit-identical to
- * the forward) and runs the reverse; one warp per world. */
+ * the forward) and runs the reverse; one warp per world.
+ *
+ * Device memory: beside the recorded steps, a backward pass takes up to 4 GiB
+ * of scratch as long as that leaves as much free (else one step's worth per
+ * world, and a third more work). When another load or tape ends the tape, up
+ * to 6 GiB, and no more than is free beside it, stay for the next one; they go
+ * back when this context runs short, with a load after a world that was not
+ * taped, and with vxb_tape_end, which gives everything back at once: call it
+ * before other code needs the memory. */
 
 /* Per-world flags of a tape / backward pass. */
 #define VXB_ADJ_REWOUND 1u     /* a conservative-advancement rewind moved a body: not smooth */
@@ -352,7 +360,7 @@ int vxb_adjoint_backward(vxb_context* ctx, const float* seed, float* grad, float
 int vxb_adjoint_backward_branches(vxb_context* ctx, const float* seed, float* grad, float* gradInverseMass,
                                   float* gradMass, uint32_t* worldFlags, uint8_t* branches, size_t capacity,
                                   size_t* branchBytes, uint32_t* branchRows);
-/* Releases the tape. */
+/* Releases the tape and all memory that this or an earlier tape kept. */
 int vxb_tape_end(vxb_context* ctx);
 
 /* ---- individual stages (parity testing) --------------------------------- */

@@ -73,17 +73,37 @@ constexpr uint32_t kNoColour = 0x7fffffffu;
 // it the segment runs forward once without a tape and each step again with one:
 // a third more row updates (backward pass of 128 rollouts of 24 steps 126 against
 // 186 ms, of 1,024 of 10 steps 65 against 98, both with the rows' state in global
-// memory).
+// memory). The scratch grows for it only while it leaves as much device memory
+// free as it takes: other contexts and allocators share the device.
 constexpr size_t kSegmentTapeLimit = (size_t)4 << 30;
-// Memory an ended tape may hold for the next one (the scratch above with the
-// allocator's half on top). Freeing and allocating it for each pass of a loop
-// over load, tape and backward took 0 to 50 of 200 ms, now and then a second
-// (128 rollouts of 24 steps).
+// Memory an ended tape may hold for the next one, and no more than is free
+// beside it. Freeing and allocating it for each pass of a loop over load, tape
+// and backward took 0 to 50 of 200 ms, now and then a second (128 rollouts of 24
+// steps).
 constexpr size_t kTapeKeepLimit = (size_t)6 << 30;
 
 inline uint32_t gridFor(uint64_t items, int threads) {
     uint64_t b = (items + threads - 1) / threads;
     return (uint32_t)std::max<uint64_t>(1, std::min<uint64_t>(b, 65535u * 16u));
+}
+
+// ensure() of the bytes alone, without room to grow.
+int ensureExact(Context& c, DevBuf& b, size_t bytes) {
+    if (bytes <= b.bytes && b.ptr) return VXB_OK;
+    if (b.ptr) cudaFree(b.ptr);
+    b = DevBuf{};
+    AD_TRY(allocate(c, b, &b.ptr, bytes));
+    b.bytes = bytes;
+    return VXB_OK;
+}
+
+size_t freeBytes() {
+    size_t free = 0, total = 0;
+    if (cudaMemGetInfo(&free, &total) != cudaSuccess) {
+        cudaGetLastError();
+        return 0;
+    }
+    return free;
 }
 
 // Grow-only allocation that keeps the first `keep` bytes.
@@ -1241,7 +1261,7 @@ int tapeBegin(Context& c, uint32_t steps, uint32_t every) {
     return VXB_OK;
 }
 
-// keep: the buffers stay up to kTapeKeepLimit in sum. A load after a world that
+// keep: the buffers stay up to kTapeKeepLimit and the free memory in sum. A load after a world that
 // was never taped keeps none, so a program that stops taping gets the memory back.
 int tapeEnd(Context& c, bool keep) {
     Tape& T = c.tape;
@@ -1250,9 +1270,10 @@ int tapeEnd(Context& c, bool keep) {
     T.stepStart.assign(1, 0u);
     if (T.contacts.ptr || T.ckpt.ptr || T.scratch.ptr || T.branches.ptr) cudaStreamSynchronize(c.stream);
     size_t held = 0;
+    const size_t limit = keep ? std::min(kTapeKeepLimit, freeBytes()) : 0;
     for (DevBuf* b : {&T.scratch, &T.contacts, &T.src, &T.color, &T.worldStart, &T.ckpt, &T.flags, &T.host,
                       &T.branches}) {
-        if (keep && held + b->bytes <= kTapeKeepLimit) {
+        if (keep && held + b->bytes <= limit) {
             held += b->bytes;
             continue;
         }
@@ -1407,13 +1428,15 @@ int adjointBackward(Context& c, const float* seed, float* grad, float* gradInv, 
     A.hotShared = A.hotBytes * std::min<uint32_t>(perSm, kAdjointWarpsPerSm) <= kAdjointShared &&
                   A.hotBytes * perBlock(worlds) <= kAdjointShared;
     // every step's tape at once, or one segment's, or one step's
+    auto tapes = [&](size_t bytes) {
+        if (bytes > kSegmentTapeLimit) return false;
+        if (bytes > T.scratch.bytes && bytes > (freeBytes() + T.scratch.bytes) / 2) return false;
+        return ensureExact(c, T.scratch, bytes) == VXB_OK;
+    };
     const size_t wholeExtra = al((size_t)steps * 4 * NBs * 16) - tape0 + A.tapeBytes * (steps - 1);
     const bool whole = A.J > 1 && A.hotShared && A.hotBytes * perBlock(segments) <= kAdjointShared &&
-                       perSm < kAdjointWarpsPerSm &&
-                       (afterTape + wholeExtra + rest) * worlds <= kSegmentTapeLimit &&
-                       ensure(c, T.scratch, (afterTape + wholeExtra + rest) * worlds) == VXB_OK;
-    A.segmentTape = whole || ((afterTape + segmentExtra + rest) * worlds <= kSegmentTapeLimit &&
-                              ensure(c, T.scratch, (afterTape + segmentExtra + rest) * worlds) == VXB_OK);
+                       perSm < kAdjointWarpsPerSm && tapes((afterTape + wholeExtra + rest) * worlds);
+    A.segmentTape = whole || tapes((afterTape + segmentExtra + rest) * worlds);
     if (whole) {
         const size_t states = al((size_t)steps * 4 * NBs * 16) - tape0;
         for (size_t* off : {&A.oSub, &A.oEnd, &A.oCorr, &A.oRin, &A.oPush, &A.oLamInit}) *off += states;
@@ -1421,7 +1444,7 @@ int adjointBackward(Context& c, const float* seed, float* grad, float* gradInv, 
     if (A.segmentTape) afterTape += whole ? wholeExtra : segmentExtra;
     A.hotOffset = afterTape;
     A.worldBytes = afterTape + rest;
-    if (!A.segmentTape) AD_TRY(ensure(c, T.scratch, A.worldBytes * worlds));
+    if (!A.segmentTape) AD_TRY(ensureExact(c, T.scratch, A.worldBytes * worlds));
     A.scratch = PT<char>(T.scratch);
     auto launch = [&](auto* kernel, uint32_t warps) {
         const uint32_t block = perBlock(warps);
