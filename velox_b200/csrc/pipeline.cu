@@ -1063,17 +1063,18 @@ __global__ void colorSlotKernel(const uint64_t* keys, const uint32_t* vals, uint
 
 // Cooperative launch. changed[3] rotate per round: the counter of round r + 1
 // is cleared during round r, after every block has read round r - 2's value.
-// color[] is indexed by island-order position and zero on entry.
+// color[] is indexed by island-order position and zero on entry; contacts of
+// other islands have no slots and so keep their zero (looking their class up
+// in every round: islands stage 4.17 / 4.05 ms with one island of 25,000
+// contacts).
 __global__ void colorFixedPointKernel(const uint64_t* keys, const uint32_t* vals, const uint32_t* slot,
-                                      const uint32_t* runStart, const uint32_t* islandIdx,
-                                      const uint32_t* islandStart, const uint32_t* bodyStart, uint32_t realIslands,
-                                      uint32_t m, uint32_t* color, CoopState* st, uint32_t maxRounds) {
+                                      const uint32_t* runStart, uint32_t m, uint32_t* color, CoopState* st,
+                                      uint32_t maxRounds) {
     const uint32_t tid = blockIdx.x * blockDim.x + threadIdx.x, stride = gridDim.x * blockDim.x;
     for (uint32_t r = 0; r < maxRounds; ++r) {
         if (tid == 0) st->changed[(r + 1) % 3] = 0u;
         uint32_t local = 0;
         for (uint32_t k = tid; k < m; k += stride) {
-            if (planClass(islandStart, bodyStart, realIslands, islandIdx[k]) != kGiantIsland) continue;
             // Past 64 colours the greedy rule continues from a per-body
             // counter: one past the highest colour (>= 64) of the body's
             // earlier contacts, 64 when there is none.
@@ -2974,8 +2975,7 @@ static int parallelColor(Context& c, const vx_contact* cs, const uint32_t* order
     VXB_CUDA(c, cudaMemsetAsync(color, 0, (size_t)m * 4, c.stream));
     VXB_TRY(resetCoop(c, st));
     const int rc = launchCooperative(c, colorFixedPointKernel, 256, (const uint64_t*)keys, (const uint32_t*)vals,
-                                     (const uint32_t*)slot, (const uint32_t*)runStart, islandIdx,
-                                     islandStart, bodyStart, realIslands, m, color, st, 4096u);
+                                     (const uint32_t*)slot, (const uint32_t*)runStart, m, color, st, 4096u);
     if (rc != VXB_OK) return rc;
     CoopState host;
     VXB_CUDA(c, cudaMemcpyAsync(&host, st, sizeof(host), cudaMemcpyDeviceToHost, c.stream));
