@@ -92,3 +92,29 @@ def test_general_pairs_run_a_thread_each(quality):
     c.close()
     print("narrow phase, quality", quality, len(pairs), "pairs:", classified, "against", threads, "ms")
     assert classified < 1.4 * threads
+
+
+# Compounds: many child pairs, most of them apart. A warp a pair took three
+# times the thread's time.
+def test_compounds_run_a_thread_each():
+    bodies, soup = world(12000, (0,))
+    dyn = np.flatnonzero(bodies["motionType"] == 2)
+    bodies["shape"][dyn], bodies["compoundFirst"][dyn], bodies["compoundCount"][dyn] = vb.binding.SHAPE["compound"], 0, 2
+    bodies["radius"][dyn] = 0.8
+    c = vb.Context(0)
+    pairs = c.pairs(bodies, DT, soup)
+    c.enable_timing(True)
+
+    def stage(call):
+        times = []
+        for _ in range(4):
+            before = c.stage_times()["narrowphase"][0]
+            call()
+            times.append(c.stage_times()["narrowphase"][0] - before)
+        return min(times)
+
+    classified = stage(lambda: c.backend_find_contacts(bodies, soup, DT))
+    threads = stage(lambda: c.collide(bodies, soup, pairs, DT))
+    c.close()
+    print("narrow phase of compounds,", len(pairs), "pairs:", classified, "against", threads, "ms")
+    assert classified < 1.4 * threads

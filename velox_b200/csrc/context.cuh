@@ -180,7 +180,7 @@ struct Context {
     DevBuf vertBuf, indexBuf, meshBuf, nodeBuf, triRefBuf, childBuf;
     DevBuf jointBuf;  // joints of the Backend path, in colour order
     std::vector<vx_mesh> hostMeshes;   // root bounds for the broad phase
-    bool generalShapes = false;        // any Robust or Paranoid body loaded (threadPair)
+    bool threadShapes = false;         // any Robust, Paranoid or compound body loaded (threadPair)
     bool kinematic = false;            // any kinematic body loaded (Backend path)
     // FNV-1a keys of the loaded bodies' shape references and of the soup's
     // array sizes (a snapshot image restores only into the same geometry)

@@ -510,21 +510,25 @@ VXD bool pointLess(const vx_contact& x, const vx_contact& y) {
 // pairs are listed in `hard` for collideHardKernel: a thread's EPA runs up to
 // 1 ms, and one such lane held its warp and the stage's tail for that long.
 // Listed pairs: the contacts of those pairs from the query results that
-// collideHardKernel left (face clipping fills a warp's lanes again). General
-// pairs: the listed ones of Robust and Paranoid bodies (threadPair), whose
-// routine is serial: one thread each, from query to contacts (launched only
-// when such bodies are loaded; heap of 10,000 of them, narrow phase of one step
-// as one lane of a warp each / here: Robust 11.5 / 7.7 ms, Paranoid 22.6 / 10.9).
-enum PairClass : int { kAnyPairs = 0, kPlanePairs = 1, kConvexPairs = 2, kListedPairs = 3, kGeneralPairs = 4 };
+// collideHardKernel left (face clipping fills a warp's lanes again). Thread
+// pairs: the listed ones that a warp would waste (threadPair), one thread each
+// from query to contacts (launched only when such bodies are loaded). Narrow phase
+// of one step, a warp / a thread a pair: heap of 10,000 Robust bodies 11.5 / 7.7
+// ms, Paranoid 22.6 / 10.9; heap of 30,000 compounds 14.4 / 4.0.
+enum PairClass : int { kAnyPairs = 0, kPlanePairs = 1, kConvexPairs = 2, kListedPairs = 3, kThreadPairs = 4 };
 
-// Listed pairs that the warps' query would run on one lane throughout (mesh
-// pairs share the triangles among the lanes all the same), where the list is
-// longer than a few rounds of the GPU's resident warps; of a shorter one a warp's
-// lone lane is faster than 32 that diverge (rewind stage with some 1,000 such
-// pairs probed 14.2 / 18.7 ms, narrow phase of 2,800 21 / 26 ms).
+// Listed pairs whose queries use a warp badly: Robust and Paranoid bodies (the
+// general routine runs on one lane) and compounds (many child pairs, most of them
+// apart, which all lanes follow alike); mesh pairs share the triangles among the
+// lanes all the same. Where the list is longer than a few rounds of the GPU's
+// resident warps they go to threads; of a shorter one a warp each is faster than
+// 32 lanes that diverge (rewind stage with some 1,000 Paranoid pairs probed 14.2
+// / 18.7 ms, narrow phase of 2,800 21 / 26 ms).
 constexpr uint32_t kLoneLaneMax = 4096;
 VXD bool threadPair(uint32_t listed, uint32_t flagsA, uint32_t flagsB) {
-    return listed > kLoneLaneMax && ((flagsA | flagsB) >> kGeomQualityShift & 3u) != 0u && shapeOf(flagsA) != kMesh && shapeOf(flagsB) != kMesh;
+    const uint32_t sa = shapeOf(flagsA), sb = shapeOf(flagsB);
+    return listed > kLoneLaneMax && sa != kMesh && sb != kMesh &&
+           (((flagsA | flagsB) >> kGeomQualityShift & 3u) != 0u || sa == kCompound || sb == kCompound);
 }
 
 // Result of one listed pair's query.
@@ -574,7 +578,7 @@ __global__ void __launch_bounds__(128) collideKernel(BodyArrays B, Soup soup, co
                                                      uint32_t recCap, uint32_t* hard, const HardResult* results,
                                                      Counters* C) {
     const uint32_t stride = gridDim.x * blockDim.x;
-    if (Class == kListedPairs || Class == kGeneralPairs) npairs = C->hardPairs;
+    if (Class == kListedPairs || Class == kThreadPairs) npairs = C->hardPairs;
     const uint32_t rounded = (npairs + 31u) & ~31u;
     for (uint32_t base = blockIdx.x * blockDim.x; base < rounded; base += stride) {
         const uint32_t slot = base + threadIdx.x;
@@ -592,7 +596,7 @@ __global__ void __launch_bounds__(128) collideKernel(BodyArrays B, Soup soup, co
             } else if (Class == kPlanePairs) {
                 if (shapeOf(b.flags) == kPlane) planeConvex(a, b, i, j, soup, dt, buf, kMaxContactsPerPair, count);
                 else planeConvex(b, a, j, i, soup, dt, buf, kMaxContactsPerPair, count);
-            } else if (Class == kGeneralPairs) {
+            } else if (Class == kThreadPairs) {
                 if (threadPair(npairs, a.flags, b.flags)) count = collidePair(a, b, i, j, soup, dt, buf, kMaxContactsPerPair);
             } else if (isComplexShape(shapeOf(a.flags)) || isComplexShape(shapeOf(b.flags)) ||
                        (Class == kListedPairs && threadPair(npairs, a.flags, b.flags))) {
@@ -667,7 +671,7 @@ __global__ void __launch_bounds__(kQueryThreads) collideHardKernel(BodyArrays B,
         const uint64_t pr = pairs[p];
         const uint32_t i = (uint32_t)(pr >> 32), j = (uint32_t)pr;
         const BodyView a = loadView(B, i), b = loadView(B, j);
-        if (threadPair(count, a.flags, b.flags)) continue;  // collideKernel<kGeneralPairs>
+        if (threadPair(count, a.flags, b.flags)) continue;  // collideKernel<kThreadPairs>
         if (!isComplexShape(shapeOf(a.flags)) && !isComplexShape(shapeOf(b.flags))) {
             const GjkResult r = gjkDistanceWarp(makeConvex(a, soup), makeConvex(b, soup));
             if (warpLane() == 0u) results[k] = HardResult{r.distance, r.normal, r.pointA, r.pointB};
@@ -2623,7 +2627,7 @@ int loadBodies(Context& c, const vx_body* bodies, uint32_t n, const uint32_t* wo
         c.backendContacts = 0;
         c.backendColored = false;
     }
-    bool general = false;
+    bool threads = false;
     c.kinematic = false;
     uint64_t key = 0xcbf29ce484222325ull;
     for (uint32_t i = 0; i < n; ++i) {
@@ -2635,14 +2639,14 @@ int loadBodies(Context& c, const vx_body* bodies, uint32_t n, const uint32_t* wo
     c.bodyGeometryKey = key;
     for (uint32_t i = 0; i < n; ++i) {
         const uint8_t s = bodies[i].shape;
-        if (bodies[i].geometryQuality & 3u) general = true;
+        if ((bodies[i].geometryQuality & 3u) || s == VX_SHAPE_COMPOUND) threads = true;
         if (s == VX_SHAPE_MESH && bodies[i].motionType != VX_MOTION_STATIC)
             return fail(c, VXB_ERR_INVALID, "mesh bodies are static");
         if (deviceWorld && bodies[i].motionType == VX_MOTION_KINEMATIC)
             return fail(c, VXB_ERR_UNSUPPORTED, "kinematic bodies are not supported by the device world");
         if (bodies[i].motionType == VX_MOTION_KINEMATIC) c.kinematic = true;
     }
-    c.generalShapes = general;
+    c.threadShapes = threads;
     c.n = n;
     // SoA arrays in one allocation (16 arrays of 16-byte elements).
     const size_t stride = ((size_t)n * 16 + 255) & ~(size_t)255;
@@ -2875,8 +2879,8 @@ static int narrowPhase(Context& c, const uint64_t* pairs, uint32_t npairs, float
                        soupOf(c), pairs, (const uint32_t*)hard, convexSplit, dt, mode, bodyBits, tmp, c.contactCap,
                        recKeys, recVals, recInfo, c.recCap, (uint32_t*)nullptr, (const HardResult*)results,
                        c.dCounters);
-                if (c.generalShapes)
-                    LAUNCH(c, collideKernel<kGeneralPairs>, blocksFor(convexSplit, 64, (uint32_t)c.smCount * 16), 64,
+                if (c.threadShapes)
+                    LAUNCH(c, collideKernel<kThreadPairs>, blocksFor(convexSplit, 64, (uint32_t)c.smCount * 16), 64,
                            c.B, soupOf(c), pairs, (const uint32_t*)hard, convexSplit, dt, mode, bodyBits, tmp,
                            c.contactCap, recKeys, recVals, recInfo, c.recCap, (uint32_t*)nullptr,
                            (const HardResult*)nullptr, c.dCounters);
@@ -3436,7 +3440,7 @@ static int conservativeAdvancement(Context& c, uint32_t npairs, float dt) {
         LAUNCH(c, caProbeKernel, sh.grid(npairs, c.smCount), sh.threads, c.B, soupOf(c), pk, probeOrder, npairs,
                flags, bodyMark, endGap, hard, c.dCounters);
     }, emptyList));
-    if (c.generalShapes)
+    if (c.threadShapes)
         LAUNCH(c, caProbeGeneralKernel, blocksFor(npairs, 64, (uint32_t)c.smCount * 16), 64, c.B, soupOf(c), pk,
                (const uint32_t*)hard, flags, bodyMark, endGap, (const Counters*)c.dCounters);
     VXB_TRY(launchQueries(c, npairs, caProbeHardKernel, c.B, soupOf(c), pk, (const uint32_t*)hard, dt, flags, bodyMark,

@@ -27,7 +27,7 @@ struct SnapshotHeader {
     uint32_t magic, version, n, worlds;
     uint32_t prevCount, cur, configured, stepContacts;
     uint32_t pairCount, sleepable, asleep;
-    uint32_t general;   // 1: Normal bodies only, 2: others too, 0: not recorded (older images)
+    uint32_t threads;   // Context::threadShapes: 1 no, 2 yes, 0 not recorded (older images)
     uint64_t bodyBytes, totalBytes;
     uint64_t geometry;  // geometryKey of the world the image was taken from
     vxb_step_config config;
@@ -61,7 +61,7 @@ SnapshotHeader headerOf(const Context& c) {
     h.pairCount = c.sleep.pairCount;
     h.sleepable = c.sleep.sleepable;
     h.asleep = c.sleep.asleep;
-    h.general = c.generalShapes ? 2u : 1u;
+    h.threads = c.threadShapes ? 2u : 1u;
     h.bodyBytes = bodyBytesOf(c);
     h.totalBytes = imageBytes(c, c.prevCount, c.sleep.pairCount);
     h.geometry = geometryKey(c);
@@ -118,7 +118,7 @@ int copyIn(Context& c, const SnapshotHeader& h, const char* src, cudaMemcpyKind 
     const size_t bb = bodyBytesOf(c);
     tapeEnd(c);
     SN_CUDA(c, cudaMemcpyAsync(c.bodyBuf.ptr, src, bb, kind, c.stream));
-    c.generalShapes = h.general != 1u;  // the body words bring their geometry quality
+    c.threadShapes = h.threads != 1u;  // the body words bring their geometry quality
     c.cur = (int)h.cur;
     if (h.prevCount) {
         VXB_TRY_SN(c, ensure(c, c.contactBuf[c.cur ^ 1], (size_t)h.prevCount * sizeof(vx_contact) + 128));
