@@ -118,3 +118,33 @@ def test_compounds_run_a_thread_each():
     c.close()
     print("narrow phase of compounds,", len(pairs), "pairs:", classified, "against", threads, "ms")
     assert classified < 1.4 * threads
+
+
+# Box stacks: pairs in touch and just apart. Their face clipping runs in one pass;
+# done in two, one behind the other, the classified phase lost to a thread a pair
+# (0.48 against 0.41 ms; 0.27 in one).
+def test_box_stacks_clip_their_faces_in_one_pass():
+    specs, pool = vb.generate_scene(3, seed=3, size=2)
+    bodies, hull, faces = vb.bodies_from_specs(specs, pool)
+    soup = vb.make_soup(hull, faces)
+    c = vb.Context(0)
+    c.load(bodies, soup)
+    c.configure(dt=DT, substeps=8)
+    c.step(6)
+    bodies = c.read_bodies()
+    pairs = c.pairs(bodies, DT, soup)
+    c.enable_timing(True)
+
+    def stage(call):
+        times = []
+        for _ in range(6):
+            before = c.stage_times()["narrowphase"][0]
+            call()
+            times.append(c.stage_times()["narrowphase"][0] - before)
+        return min(times)
+
+    classified = stage(lambda: c.backend_find_contacts(bodies, soup, DT))
+    threads = stage(lambda: c.collide(bodies, soup, pairs, DT))
+    c.close()
+    print("narrow phase of box stacks:", classified, "against", threads, "ms")
+    assert classified < threads

@@ -536,6 +536,16 @@ struct HardResult {
     float distance;
     V3 normal, pointA, pointB;
 };
+// Mark on a listed pair whose query the thread kernel has answered: two boxes or
+// hulls close to each other, whose face clipping waits for kListedPairs, where it
+// runs beside that of the overlapping pairs instead of before it, in full warps
+// (narrow phase of one step: heap of 3,000 bodies 0.57 -> 0.41 ms, of 40,000 1.40
+// -> 0.98, 64 box pyramids 1.66 -> 1.14).
+constexpr uint32_t kAnswered = 0x80000000u;
+VXD bool clipsFaces(float distance, uint32_t flagsA, uint32_t flagsB) {
+    const uint32_t sa = shapeOf(flagsA), sb = shapeOf(flagsB);
+    return distance < 0.05f && (sa == kBox || sa == kHull) && (sb == kBox || sb == kHull);
+}
 
 // Contacts of one pair in the order of the reference's host sort within one
 // (a, b) key (mode 0; mode 1 keeps the emission order).
@@ -575,14 +585,20 @@ __global__ void __launch_bounds__(128) collideKernel(BodyArrays B, Soup soup, co
                                                      const uint32_t* order, uint32_t npairs, float dt, int mode,
                                                      int bodyBits, vx_contact* tmp, uint32_t contactCap,
                                                      uint64_t* recKeys, uint32_t* recVals, uint2* recInfo,
-                                                     uint32_t recCap, uint32_t* hard, const HardResult* results,
+                                                     uint32_t recCap, uint32_t* hard, HardResult* results,
                                                      Counters* C) {
     const uint32_t stride = gridDim.x * blockDim.x;
     if (Class == kListedPairs || Class == kThreadPairs) npairs = C->hardPairs;
     const uint32_t rounded = (npairs + 31u) & ~31u;
     for (uint32_t base = blockIdx.x * blockDim.x; base < rounded; base += stride) {
         const uint32_t slot = base + threadIdx.x;
-        const uint32_t p = slot < npairs && order ? order[slot] : slot;
+        uint32_t p = slot < npairs && order ? order[slot] : slot;
+        bool answered = false;
+        if (Class == kListedPairs || Class == kThreadPairs) {
+            answered = p & kAnswered;
+            p &= ~kAnswered;
+        }
+        HardResult answer;
         vx_contact buf[kMaxContactsPerPair];
         int count = 0;
         bool later = false;
@@ -597,7 +613,7 @@ __global__ void __launch_bounds__(128) collideKernel(BodyArrays B, Soup soup, co
                 if (shapeOf(b.flags) == kPlane) planeConvex(a, b, i, j, soup, dt, buf, kMaxContactsPerPair, count);
                 else planeConvex(b, a, j, i, soup, dt, buf, kMaxContactsPerPair, count);
             } else if (Class == kThreadPairs) {
-                if (threadPair(npairs, a.flags, b.flags)) count = collidePair(a, b, i, j, soup, dt, buf, kMaxContactsPerPair);
+                if (!answered && threadPair(npairs, a.flags, b.flags)) count = collidePair(a, b, i, j, soup, dt, buf, kMaxContactsPerPair);
             } else if (isComplexShape(shapeOf(a.flags)) || isComplexShape(shapeOf(b.flags)) ||
                        (Class == kListedPairs && threadPair(npairs, a.flags, b.flags))) {
                 later = Class == kConvexPairs;  // (as a listed pair: done by its warp or thread)
@@ -614,6 +630,10 @@ __global__ void __launch_bounds__(128) collideKernel(BodyArrays B, Soup soup, co
                 GjkResult r;
                 Simplex s;
                 later = gjkDistanceFast(ca, cb, r, s) != kGjkSeparated;
+                if (!later && clipsFaces(r.distance, a.flags, b.flags)) {
+                    later = answered = true;
+                    answer = HardResult{r.distance, r.normal, r.pointA, r.pointB};
+                }
                 if (!later) convexContacts(a, b, i, j, ca, cb, r, dt, buf, kMaxContactsPerPair, count);
             }
             orderContacts(buf, count, mode);
@@ -623,7 +643,9 @@ __global__ void __launch_bounds__(128) collideKernel(BodyArrays B, Soup soup, co
             uint32_t at = 0;
             if (m && (threadIdx.x & 31) == 0) at = atomicAdd(&C->hardPairs, (uint32_t)__popc(m));
             at = __shfl_sync(0xffffffffu, at, 0);
-            if (later) hard[at + __popc(m & laneMaskLt())] = p;
+            at += __popc(m & laneMaskLt());
+            if (later) hard[at] = answered ? p | kAnswered : p;
+            if (answered) results[at] = answer;
         }
         // Warp-wide exclusive scan of the counts, one atomic per warp.
         const int lane = threadIdx.x & 31;
@@ -668,6 +690,7 @@ __global__ void __launch_bounds__(kQueryThreads) collideHardKernel(BodyArrays B,
     const uint32_t count = C->hardPairs, warps = (gridDim.x * blockDim.x) >> 5;
     for (uint32_t k = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; k < count; k += warps) {
         const uint32_t p = hard[k];
+        if (p & kAnswered) continue;
         const uint64_t pr = pairs[p];
         const uint32_t i = (uint32_t)(pr >> 32), j = (uint32_t)pr;
         const BodyView a = loadView(B, i), b = loadView(B, j);
@@ -2869,7 +2892,7 @@ static int narrowPhase(Context& c, const uint64_t* pairs, uint32_t npairs, float
                 VXB_TRY(tunedLaunch(c, kTuneCollideConvex, convexSplit, [&](LaunchShape sh) {
                     LAUNCH(c, collideKernel<kConvexPairs>, sh.grid(convexSplit, c.smCount), sh.threads, c.B, soupOf(c),
                            pairs, order, convexSplit, dt, mode, bodyBits, tmp, c.contactCap, recKeys, recVals, recInfo,
-                           c.recCap, hard, (const HardResult*)nullptr, c.dCounters);
+                           c.recCap, hard, results, c.dCounters);
                 }, CounterRestore{c}));
                 const int rc = launchQueries(c, convexSplit, collideHardKernel, c.B, soupOf(c), pairs,
                                              (const uint32_t*)hard, dt, mode, bodyBits, tmp, c.contactCap, recKeys,
@@ -2877,25 +2900,25 @@ static int narrowPhase(Context& c, const uint64_t* pairs, uint32_t npairs, float
                 if (rc != VXB_OK) return rc;
                 LAUNCH(c, collideKernel<kListedPairs>, blocksFor(convexSplit, 64, (uint32_t)c.smCount * 16), 64, c.B,
                        soupOf(c), pairs, (const uint32_t*)hard, convexSplit, dt, mode, bodyBits, tmp, c.contactCap,
-                       recKeys, recVals, recInfo, c.recCap, (uint32_t*)nullptr, (const HardResult*)results,
+                       recKeys, recVals, recInfo, c.recCap, (uint32_t*)nullptr, results,
                        c.dCounters);
                 if (c.threadShapes)
                     LAUNCH(c, collideKernel<kThreadPairs>, blocksFor(convexSplit, 64, (uint32_t)c.smCount * 16), 64,
                            c.B, soupOf(c), pairs, (const uint32_t*)hard, convexSplit, dt, mode, bodyBits, tmp,
                            c.contactCap, recKeys, recVals, recInfo, c.recCap, (uint32_t*)nullptr,
-                           (const HardResult*)nullptr, c.dCounters);
+                           (HardResult*)nullptr, c.dCounters);
             }
             if (np)
                 VXB_TRY(tunedLaunch(c, kTuneCollidePlane, np, [&](LaunchShape sh) {
                     LAUNCH(c, collideKernel<kPlanePairs>, sh.grid(np, c.smCount), sh.threads, c.B, soupOf(c), planePairs,
                            (const uint32_t*)nullptr, np, dt, mode, bodyBits, tmp, c.contactCap, recKeys, recVals,
-                           recInfo, c.recCap, (uint32_t*)nullptr, (const HardResult*)nullptr, c.dCounters);
+                           recInfo, c.recCap, (uint32_t*)nullptr, (HardResult*)nullptr, c.dCounters);
                 }, CounterRestore{c}));
         } else if (npairs) {
             VXB_TRY(tunedLaunch(c, kTuneCollideAny, npairs, [&](LaunchShape sh) {
                 LAUNCH(c, collideKernel<kAnyPairs>, sh.grid(npairs, c.smCount), sh.threads, c.B, soupOf(c), pairs,
                        (const uint32_t*)nullptr, npairs, dt, mode, bodyBits, tmp, c.contactCap, recKeys, recVals,
-                       recInfo, c.recCap, (uint32_t*)nullptr, (const HardResult*)nullptr, c.dCounters);
+                       recInfo, c.recCap, (uint32_t*)nullptr, (HardResult*)nullptr, c.dCounters);
             }, CounterRestore{c}));
         }
         stageEnd(c, kStageNarrowphase);
