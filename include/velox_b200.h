@@ -155,7 +155,7 @@ uint64_t vxb_context_host_syncs(const vxb_context* ctx);
  * launches a fixed 256-thread block per 256 pairs (src/backend_cuda.cu:459,
  * :556-561). */
 #define VXB_TUNE_COLLIDE_CONVEX 0
-#define VXB_TUNE_COLLIDE_COMPLEX 1
+#define VXB_TUNE_COLLIDE_COMPLEX 1 /* keeps its number; nothing launches this site any more */
 #define VXB_TUNE_COLLIDE_PLANE 2
 #define VXB_TUNE_COLLIDE_ANY 3
 #define VXB_TUNE_REWIND_PROBE 4

@@ -15,6 +15,9 @@
 // phase of 1,000 boxes: 9.2 of 14 cycles per instruction). The shapes lie in
 // shared memory and one out-of-line support mapping serves all callers; the
 // faces of GJK's tetrahedron go to four lanes through one copy of the code.
+//
+// Robust and Paranoid pairs take the general routine on one lane; the kernels
+// that can meet one carry it (255 registers and its 11 KB of stack).
 #pragma once
 #include "geom.cuh"
 
@@ -291,7 +294,7 @@ static __device__ __noinline__ void horizon(WarpQuery& W, unsigned mask, uint32_
     }
 }
 
-// epaPenetration.
+// epaPenetration at Normal quality (other qualities take the general routine).
 static __device__ __noinline__ bool epaWarp(const Simplex& s, GjkResult& result) {
     WarpQuery& W = warpQuery();
     const Convex &A = W.shape[0], &B = W.shape[1];
@@ -300,19 +303,7 @@ static __device__ __noinline__ bool epaWarp(const Simplex& s, GjkResult& result)
     if (lane == 0u)
         for (int i = 0; i < 4; ++i) W.verts[i] = s.v[i];
     __syncwarp();
-    const float scale = pairScale(A, B);
-    const uint8_t quality = pairQuality(A, B);
-    float areaFloorSq = 1e-16f;
-    if (quality != 0) {
-        float maxInitialAreaSq = 0.0f;
-#pragma unroll 1
-        for (int i = 0; i < 4; ++i) {
-            const V3 a = W.verts[kEpaInitial[i][0]].p, b = W.verts[kEpaInitial[i][1]].p,
-                     c = W.verts[kEpaInitial[i][2]].p;
-            maxInitialAreaSq = vmax(maxInitialAreaSq, lengthSq(crossRaw(b - a, c - a)));
-        }
-        areaFloorSq = vmax(maxInitialAreaSq * 1e-16f, 1e-20f * scale * scale * scale * scale);
-    }
+    constexpr float areaFloorSq = 1e-16f;
     int vertexCount = 4, faceCount = 4;
     auto put = [&](uint32_t slot, const EpaFace& f) {
         W.face[slot] = pack(f.normal, f.distance);
@@ -322,16 +313,15 @@ static __device__ __noinline__ bool epaWarp(const Simplex& s, GjkResult& result)
     if (lane < 4u) {
         EpaFace f;
         ok0 = makeEpaFace(W.verts, kEpaInitial[lane][0], kEpaInitial[lane][1], kEpaInitial[lane][2],
-                          quality == 0 ? 1e-16f : 0.0f, f);
+                          areaFloorSq, f);
         if (ok0) put(lane, f);
     }
     if (!__all_sync(kFullWarp, ok0)) return false;
     __syncwarp();
     const float dupSq = duplicateDistanceSq(A, B);
     int bestFace = 0;
-    const int maxIterations = quality == 0 ? 48 : 64;
 #pragma unroll 1
-    for (int it = 0; it < maxIterations; ++it) {
+    for (int it = 0; it < 48; ++it) {
         uint32_t key = 0xffffffffu, index = 0xffffffffu;  // nearest valid face, the first of equals
         for (uint32_t i = lane; i < (uint32_t)faceCount; i += 32u) {
             const float dist = W.face[i].w;
@@ -346,8 +336,7 @@ static __device__ __noinline__ bool epaWarp(const Simplex& s, GjkResult& result)
         const V3 normal = f3(closest);
         const SupportVert w = supportVertexWarp(normal);
         const float supportDistance = dot(normal, w.p);
-        const float tolerance = quality == 0 ? 1e-4f * vmax(1.0f, supportDistance)
-                                             : 1e-4f * vmax(scale, fabsf(supportDistance));
+        const float tolerance = 1e-4f * vmax(1.0f, supportDistance);
         bool near = false;
         for (uint32_t i = lane; i < (uint32_t)vertexCount; i += 32u)
             near |= lengthSq(w.p - W.verts[i].p) < dupSq;
@@ -418,12 +407,9 @@ static __device__ __noinline__ bool epaWarp(const Simplex& s, GjkResult& result)
     return false;
 }
 
-// gjkOverlapTail.
+// gjkOverlapTail at Normal quality.
 static __device__ __noinline__ GjkResult overlapTailWarp(Simplex& s, bool expand) {
     const Convex &A = warpQuery().shape[0], &B = warpQuery().shape[1];
-    const float scale = pairScale(A, B);
-    const float scaleSq = scale * scale;
-    const bool robust = pairQuality(A, B) != 0;
     if (expand && s.count < 4) expandOverlapWarp(s);
     GjkResult r;
     r.distance = 0.0f;
@@ -431,7 +417,7 @@ static __device__ __noinline__ GjkResult overlapTailWarp(Simplex& s, bool expand
     r.overlapping = true;
     if (s.count == 4 && epaWarp(s, r)) return r;
     V3 n = A.position - B.position;
-    n = lengthSq(n) > (robust ? scaleSq * 1e-14f : 1e-12f) ? normalize(n) : V3{0.0f, 1.0f, 0.0f};
+    n = lengthSq(n) > 1e-12f ? normalize(n) : V3{0.0f, 1.0f, 0.0f};
     const SupportVert v = supportVertexWarp(-n);  // A's support along -n, B's along n
     const V3 sa = v.a, sb = v.b;
     const float depth = dot(n, sb - sa);

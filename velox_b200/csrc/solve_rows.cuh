@@ -1,28 +1,28 @@
-// Island solve on one block: the substep loop (integration, warm start, the
-// coloured sweeps, transform integration) or the position correction of every
-// island that one block's shared memory can hold.
+// Island solve on one warp or one block: the substep loop (integration, warm
+// start, the coloured sweeps, transform integration) or the position correction
+// of every island that one block's shared memory can hold.
 //
-// What bounds it: a colour's rows run in parallel, colours in order, so an
-// island costs (sweeps x colours) dependent steps, and a step costs the
-// latency of one row: read two bodies, two impulses through a world-space
-// inverse inertia each, write two bodies, barrier. Everything here shortens
-// that step:
+// What bounds it: rows that share a body run in colour order, so an island costs
+// its longest chain of such rows times the sweeps, and a link costs the latency
+// of one row: read two bodies, two impulses through a world-space inverse inertia
+// each, write two bodies. Everything here shortens that link:
 //   * two lanes per row, one per body: each lane forms its own point velocity
 //     and applies the impulses to its own body, and the two velocities cross
 //     by shuffle, so a lane issues about half of the row's instructions;
 //   * a row's prepared terms lie in planes of 16-byte words indexed by solve
 //     position (a colour's rows are consecutive there, so a warp's loads are
-//     whole lines), and a lane loads its next row, of this colour or of the
-//     next, while it computes the current one;
-//   * a lane keeps its own copy of the row's impulses (the side planes), so
-//     no lane reads what another wrote except body velocities, which live in
-//     shared memory and are ordered by the colour barrier;
+//     whole lines), and a lane loads its next row while it computes the current
+//     one;
+//   * a lane keeps its own copy of the row's impulses (the side planes), so no
+//     lane reads what another wrote except body velocities, which live in shared
+//     memory; one warp orders them colour by colour, several by a tag on each
+//     body (the dataflow below), without a barrier;
 //   * no branch, predicate chain or general division where the operands allow
 //     it (laneSweep, quotient): a warp alone on its scheduler pays each in full.
-// A step fell from 3.8 us (256 threads, a row per thread, 128- and 176-byte
-// records read at the start of the step) to 1.2 us on an island of 400 rows in
-// 25 colours. Solve stage of one step: 13.3 -> 5.4 ms for 64 islands of 2,400
-// rows (31 colours, 8 substeps), 4.8 -> 1.9 ms for one of 310 rows (20 colours).
+// Solve stage of one step, one row per thread on 128- and 176-byte records with a
+// barrier a colour -> two lanes on planes -> the dataflow: 64 islands of 2,400
+// rows (31 colours, 8 substeps) 13.3 -> 5.4 -> 4.5 ms, one of 310 rows (20
+// colours) 4.8 -> 1.9 -> 1.6 ms.
 // Measured and not kept: cross's sign rule behind a branch (20 % slower), one
 // lane per row with the same planes (about equal for narrow colours, slower
 // for wide ones).
@@ -422,8 +422,8 @@ VXD LaneBody loadLane(const SolveArgs& A, const BodyTable& T, int li) {
 }
 
 // One lane of one row (all 32 lanes call; `act`: this lane holds a row).
-// warmPrepRow / sweepRow / sharedRow's position step on the pair's two lanes,
-// the same arithmetic in the same order.
+// warmPrepRow / sweepRow / positionRow on the pair's two lanes, the same
+// arithmetic in the same order.
 template <int Op, bool Cone>
 VXD void laneRow(const SolveArgs& A, const RowPlanes& R, const BodyTable& T, bool act, uint32_t k, uint32_t side,
                  RowRegs& r, LaneBody& b) {

@@ -27,7 +27,7 @@ namespace vxb {
 
 enum TuneSite : int {
     kTuneCollideConvex = 0,  // collideKernel over convex-convex pairs (GJK / EPA, clipping)
-    kTuneCollideComplex,     // collideKernel over pairs with a mesh, heightfield or compound
+    kTuneCollideComplex,     // launched no more (mesh and compound pairs); keeps its number and its cache lines
     kTuneCollidePlane,       // collideKernel over body-plane pairs
     kTuneCollideAny,         // collideKernel over unclassified pairs (stage entry points)
     kTuneProbe,              // caProbeKernel: the rewind's end-of-step distance query per pair
