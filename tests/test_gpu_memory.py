@@ -28,3 +28,32 @@ def test_rows_of_a_first_solve_fit_the_reserved_memory():
     # the plan's per-body and per-row words: about 100 bytes a body and 60 a row,
     # half as much on top; the rows' prepared terms would be 384 bytes a row
     assert held < 250 << 20
+
+
+def test_a_world_loads_without_the_reserve():
+    """Memory for rows that a world may never have is asked for, not required."""
+    n = 400_000
+    body = np.zeros(n, vb.BODY)
+    body["orientation"] = body["inertiaOrientation"] = (0, 0, 0, 1)
+    body["motionType"], body["invMass"], body["invInertia"], body["radius"] = 2, 1.0, 2.0, 0.5
+    body["position"][:, 0] = 3.0 * np.arange(n)
+
+    def advance(ctx):
+        moved = body.copy()
+        ctx.backend_integrate(moved, (0.0, -9.81, 0.0), 1.0 / 60.0)
+        return moved["velocity"]
+
+    ctx = vb.Context(0)
+    before = torch.cuda.mem_get_info()[0]
+    want = advance(ctx)
+    held = before - torch.cuda.mem_get_info()[0]
+    ctx.close()
+    # the reserve is 2 x 252 bytes a body and half as much on top: 300 MB
+    filler = torch.empty(torch.cuda.mem_get_info()[0] - held + (200 << 20), dtype=torch.uint8, device="cuda")
+    ctx = vb.Context(0)
+    try:
+        assert np.array_equal(advance(ctx), want)
+    finally:
+        ctx.close()
+        del filler
+        torch.cuda.empty_cache()

@@ -2641,6 +2641,15 @@ static Soup soupOf(Context& c) {
                 P<uint32_t>(c.triRefBuf), P<vx_compound_child>(c.childBuf)};
 }
 
+// ensure() for what a later call may need and asks for itself, at most an eighth
+// of the free memory: a world that fits without it still loads and steps.
+static void reserve(Context& c, DevBuf& b, size_t bytes) {
+    size_t free = 0, total = 0;
+    if (bytes <= b.bytes || cudaMemGetInfo(&free, &total) != cudaSuccess || bytes > free / 8) return;
+    const std::string last = c.lastError;
+    if (ensure(c, b, bytes) != VXB_OK) c.lastError = last;
+}
+
 int loadBodies(Context& c, const vx_body* bodies, uint32_t n, const uint32_t* worldOf, bool deviceWorld) {
     if (n == 0) return fail(c, VXB_ERR_INVALID, "no bodies");
     // The Backend path reloads the same bodies between its calls of one step
@@ -2740,8 +2749,8 @@ int loadBodies(Context& c, const vx_body* bodies, uint32_t n, const uint32_t* wo
     // of a world's first steps, they were freed and allocated a dozen times each
     // (solve stage of steps 6 to 25 of 4,096 worlds 15.3 -> 9.7 ms; a free now and
     // then takes tens of ms more).
-    VXB_TRY(ensure(c, c.planeBuf, ((size_t)2 * n + 4096) * kRowPlaneBytes + 256));
-    VXB_TRY(ensure(c, c.hardBuf, ((size_t)2 * n + 4096) * (4 + sizeof(HardResult)) + 64));
+    reserve(c, c.planeBuf, ((size_t)2 * n + 4096) * kRowPlaneBytes + 256);
+    reserve(c, c.hardBuf, ((size_t)2 * n + 4096) * (4 + sizeof(HardResult)) + 64);
     c.prevCount = 0;
     c.stepContacts = 0;
     VXB_TRY(sleepLoad(c, bodies, n));
