@@ -2745,12 +2745,26 @@ int loadBodies(Context& c, const vx_body* bodies, uint32_t n, const uint32_t* wo
                       &c.sortKeysAlt})
         VXB_TRY(ensure(c, *b, mcap * 8 + 64));
     VXB_TRY(ensure(c, c.sortValsAlt, std::max<size_t>(mcap, (size_t)c.pairCap) * 4 + 64));
-    // The rows' planes and the listed pairs, two a body: grown with the contacts
-    // of a world's first steps, they were freed and allocated a dozen times each
-    // (solve stage of steps 6 to 25 of 4,096 worlds 15.3 -> 9.7 ms; a free now and
-    // then takes tens of ms more).
-    reserve(c, c.planeBuf, ((size_t)2 * n + 4096) * kRowPlaneBytes + 256);
-    reserve(c, c.hardBuf, ((size_t)2 * n + 4096) * (4 + sizeof(HardResult)) + 64);
+    // What grows with the contacts of a world's first steps: the rows' planes and
+    // the listed pairs for two a body, the island plan and the rewind for fewer.
+    // Each was freed and allocated a dozen times on the way (4,096 worlds from rest,
+    // 60 steps: 170 allocations and 299 ms -> 27 and 279; a free now and then takes
+    // tens of ms more).
+    const size_t half = (size_t)n / 2 + 4096, few = (size_t)n / 16 + 1024;
+    const struct {
+        DevBuf* buf;
+        size_t bytes;
+    } later[] = {{&c.planeBuf, ((size_t)2 * n + 4096) * kRowPlaneBytes + 256},
+                 {&c.hardBuf, ((size_t)2 * n + 4096) * (4 + sizeof(HardResult)) + 64},
+                 {&c.caFlagBuf, 2 * half * 28 + 64},
+                 {&c.caCandBuf, 2 * half * 28 + 64},
+                 {&c.islandBodyStartBuf, half * 4 + 64},
+                 {&c.tinyBuf, half * 17 + 1024},
+                 {&c.tinyKeyBuf, half * 8 + 64},
+                 {&c.caSpecBuf, few * 136 + 64},
+                 {&c.islandInfoBuf, few * 24 + 512},
+                 {&c.caInfoBuf, few * 16 + 64}};
+    for (const auto& r : later) reserve(c, *r.buf, r.bytes);
     c.prevCount = 0;
     c.stepContacts = 0;
     VXB_TRY(sleepLoad(c, bodies, n));
