@@ -2641,13 +2641,38 @@ static Soup soupOf(Context& c) {
                 P<uint32_t>(c.triRefBuf), P<vx_compound_child>(c.childBuf)};
 }
 
-// ensure() for what a later call may need and asks for itself, at most an eighth
-// of the free memory: a world that fits without it still loads and steps.
-static void reserve(Context& c, DevBuf& b, size_t bytes) {
+// What grows with the contacts of a world's first steps: the rows' planes and the
+// listed pairs for two a body, the island plan and the rewind for fewer. Each was
+// freed and allocated a dozen times on the way (4,096 worlds from rest, 60 steps:
+// 170 allocations and 299 ms -> 27 and 279; a free now and then takes tens of ms
+// more). Asked for, not required: a world that fits the device without it loads
+// and steps. A small world's buffers grow from one small block to the next, and
+// ten allocations would double its load (3,000 bodies 2 -> 4 ms).
+constexpr uint32_t kReserveBodies = 16384;
+static void reserve(Context& c, uint32_t n) {
+    if (n < kReserveBodies) return;
+    const size_t half = n / 2, few = n / 16;
+    const struct {
+        DevBuf* buf;
+        size_t bytes;
+    } later[] = {{&c.planeBuf, 4 * half * kRowPlaneBytes},
+                 {&c.hardBuf, 4 * half * (4 + sizeof(HardResult))},
+                 {&c.caFlagBuf, 2 * half * 28},
+                 {&c.caCandBuf, 2 * half * 28},
+                 {&c.islandBodyStartBuf, half * 4},
+                 {&c.tinyBuf, half * 17},
+                 {&c.tinyKeyBuf, half * 8},
+                 {&c.caSpecBuf, few * 136},
+                 {&c.islandInfoBuf, few * 24},
+                 {&c.caInfoBuf, few * 16}};
     size_t free = 0, total = 0;
-    if (bytes <= b.bytes || cudaMemGetInfo(&free, &total) != cudaSuccess || bytes > free / 8) return;
-    const std::string last = c.lastError;
-    if (ensure(c, b, bytes) != VXB_OK) c.lastError = last;
+    for (const auto& r : later) {
+        if (r.bytes <= r.buf->bytes) continue;
+        if (!total && cudaMemGetInfo(&free, &total) != cudaSuccess) return;
+        if (r.bytes > free / 8) continue;  // an eighth of what is free at most
+        const std::string last = c.lastError;
+        if (ensure(c, *r.buf, r.bytes) != VXB_OK) c.lastError = last;
+    }
 }
 
 int loadBodies(Context& c, const vx_body* bodies, uint32_t n, const uint32_t* worldOf, bool deviceWorld) {
@@ -2745,26 +2770,7 @@ int loadBodies(Context& c, const vx_body* bodies, uint32_t n, const uint32_t* wo
                       &c.sortKeysAlt})
         VXB_TRY(ensure(c, *b, mcap * 8 + 64));
     VXB_TRY(ensure(c, c.sortValsAlt, std::max<size_t>(mcap, (size_t)c.pairCap) * 4 + 64));
-    // What grows with the contacts of a world's first steps: the rows' planes and
-    // the listed pairs for two a body, the island plan and the rewind for fewer.
-    // Each was freed and allocated a dozen times on the way (4,096 worlds from rest,
-    // 60 steps: 170 allocations and 299 ms -> 27 and 279; a free now and then takes
-    // tens of ms more).
-    const size_t half = (size_t)n / 2 + 4096, few = (size_t)n / 16 + 1024;
-    const struct {
-        DevBuf* buf;
-        size_t bytes;
-    } later[] = {{&c.planeBuf, ((size_t)2 * n + 4096) * kRowPlaneBytes + 256},
-                 {&c.hardBuf, ((size_t)2 * n + 4096) * (4 + sizeof(HardResult)) + 64},
-                 {&c.caFlagBuf, 2 * half * 28 + 64},
-                 {&c.caCandBuf, 2 * half * 28 + 64},
-                 {&c.islandBodyStartBuf, half * 4 + 64},
-                 {&c.tinyBuf, half * 17 + 1024},
-                 {&c.tinyKeyBuf, half * 8 + 64},
-                 {&c.caSpecBuf, few * 136 + 64},
-                 {&c.islandInfoBuf, few * 24 + 512},
-                 {&c.caInfoBuf, few * 16 + 64}};
-    for (const auto& r : later) reserve(c, *r.buf, r.bytes);
+    reserve(c, n);
     c.prevCount = 0;
     c.stepContacts = 0;
     VXB_TRY(sleepLoad(c, bodies, n));
